@@ -1636,14 +1636,10 @@ int litho_reinit_sdf(litho_ctx* ctx, int rows, int cols, const float* d_phi, dou
   if (d_sdf == d_phi) return ctx->fail(LITHO_ERR_INVALID_ARGUMENT, "reinit_sdf: sdf must not alias phi");
   ctx->stage_begin(8);
   st = check_launch(ctx, launch_reinit_sdf(ctx->stream, rows, cols, d_phi, 0.f, 0, (float)dx, d_sdf,
-                                           1, ctx->chamfer_threads(cols, 1)),
+                                           d_mask, 1, ctx->chamfer_threads(cols, 1)),
                     "reinit_sdf");
-  if (!st && d_mask)
-    st = check_launch(ctx, launch_levelset(ctx->stream, 5, rows, cols, d_sdf, nullptr, nullptr,
-                                           (float)dx, (float)dy, 0.f, nullptr, d_mask, nullptr),
-                      "mask");
   ctx->stage_end(8);
-  ctx->launches += d_mask ? 2 : 1;
+  ctx->launches += 2;
   if (!st) LITHO_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
   if (!st) ctx->collect_stages();
   return st;
@@ -1772,11 +1768,9 @@ int litho_ctx_autotune(litho_ctx* ctx, const litho_cache* cache, int batch, int 
       int bt = 0;
       for (const int t : {128, 256, 512, 1024}) {
         if (st) break;
-        const int per = (cols + t - 1) / t;
-        if ((t <= 256 && per > 32) || (t == 512 && per > 16)) continue;
         float ms = 0.f;
         st = timed([&]() {
-          return launch_reinit_sdf(s, rows, cols, phi, 0.f, 0, 1.f, out, nt, t);
+          return launch_reinit_sdf(s, rows, cols, phi, 0.f, 0, 1.f, out, nullptr, nt, t);
         }, &ms);
         if (!st && (bt == 0 || ms < best)) { best = ms; bt = t; }
       }
@@ -1869,15 +1863,11 @@ int litho_reinit_sdf_batch(litho_ctx* ctx, int batch, int rows, int cols, const 
   for (int b0 = 0; b0 < batch && !st; b0 += 65535) {
     const int B = std::min(batch - b0, 65535);
     st = check_launch(ctx, launch_reinit_sdf(ctx->stream, rows, cols, d_phi + b0 * n, (float)level,
-                                             0, (float)dx, d_sdf + b0 * n, B,
+                                             0, (float)dx, d_sdf + b0 * n,
+                                             d_mask ? d_mask + b0 * n : nullptr, B,
                                              ctx->chamfer_threads(cols, B)),
                       "reinit_sdf");
-    if (!st && d_mask)
-      st = check_launch(ctx, launch_levelset(ctx->stream, 5, rows, cols, d_sdf + b0 * n, nullptr,
-                                             nullptr, (float)dx, (float)dy, 0.f, nullptr,
-                                             d_mask + b0 * n, nullptr, nullptr, B),
-                        "mask");
-    ctx->launches += d_mask ? 2 : 1;
+    ctx->launches += 2;
   }
   return st;
 }
@@ -2740,6 +2730,7 @@ int litho_fullchip_lsm_init(litho_ctx* ctx, const litho_partition* p, const floa
   for (int t0 = 0; t0 < p->ntiles && !st; t0 += 65535)
     st = check_launch(ctx, launch_reinit_sdf(s, p->ts, p->ts, d_masks + (size_t)t0 * p->ts * p->ts,
                                              0.5f, 0, (float)dx, d_phi + (size_t)t0 * p->ts * p->ts,
+                                             nullptr,
                                              std::min(p->ntiles - t0, 65535),
                                              ctx->chamfer_threads(p->ts,
                                                                   std::min(p->ntiles - t0, 65535))),
@@ -2748,7 +2739,7 @@ int litho_fullchip_lsm_init(litho_ctx* ctx, const litho_partition* p, const floa
     st = check_launch(ctx, launch_render_mask(s, d_phi, p->ts, p->ts, p->ntiles,
                                               mask_type == LITHO_MASK_GRAY, scale, d_masks),
                       "render_levelset_mask");
-  ctx->launches += 3;
+  ctx->launches += 4;
   if (!st) LITHO_CUDA_TRY(ctx, cudaStreamSynchronize(s));
   return st;
 }
@@ -2818,7 +2809,8 @@ int litho_fullchip_lsm_step(litho_ctx* ctx, const litho_partition* p, const floa
   for (int t0 = 0; reinit && t0 < n && !st; t0 += 65535) {
     const int B = std::min(n - t0, 65535);
     st = check_launch(ctx, launch_reinit_sdf(s, ts, ts, d_phi_out + t0 * tt, 0.f, 1, (float)dx,
-                                             d_masks + t0 * tt, B, ctx->chamfer_threads(ts, B)),
+                                             d_masks + t0 * tt, nullptr, B,
+                                             ctx->chamfer_threads(ts, B)),
                       "reinit_sdf");
     if (!st)
       st = check_launch(ctx, launch_levelset(s, 8, ts, ts, d_masks + t0 * tt, d_phi_out + t0 * tt,
@@ -2826,7 +2818,7 @@ int litho_fullchip_lsm_step(litho_ctx* ctx, const litho_partition* p, const floa
                                              d_phi_out + t0 * tt, nullptr, nullptr, B,
                                              wins + 4 * (size_t)t0, 0),
                         "window commit");
-    ctx->launches += 2;
+    ctx->launches += 3;
   }
   if (!st)
     st = check_launch(ctx, launch_render_mask(s, d_phi_out, p->ts, p->ts, n,

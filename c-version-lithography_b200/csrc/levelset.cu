@@ -441,313 +441,6 @@ cudaError_t launch_render_mask(cudaStream_t s, const float* phi, int rows, int c
   return cudaGetLastError();
 }
 
-// ---------------------------------------------------------------- reinit_sdf
-// LevelSetUtils::reinit_sdf (level_set_utils.cpp:290-319): two OpenCV
-// distanceTransform(DIST_L2, 5) calls, i.e. the 5x5 chamfer distance with
-// weights a = 1, b = 1.4, c = 2.1969 (float32) to the nearest feature pixel,
-// computed by a forward raster pass (rows top to bottom, left to right) and a
-// backward pass, each pixel taking the minimum of its own value and its already
-// final neighbours plus the weights. Within a row the only dependency is
-// d(j) = min(g(j), d(j-1) + a), g being the minimum over the rows above (below)
-// plus the pixel's own value. A CTA splits a row into one contiguous segment per
-// thread: each thread runs the recurrence over its segment from +inf, the segment
-// results are combined by a block scan with the composition
-//   (A1, L1) then (A2, L2)  ->  (min(A2, A1 + L2), L1 + L2)
-// (A: the value at the segment's last column, L: its length), and each thread reruns
-// its segment from the carry it receives. Float throughout, in a fixed order.
-//
-// One CTA runs one transform of one image (blockIdx.y): blockIdx.x = 0 measures
-// inside pixels to the outside and writes +d dx at the inside pixels, blockIdx.x = 1
-// measures outside pixels to the inside and writes -d dx at the outside pixels. A
-// transform's distance is 0 at its feature pixels (the other class), so each CTA keeps
-// its forward-pass values in the output at its own pixels only: the two CTAs of an
-// image touch disjoint pixels and need no other buffer. Inside means phi > level
-// (phi >= level when `inclusive`). With no feature pixel at all the distance stays
-// FLT_MAX, as OpenCV returns.
-//
-// PMAX > 0: a thread owns at most PMAX columns and holds their classification (and,
-// backward, their forward-pass values) in registers, loading the following rows'
-// while the current row is processed, so that the row loop waits on no global load.
-// PMAX == 0: the same transform with direct loads (very long rows).
-constexpr float DT_A = 1.0f, DT_B = 1.4f, DT_C = 2.1969f;
-
-template <int NT, int PMAX>
-__global__ void __launch_bounds__(NT)
-chamfer_sdf_kernel(const float* __restrict__ phi_all, int rows, int cols, float level,
-                   int inclusive, float dx, float* __restrict__ sdf_all) {
-  extern __shared__ float rowbuf[];  // ring of 3 rows of W = cols + 4 floats, column j at j + 2
-  __shared__ float wtot[32];
-  constexpr int NW = NT / 32;
-  constexpr int QN = PMAX > 0 ? PMAX : 1;
-  const float FMAX = 3.402823466e38f;
-  const int W = cols + 4;
-  const bool inside_pass = blockIdx.x == 0;
-  const size_t img = (size_t)blockIdx.y * rows * cols;
-  const float* phi = phi_all + img;
-  float* sdf = sdf_all + img;
-  const int per = (cols + NT - 1) / NT;  // columns per thread
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int j0 = min((int)threadIdx.x * per, cols);
-  const int nq = min(per, cols - j0);    // columns this thread owns (0 past the row end)
-  auto seg_end = [&](int t) { return min((t + 1) * per, cols); };   // one past the last column
-  auto seg_start = [&](int t) { return min(t * per, cols); };
-  if (threadIdx.x < 3) {  // +inf pads: two columns on each side of every ring row
-    float* r = rowbuf + threadIdx.x * W;
-    r[0] = r[1] = r[W - 2] = r[W - 1] = FMAX;
-  }
-  auto cls = [&](float p) { return (inclusive ? p >= level : p > level) == inside_pass; };
-  auto load_bits = [&](int i) {
-    unsigned b = 0;
-#pragma unroll
-    for (int q = 0; q < QN; ++q)
-      if (q < nq && cls(phi[(size_t)i * cols + j0 + q])) b |= 1u << q;
-    return b;
-  };
-  unsigned bits0 = 0, bits1 = 0;   // own-pixel bits of the current row and the next one
-  float pf[QN];                    // phi of a following row, in flight
-  float fv[QN];                    // backward: forward-pass values of the current row
-  auto own = [&](int i, int q) -> bool {
-    if constexpr (PMAX > 0) return ((bits0 >> q) & 1u) != 0u;
-    else return cls(phi[(size_t)i * cols + j0 + q]);
-  };
-  const int qn = PMAX > 0 ? QN : per;
-
-  // ---- forward pass
-  if constexpr (PMAX > 0) bits0 = load_bits(0);
-  for (int i = 0; i < rows; ++i) {
-    float* r0 = rowbuf + (i % 3) * W + 2;
-    const float* r1 = rowbuf + ((i + 2) % 3) * W + 2;  // row i-1
-    const float* r2 = rowbuf + ((i + 1) % 3) * W + 2;  // row i-2
-    float a = FMAX;
-#pragma unroll
-    for (int q = 0; q < qn; ++q) {
-      if (q >= nq) break;
-      const int j = j0 + q;
-      float g = 0.f;   // a feature pixel of this transform
-      if (own(i, q)) {
-        g = FMAX;
-        if (i >= 1)
-          g = fminf(fminf(fminf(r1[j] + DT_A, r1[j - 1] + DT_B), fminf(r1[j + 1] + DT_B, r1[j - 2] + DT_C)),
-                    r1[j + 2] + DT_C);
-        if (i >= 2) g = fminf(g, fminf(r2[j - 1] + DT_C, r2[j + 1] + DT_C));
-      }
-      a = fminf(g, a + DT_A);
-      r0[j] = g;
-    }
-    if constexpr (PMAX > 0) {
-      if (i + 1 < rows) {
-#pragma unroll
-        for (int q = 0; q < QN; ++q) pf[q] = q < nq ? phi[(size_t)(i + 1) * cols + j0 + q] : 0.f;
-      }
-    }
-    // inclusive scan over the threads of the segment results
-    float v = a;
-    const int e = seg_end(threadIdx.x);
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const float u = __shfl_up_sync(0xffffffffu, v, o);
-      if (lane >= o) v = fminf(v, u + (float)(e - seg_end(threadIdx.x - o)));
-    }
-    if (lane == 31) wtot[warp] = v;
-    __syncthreads();
-    if (warp == 0) {
-      float x = lane < NW ? wtot[lane] : FMAX;
-      const int ew = seg_end(32 * lane + 31);
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const float u = __shfl_up_sync(0xffffffffu, x, o);
-        if (lane >= o && lane < NW) x = fminf(x, u + (float)(ew - seg_end(32 * (lane - o) + 31)));
-      }
-      if (lane < NW) wtot[lane] = x;
-    }
-    __syncthreads();
-    // carry: the value at column j0 - 1
-    float c = __shfl_up_sync(0xffffffffu, v, 1);
-    if (lane == 0) c = FMAX;
-    if (warp > 0) {
-      const int wend = seg_end(32 * warp - 1);   // end of the previous warp's segments
-      const float wc = wtot[warp - 1] + (float)(j0 - wend);
-      c = lane == 0 ? wtot[warp - 1] : fminf(c, wc);
-    }
-    float d = c;
-#pragma unroll
-    for (int q = 0; q < qn; ++q) {
-      if (q >= nq) break;
-      const int j = j0 + q;
-      d = fminf(r0[j], d + DT_A);
-      r0[j] = d;
-      if (own(i, q)) sdf[(size_t)i * cols + j] = d;
-    }
-    if constexpr (PMAX > 0) {
-      if (i + 1 < rows) {
-        unsigned b = 0;
-#pragma unroll
-        for (int q = 0; q < QN; ++q)
-          if (q < nq && cls(pf[q])) b |= 1u << q;
-        bits0 = b;
-      }
-    }
-    __syncthreads();
-  }
-  // ---- backward pass
-  if constexpr (PMAX > 0) {
-    bits0 = load_bits(rows - 1);
-    bits1 = rows >= 2 ? load_bits(rows - 2) : 0u;
-#pragma unroll
-    for (int q = 0; q < QN; ++q)
-      fv[q] = (q < nq && ((bits0 >> q) & 1u)) ? sdf[(size_t)(rows - 1) * cols + j0 + q] : 0.f;
-  }
-  for (int i = rows - 1; i >= 0; --i) {
-    const int slot = (rows - 1 - i);
-    float* r0 = rowbuf + (slot % 3) * W + 2;
-    const float* r1 = rowbuf + ((slot + 2) % 3) * W + 2;  // row i+1 (final)
-    const float* r2 = rowbuf + ((slot + 1) % 3) * W + 2;  // row i+2 (final)
-    float a = FMAX;
-#pragma unroll
-    for (int qq = 0; qq < qn; ++qq) {
-      const int q = qn - 1 - qq;   // right to left
-      if (q >= nq) continue;
-      const int j = j0 + q;
-      float g;   // the forward-pass value (0 at a feature pixel)
-      if constexpr (PMAX > 0) g = fv[q];
-      else g = own(i, q) ? sdf[(size_t)i * cols + j] : 0.f;
-      if (g > DT_A) {
-        if (i + 1 < rows)
-          g = fminf(g, fminf(fminf(fminf(r1[j] + DT_A, r1[j + 1] + DT_B), fminf(r1[j - 1] + DT_B, r1[j + 2] + DT_C)),
-                             r1[j - 2] + DT_C));
-        if (i + 2 < rows) g = fminf(g, fminf(r2[j + 1] + DT_C, r2[j - 1] + DT_C));
-      }
-      a = fminf(g, a + DT_A);
-      r0[j] = g;
-    }
-    if constexpr (PMAX > 0) {
-      // forward values of row i - 1 (its bits are known), phi of row i - 2
-      if (i >= 1) {
-#pragma unroll
-        for (int q = 0; q < QN; ++q)
-          fv[q] = (q < nq && ((bits1 >> q) & 1u)) ? sdf[(size_t)(i - 1) * cols + j0 + q] : 0.f;
-      }
-      if (i >= 2) {
-#pragma unroll
-        for (int q = 0; q < QN; ++q) pf[q] = q < nq ? phi[(size_t)(i - 2) * cols + j0 + q] : 0.f;
-      }
-    }
-    // inclusive scan from the right of the segment results (value at a segment's first column)
-    float v = a;
-    const int st = seg_start(threadIdx.x);
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const float u = __shfl_down_sync(0xffffffffu, v, o);
-      if (lane + o < 32) v = fminf(v, u + (float)(seg_start(threadIdx.x + o) - st));
-    }
-    if (lane == 0) wtot[warp] = v;
-    __syncthreads();
-    if (warp == 0) {
-      float x = lane < NW ? wtot[lane] : FMAX;
-      const int sw = seg_start(32 * lane);
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const float u = __shfl_down_sync(0xffffffffu, x, o);
-        if (lane + o < NW) x = fminf(x, u + (float)(seg_start(32 * (lane + o)) - sw));
-      }
-      if (lane < NW) wtot[lane] = x;
-    }
-    __syncthreads();
-    // carry: the value at column j0 + nq (the next segment's first column)
-    float c = __shfl_down_sync(0xffffffffu, v, 1);
-    if (lane == 31) c = FMAX;
-    if (warp < NW - 1) {
-      const int wst = seg_start(32 * (warp + 1));   // first column of the next warp's segments
-      const float wc = wtot[warp + 1] + (float)(wst - seg_start(threadIdx.x + 1));
-      c = lane == 31 ? wtot[warp + 1] : fminf(c, wc);
-    }
-    float d = c;
-#pragma unroll
-    for (int qq = 0; qq < qn; ++qq) {
-      const int q = qn - 1 - qq;
-      if (q >= nq) continue;
-      const int j = j0 + q;
-      d = fminf(r0[j], d + DT_A);
-      r0[j] = d;
-      if (own(i, q)) {
-        if (inside_pass) sdf[(size_t)i * cols + j] = d >= FMAX ? FMAX : d * dx;
-        else sdf[(size_t)i * cols + j] = d >= FMAX ? -FMAX : -d * dx;
-      }
-    }
-    if constexpr (PMAX > 0) {
-      unsigned b = 0;
-      if (i >= 2) {
-#pragma unroll
-        for (int q = 0; q < QN; ++q)
-          if (q < nq && cls(pf[q])) b |= 1u << q;
-      }
-      bits0 = bits1;
-      bits1 = b;
-    }
-    __syncthreads();
-  }
-}
-
-// A smooth test pattern (sin x cos y with a per-image phase) whose zero set crosses
-// every row: the input of the chamfer timing of litho_ctx_autotune.
-__global__ void chamfer_probe_kernel(float* __restrict__ p, int rows, int cols, int nimg) {
-  const size_t n = (size_t)rows * cols * nimg;
-  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-       i += (size_t)gridDim.x * blockDim.x) {
-    const int x = (int)(i % cols), y = (int)((i / cols) % rows), k = (int)(i / ((size_t)rows * cols));
-    p[i] = sinf(0.031f * x + k) * cosf(0.027f * y) - 0.1f;
-  }
-}
-
-cudaError_t launch_chamfer_probe(cudaStream_t s, float* p, int rows, int cols, int nimg) {
-  chamfer_probe_kernel<<<1184, 256, 0, s>>>(p, rows, cols, nimg);
-  return cudaGetLastError();
-}
-
-template <int NT, int PMAX>
-static cudaError_t chamfer_launch(cudaStream_t s, int rows, int cols, const float* phi,
-                                  float level, int inclusive, float dx, float* sdf, int nimg) {
-  const size_t smem = (size_t)3 * (cols + 4) * sizeof(float);
-  if (smem > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(chamfer_sdf_kernel<NT, PMAX>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-  }
-  chamfer_sdf_kernel<NT, PMAX><<<dim3(2, nimg), NT, smem, s>>>(phi, rows, cols, level, inclusive,
-                                                               dx, sdf);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_reinit_sdf(cudaStream_t s, int rows, int cols, const float* phi, float level,
-                              int inclusive, float dx, float* sdf, int nimg, int threads) {
-  if (nimg < 1 || nimg > 65535 || rows < 1 || cols < 1) return cudaErrorInvalidValue;
-  // Many images: small CTAs (long segments, little scan overhead, many CTAs per SM).
-  // Few images: the row latency decides, so short segments over more threads.
-  if (threads <= 0) {
-    if (nimg >= 64) threads = cols <= 4096 ? 128 : cols <= 8192 ? 256 : 1024;
-    else threads = cols <= 1536 ? 512 : 1024;
-  }
-  const int per = (cols + threads - 1) / threads;
-  // the register arrays hold the smallest of 8, 16, 32 columns that covers a segment
-  switch (threads) {
-    case 128:
-      if (per <= 8) return chamfer_launch<128, 8>(s, rows, cols, phi, level, inclusive, dx, sdf, nimg);
-      if (per <= 16) return chamfer_launch<128, 16>(s, rows, cols, phi, level, inclusive, dx, sdf, nimg);
-      if (per <= 32) return chamfer_launch<128, 32>(s, rows, cols, phi, level, inclusive, dx, sdf, nimg);
-      return cudaErrorInvalidValue;
-    case 256:
-      if (per <= 32) return chamfer_launch<256, 32>(s, rows, cols, phi, level, inclusive, dx, sdf, nimg);
-      return cudaErrorInvalidValue;
-    case 512:
-      if (per <= 8) return chamfer_launch<512, 8>(s, rows, cols, phi, level, inclusive, dx, sdf, nimg);
-      if (per <= 16) return chamfer_launch<512, 16>(s, rows, cols, phi, level, inclusive, dx, sdf, nimg);
-      return cudaErrorInvalidValue;
-    case 1024:
-      return chamfer_launch<1024, 0>(s, rows, cols, phi, level, inclusive, dx, sdf, nimg);
-    default: return cudaErrorInvalidValue;
-  }
-}
-
 cudaError_t launch_dt(cudaStream_t s, const float* vn, size_t n, float dx, float dy, float cfl,
                       float b, float* part, float* vmax, float* dt, int* bad) {
   int nb = (int)((n + LS_NT - 1) / LS_NT);

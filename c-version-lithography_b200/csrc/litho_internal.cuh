@@ -376,11 +376,11 @@ cudaError_t launch_render_mask(cudaStream_t s, const float* phi, int rows, int c
 cudaError_t launch_dt(cudaStream_t s, const float* vn, size_t n, float dx, float dy, float cfl,
                       float b, float* part, float* vmax, float* dt, int* bad);
 // Chamfer signed distance of reinit_sdf over nimg rows x cols images back to back:
-// inside = phi > level (phi >= level when inclusive); sdf must not alias phi.
-// threads: CTA size (128 or 256 for rows of up to 32 columns per thread, 1024; 0 picks
-// by the row length).
+// inside = phi > level (phi >= level when inclusive); sdf must not alias phi. mask
+// (nullable): sdf >= 0. threads: CTA size of the row search (128, 256, 512 or 1024; 0: 256).
 cudaError_t launch_reinit_sdf(cudaStream_t s, int rows, int cols, const float* phi, float level,
-                              int inclusive, float dx, float* sdf, int nimg = 1, int threads = 0);
+                              int inclusive, float dx, float* sdf, float* mask, int nimg = 1,
+                              int threads = 0);
 // Fills nimg rows x cols images with a pattern whose zero set crosses every row.
 cudaError_t launch_chamfer_probe(cudaStream_t s, float* p, int rows, int cols, int nimg);
 // max |Vn| and dt of nimg images of n pixels: vd[2 i] = max |Vn_i|, vd[2 i + 1] = dt_i;
