@@ -105,6 +105,7 @@ bool finite_all(const double* p, size_t n) {
 
 // Reduction slots in ctx->d_red: [0] flag (as int), partial sums after 8.
 constexpr int RED_FLAG = 0;
+constexpr int RED_COUNT = 1;  // CTA counter of the single-image dt
 constexpr int RED_SUM = 2;    // summed results (up to 4 doubles)
 constexpr int RED_PART = 8;   // per-block partials
 
@@ -1587,20 +1588,22 @@ int litho_kappa(litho_ctx* ctx, int rows, int cols, const float* d_phi, double d
   return st;
 }
 
+// Reduction slots (doubles) of n images' (max |Vn|, dt) pairs and their CTA counters.
+static size_t dt_slots(int n) { return (size_t)n + ((size_t)n + 1) / 2; }
+
 static int ls_dt(litho_ctx* ctx, int rows, int cols, const float* d_vn, double dx, double dy,
                  double cfl, double b, float** dt_dev) {
   int st = ctx->ensure_red(RED_PART + 2 * 600);
   if (st) return st;
   LITHO_CUDA_TRY(ctx, cudaMemsetAsync(ctx->d_red, 0, RED_PART * sizeof(double), ctx->stream));
-  float* part = reinterpret_cast<float*>(ctx->d_red + RED_PART);
-  float* vmax = reinterpret_cast<float*>(ctx->d_red + RED_SUM);
-  float* dt = vmax + 1;
-  st = check_launch(ctx, launch_dt(ctx->stream, d_vn, (size_t)rows * cols, (float)dx, (float)dy,
-                                   (float)cfl, (float)b, part, vmax, dt,
-                                   reinterpret_cast<int*>(ctx->d_red + RED_FLAG)),
+  float* vd = reinterpret_cast<float*>(ctx->d_red + RED_SUM);   // max |Vn|, dt
+  st = check_launch(ctx, launch_speed_dt(ctx->stream, d_vn, (size_t)rows * cols, 1, (float)dx,
+                                         (float)dy, (float)cfl, (float)b, vd,
+                                         reinterpret_cast<unsigned*>(ctx->d_red + RED_COUNT),
+                                         reinterpret_cast<int*>(ctx->d_red + RED_FLAG)),
                     "dt");
-  ctx->launches += 2;
-  *dt_dev = dt;
+  ctx->launches += 1;
+  *dt_dev = vd + 1;
   return st;
 }
 
@@ -1654,8 +1657,7 @@ int litho_ctx_reserve(litho_ctx* ctx, const litho_cache* cache, int batch) {
   const size_t n = (size_t)cache->g.N * cache->g.N;
   st = ctx->ensure_scratch(std::max(L.total, n * batch * sizeof(float)));
   if (st) return st;
-  st = ctx->ensure_red(RED_PART + ((size_t)batch * dt_batch_blocks(n, batch) + 1) / 2 + 8 +
-                       (size_t)batch + 8);
+  st = ctx->ensure_red(RED_PART + std::max(dt_slots(batch), (size_t)batch + 8));
   if (!st) st = ctx->ensure_deferred();
   if (st) return st;
   LITHO_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
@@ -1917,32 +1919,31 @@ static int rk2_update_batch_impl(litho_ctx* ctx, int batch, int rows, int cols,
   const size_t n = (size_t)rows * cols;
   st = ctx->ensure_scratch(n * batch * sizeof(float));
   if (st) return st;
-  // Per-image absmax partials, then the per-image (max |Vn|, dt) pairs.
-  const size_t nparts = (size_t)batch * dt_batch_blocks(n, batch);
-  const size_t part_dbl = (nparts + 1) / 2 + 8;
-  st = ctx->ensure_red(RED_PART + part_dbl + (size_t)batch + 8);
+  // The per-image (max |Vn|, dt) pairs and CTA counters, cleared with the header.
+  st = ctx->ensure_red(RED_PART + dt_slots(batch));
   if (st) return st;
-  LITHO_CUDA_TRY(ctx, cudaMemsetAsync(ctx->d_red, 0, RED_PART * sizeof(double), ctx->stream));
+  LITHO_CUDA_TRY(ctx, cudaMemsetAsync(ctx->d_red, 0, (RED_PART + dt_slots(batch)) * sizeof(double),
+                                      ctx->stream));
   float* phi1 = static_cast<float*>(ctx->scratch.base);
-  float* part = reinterpret_cast<float*>(ctx->d_red + RED_PART);
-  float* vd = reinterpret_cast<float*>(ctx->d_red + RED_PART + part_dbl);   // [batch][2]
+  float* vd = reinterpret_cast<float*>(ctx->d_red + RED_PART);   // [batch][2]
+  unsigned* count = reinterpret_cast<unsigned*>(ctx->d_red + RED_PART + batch);
   int* bad = reinterpret_cast<int*>(ctx->d_red + RED_FLAG);
   cudaStream_t s = ctx->stream;
   // Every image in each launch: dt per image, then the two RK2 stages with dt[2 i + 1].
-  st = check_launch(ctx, launch_dt_batch(s, d_vn, n, batch, (float)dx, (float)dy, (float)cfl,
-                                         (float)b, part, vd, bad),
+  st = check_launch(ctx, launch_speed_dt(s, d_vn, n, batch, (float)dx, (float)dy, (float)cfl,
+                                         (float)b, vd, count, bad),
                     "dt");
   if (!st)
     st = check_launch(ctx, launch_levelset(s, 3, rows, cols, d_phi, nullptr, d_vn, (float)dx,
-                                           (float)dy, (float)b, vd + 1, phi1, nullptr, nullptr,
-                                           batch, nullptr, 2),
+                                           (float)dy, (float)b, vd + 1, phi1, nullptr, batch,
+                                           nullptr, 2),
                       "rk2 stage 1");
   if (!st)
     st = check_launch(ctx, launch_levelset(s, 4, rows, cols, phi1, d_phi, d_vn, (float)dx,
-                                           (float)dy, (float)b, vd + 1, d_phi_out, d_mask, nullptr,
-                                           batch, nullptr, 2),
+                                           (float)dy, (float)b, vd + 1, d_phi_out, d_mask, batch,
+                                           nullptr, 2),
                       "rk2 stage 2");
-  ctx->launches += 4;
+  ctx->launches += 3;
   if (device_out) {
     if (!st && d_dts) {
       dt_export_kernel<<<(batch + 255) / 256, 256, 0, s>>>(vd, batch, d_dts);
@@ -2769,15 +2770,14 @@ int litho_fullchip_lsm_step(litho_ctx* ctx, const litho_partition* p, const floa
       1, std::min<size_t>({(size_t)n, (size_t)65535, ((size_t)512 << 20) / (2 * tt * sizeof(float))}));
   int st = ctx->ensure_scratch(2 * (size_t)G * tt * sizeof(float));
   if (st) return st;
-  const size_t part_dbl = (std::max<size_t>(1184, (size_t)G) + 1) / 2 + 8;  // absmax partials
-  st = ctx->ensure_red(RED_PART + part_dbl + (size_t)n + 8);
+  st = ctx->ensure_red(RED_PART + dt_slots(n));
   if (st) return st;
   float* vw = static_cast<float*>(ctx->scratch.base);  // windowed speed of the chunk
   float* phi1 = vw + (size_t)G * tt;                   // RK2 stage 1, then the reinit distance
   cudaStream_t s = ctx->stream;
-  LITHO_CUDA_TRY(ctx, cudaMemsetAsync(ctx->d_red, 0, RED_PART * sizeof(double), s));
-  float* part = reinterpret_cast<float*>(ctx->d_red + RED_PART);
-  float* vd = reinterpret_cast<float*>(ctx->d_red + RED_PART + part_dbl);  // [tile][max |V|, dt]
+  LITHO_CUDA_TRY(ctx, cudaMemsetAsync(ctx->d_red, 0, (RED_PART + dt_slots(n)) * sizeof(double), s));
+  float* vd = reinterpret_cast<float*>(ctx->d_red + RED_PART);  // [tile][max |V|, dt]
+  unsigned* count = reinterpret_cast<unsigned*>(ctx->d_red + RED_PART + n);
   int* bad = reinterpret_cast<int*>(ctx->d_red + RED_FLAG);
   const int* wins = p->d_meta + p->off_update;                            // update_local per tile
   for (int t0 = 0; t0 < n && !st; t0 += G) {
@@ -2787,21 +2787,21 @@ int litho_fullchip_lsm_step(litho_ctx* ctx, const litho_partition* p, const floa
     const int* w = wins + 4 * (size_t)t0;
     float* dtd = vd + 2 * (size_t)t0 + 1;
     st = check_launch(ctx, launch_levelset(s, 6, ts, ts, ph, nullptr, d_grad + t0 * tt, (float)dx,
-                                           (float)dy, 0.f, nullptr, vw, nullptr, nullptr, B, w, 0),
+                                           (float)dy, 0.f, nullptr, vw, nullptr, B, w, 0),
                       "windowed speed");
     if (!st)
-      st = check_launch(ctx, launch_dt_batch(s, vw, tt, B, (float)dx, (float)dy, (float)cfl,
-                                             (float)b, part, vd + 2 * (size_t)t0, bad),
+      st = check_launch(ctx, launch_speed_dt(s, vw, tt, B, (float)dx, (float)dy, (float)cfl,
+                                             (float)b, vd + 2 * (size_t)t0, count + t0, bad),
                         "dt");
     if (!st)
       st = check_launch(ctx, launch_levelset(s, 3, ts, ts, ph, nullptr, vw, (float)dx, (float)dy,
-                                             (float)b, dtd, phi1, nullptr, nullptr, B, w, 2),
+                                             (float)b, dtd, phi1, nullptr, B, w, 2),
                         "rk2 stage 1");
     if (!st)
       st = check_launch(ctx, launch_levelset(s, 4, ts, ts, phi1, ph, vw, (float)dx, (float)dy,
-                                             (float)b, dtd, out, nullptr, nullptr, B, w, 2),
+                                             (float)b, dtd, out, nullptr, B, w, 2),
                         "rk2 stage 2");
-    ctx->launches += 5;
+    ctx->launches += 4;
   }
   // reinit_sdf of the +-0.5 sign image of phi >= 0 (full_chip_lsm.cpp:229-230) of every
   // tile at once: the chamfer transform with inside = phi >= 0, into the mask buffer
@@ -2815,7 +2815,7 @@ int litho_fullchip_lsm_step(litho_ctx* ctx, const litho_partition* p, const floa
     if (!st)
       st = check_launch(ctx, launch_levelset(s, 8, ts, ts, d_masks + t0 * tt, d_phi_out + t0 * tt,
                                              nullptr, (float)dx, (float)dy, 0.f, nullptr,
-                                             d_phi_out + t0 * tt, nullptr, nullptr, B,
+                                             d_phi_out + t0 * tt, nullptr, B,
                                              wins + 4 * (size_t)t0, 0),
                         "window commit");
     ctx->launches += 3;

@@ -14,107 +14,141 @@
 
 namespace litho_b200 {
 
-constexpr int LS_TX = 32;      // tile width (x, columns)
-constexpr int LS_TY = 8;       // rows per pass of the CTA; each thread computes LS_RPT rows
-constexpr int LS_RPT = 4;
-constexpr int LS_H = 3;        // halo
-constexpr int LS_SW = LS_TX + 2 * LS_H;
-constexpr int LS_SH = LS_TY * LS_RPT + 2 * LS_H;
-constexpr int LS_NT = LS_TX * LS_TY;
-static_assert(LS_TX == 32 && LS_SW <= 64, "the tile loader maps one warp to one tile row");
+constexpr int LS_PX = 2;             // a thread computes blocks of LS_PX x 2 pixels
+constexpr int LS_TX = 32 * LS_PX;    // tile width (x, columns): one warp
+constexpr int LS_TY = 8;             // rows per pass of the CTA (4 warps x 2 rows)
+constexpr int LS_H = 3;              // halo rows
+constexpr int LS_HX = 4;             // halo columns on each side (3 used; keeps pairs aligned)
+constexpr int LS_SW = LS_TX + 2 * LS_HX;
+constexpr int LS_NT = 128;
+constexpr int LS_ET = 256;           // threads of the elementwise and reduction kernels
+// CTAs of tall tiles from which they are used (at least four per SM).
+constexpr int LS_TALL_CTAS = 592;
+static_assert(LS_SW % 4 == 0, "tile rows are 16-byte aligned");
 
-// WENO5-JS one-sided derivative from the five differences v1..v5 (already divided by
-// the spacing), level_set_utils.cpp:45-113, for two stencils at once: lane x of the
-// result is the derivative of (v1.x .. v5.x), lane y that of (v1.y .. v5.y). The
-// arithmetic is packed FP32x2 (sm_100 FFMA2 / FMUL2 / FADD2: one instruction for both
-// lanes, each lane rounded as the scalar operation), which halves the instructions of
-// this part of an issue-bound stencil. The smoothness indicators are scaled by
-// 1/max(v^2) before forming the weights: the weights are invariant under that scaling
-// (eps = 1e-6 max v^2 scales the same way) and the scaled values stay inside FP32
-// range. alpha_i = gamma_i / S_i^2 and the result sum(alpha_i d_i) / sum(alpha_i) are
-// both multiplied by S1^2 S2^2 S3^2 (one division instead of four; the scaled S_i lie
-// in [1e-6, 34], so the products stay well inside FP32 range). __fdividef (within 2
-// ulp) serves the reciprocal and the division: max v^2 and the weight sum stay far
-// inside the range where it is accurate.
 __device__ __forceinline__ float2 f2(float a) { return make_float2(a, a); }
-__device__ __forceinline__ float2 weno5x2(float2 v1, float2 v2, float2 v3, float2 v4, float2 v5) {
-  const float2 d1 = __ffma2_rn(f2(11.f / 6.f), v3, __ffma2_rn(f2(-7.f / 6.f), v2, __fmul2_rn(f2(1.f / 3.f), v1)));
-  const float2 d2 = __ffma2_rn(f2(1.f / 3.f), v4, __ffma2_rn(f2(5.f / 6.f), v3, __fmul2_rn(f2(-1.f / 6.f), v2)));
-  const float2 d3 = __ffma2_rn(f2(-1.f / 6.f), v5, __ffma2_rn(f2(5.f / 6.f), v4, __fmul2_rn(f2(1.f / 3.f), v3)));
-  const float2 s1 = __fmul2_rn(v1, v1), s2 = __fmul2_rn(v2, v2), s3 = __fmul2_rn(v3, v3);
-  const float2 s4 = __fmul2_rn(v4, v4), s5 = __fmul2_rn(v5, v5);
-  const float mx = fmaxf(fmaxf(fmaxf(s1.x, s2.x), fmaxf(s3.x, s4.x)), s5.x);
-  const float my = fmaxf(fmaxf(fmaxf(s1.y, s2.y), fmaxf(s3.y, s4.y)), s5.y);
-  // all differences of a lane zero: its candidates are zero, and so is its result
-  // (inv = 0 keeps its weights finite)
-  const float2 inv = make_float2(mx > 0.f ? __fdividef(1.f, mx) : 0.f,
-                                 my > 0.f ? __fdividef(1.f, my) : 0.f);
-  const float2 t1 = __fadd2_rn(__ffma2_rn(f2(-2.f), v2, v1), v3);
-  const float2 t2 = __fadd2_rn(__ffma2_rn(f2(-2.f), v3, v2), v4);
-  const float2 t3 = __fadd2_rn(__ffma2_rn(f2(-2.f), v4, v3), v5);
-  const float2 q1 = __ffma2_rn(f2(3.f), v3, __ffma2_rn(f2(-4.f), v2, v1));
-  const float2 q2 = __ffma2_rn(f2(-1.f), v4, v2);
-  const float2 q3 = __fadd2_rn(__ffma2_rn(f2(-4.f), v4, __fmul2_rn(f2(3.f), v3)), v5);
-  auto smooth = [&](float2 t, float2 q) {
-    const float2 a = __fmul2_rn(__fmul2_rn(f2(13.f / 12.f), t), t);
-    return __ffma2_rn(__ffma2_rn(__fmul2_rn(f2(0.25f), q), q, a), inv, f2(1e-6f));
+__device__ __forceinline__ float2 sub2(float2 a, float2 b) { return __ffma2_rn(b, f2(-1.f), a); }
+// Reciprocal within 1 ulp of a normal x (the callers keep x normal).
+__device__ __forceinline__ float rcp_normal(float x) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+__device__ __forceinline__ float2 rcp2(float2 x) { return make_float2(rcp_normal(x.x), rcp_normal(x.y)); }
+
+// sqrt(x), x >= 0, within 1 ulp, without the branches of the IEEE one.
+__device__ __forceinline__ float sqrt_normal(float x) {
+  float r;
+  asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+
+// WENO5-JS one-sided derivatives (level_set_utils.cpp:45-113) of N neighbouring pixels along
+// one axis, for the two lanes of packed FP32x2 arithmetic at once: D[i .. i + 5] are the
+// undivided differences around pixel i (D[i + 2], D[i + 3] next to it). The results m[i]
+// (minus) and p[i] (plus) are undivided too: the weights do not depend on the spacing.
+//
+// Minus of pixel i and plus of pixel i - 1 are the two mirrored stencils over the same five
+// differences (window i), so they share the smoothness indicators, their normaliser and the
+// products of the weights. With e_i = D_{i+1} - D_i and t_i = e_{i+1} - e_i the indicators
+// of the triples T_i = (D_i, D_{i+1}, D_{i+2}), T_{i+1}, T_{i+2} are 13/12 t^2 + 1/4 q^2, with
+//   q = t_i + 2 e_{i+1}, e_{i+1} + e_{i+2}, t_{i+2} - 2 e_{i+2},
+// and the candidates are a difference plus multiples of its triple's two e. Two pixels take
+// 127 packed instructions for their 8 derivatives; evaluated one stencil at a time they
+// took 4 x 55.
+//
+// The indicators (scaled by 12/13, and eps with them) are divided by the window's max D^2
+// before the weights, which are invariant under that; the scaled values stay inside FP32
+// range. alpha_i = gamma_i / S_i^2 and sum(alpha_i d_i) / sum(alpha_i) are both multiplied
+// by 10 S1^2 S2^2 S3^2: one division, of values in [1e-24, 1e8]. A window of differences
+// below 1e-18 counts as 1e-18: its weights only mix values of that size.
+template <int N>
+__device__ __forceinline__ void weno5_chain(const float2 (&D)[N + 5], float2 (&m)[N], float2 (&p)[N]) {
+  float2 e[N + 4], t[N + 3], t2[N + 3];
+#pragma unroll
+  for (int i = 0; i < N + 4; ++i) e[i] = sub2(D[i + 1], D[i]);
+#pragma unroll
+  for (int i = 0; i < N + 3; ++i) {
+    t[i] = sub2(e[i + 1], e[i]);
+    t2[i] = __fmul2_rn(t[i], t[i]);
+  }
+  auto cand = [&](float2 d, float ca, float2 ea, float cb, float2 eb) {
+    return __ffma2_rn(f2(cb), eb, __ffma2_rn(f2(ca), ea, d));
   };
-  const float2 S1 = smooth(t1, q1), S2 = smooth(t2, q2), S3 = smooth(t3, q3);
-  const float2 w1 = __fmul2_rn(S1, S1), w2 = __fmul2_rn(S2, S2), w3 = __fmul2_rn(S3, S3);
-  const float2 b1 = __fmul2_rn(f2(0.1f), __fmul2_rn(w2, w3));
-  const float2 b2 = __fmul2_rn(f2(0.6f), __fmul2_rn(w1, w3));
-  const float2 b3 = __fmul2_rn(f2(0.3f), __fmul2_rn(w1, w2));
-  const float2 num = __ffma2_rn(b3, d3, __ffma2_rn(b2, d2, __fmul2_rn(b1, d1)));
-  const float2 den = __fadd2_rn(__fadd2_rn(b1, b2), b3);
-  return make_float2(__fdividef(num.x, den.x), __fdividef(num.y, den.y));
-}
-
-// Godunov |grad phi| for the sign of the normal speed (level_set_utils.cpp:180-213).
-__device__ __forceinline__ float godunov(float speed, float xm, float xp, float ym, float yp) {
-  float gx2 = 0.f, gy2 = 0.f;
-  if (speed > 0.f) {
-    const float a = fmaxf(xm, 0.f), b = fminf(xp, 0.f);
-    const float c = fmaxf(ym, 0.f), d = fminf(yp, 0.f);
-    gx2 = fmaxf(a * a, b * b);
-    gy2 = fmaxf(c * c, d * d);
-  } else if (speed < 0.f) {
-    const float a = fminf(xm, 0.f), b = fmaxf(xp, 0.f);
-    const float c = fminf(ym, 0.f), d = fmaxf(yp, 0.f);
-    gx2 = fmaxf(a * a, b * b);
-    gy2 = fmaxf(c * c, d * d);
+  // the triples' central candidates: of T_i from its left (two upwind) and right neighbour
+  float2 cA[N + 2], cB[N + 2];
+#pragma unroll
+  for (int i = 1; i < N + 1; ++i) {
+    cA[i] = cand(D[i + 1], 1.f / 6.f, e[i], 1.f / 3.f, e[i + 1]);
+    cB[i + 1] = cand(D[i + 2], -1.f / 3.f, e[i + 1], -1.f / 6.f, e[i + 2]);
   }
-  return sqrtf(gx2 + gy2);
+  static_assert(N == 2, "three windows around D[2 .. 4]");
+  const float2 mid = make_float2(fmaxf(fmaxf(fabsf(D[2].x), fabsf(D[3].x)), fmaxf(fabsf(D[4].x), 1e-18f)),
+                                 fmaxf(fmaxf(fabsf(D[2].y), fabsf(D[3].y)), fmaxf(fabsf(D[4].y), 1e-18f)));
+#pragma unroll
+  for (int i = 0; i <= N; ++i) {
+    // the largest |D| of the window: its three middle ones and two of (left, right) ends
+    const float2 top = make_float2(
+        i < 2 ? fmaxf(fmaxf(mid.x, fabsf(D[1].x)), fabsf(D[i ? 5 : 0].x)) : fmaxf(fmaxf(mid.x, fabsf(D[5].x)), fabsf(D[6].x)),
+        i < 2 ? fmaxf(fmaxf(mid.y, fabsf(D[1].y)), fabsf(D[i ? 5 : 0].y)) : fmaxf(fmaxf(mid.y, fabsf(D[5].y)), fabsf(D[6].y)));
+    const float2 inv = rcp2(__fmul2_rn(top, top));
+    auto smooth = [&](float2 q, float2 tt) {
+      return __ffma2_rn(__ffma2_rn(__fmul2_rn(q, q), f2(3.f / 13.f), tt), inv, f2(1e-6f * 12.f / 13.f));
+    };
+    const float2 s1 = smooth(__ffma2_rn(f2(2.f), e[i + 1], t[i]), t2[i]);
+    const float2 s2 = smooth(__fadd2_rn(e[i + 1], e[i + 2]), t2[i + 1]);
+    const float2 s3 = smooth(__ffma2_rn(f2(-2.f), e[i + 2], t[i + 2]), t2[i + 2]);
+    const float2 p1 = __fmul2_rn(s2, s3), p2 = __fmul2_rn(s1, s3), p3 = __fmul2_rn(s1, s2);
+    const float2 b1 = __fmul2_rn(p1, p1), b2 = __fmul2_rn(f2(6.f), __fmul2_rn(p2, p2)),
+                 b3 = __fmul2_rn(p3, p3);
+    auto blend = [&](float2 w1, float2 w3, float2 d1, float2 d2, float2 d3) {
+      const float2 w = __fmul2_rn(f2(3.f), w3);
+      const float2 num = __ffma2_rn(w, d3, __ffma2_rn(b2, d2, __fmul2_rn(w1, d1)));
+      return __fmul2_rn(num, rcp2(__fadd2_rn(__fadd2_rn(w1, b2), w)));
+    };
+    if (i < N)
+      m[i] = blend(b1, b3, cand(D[i + 2], -1.f / 3.f, e[i], 5.f / 6.f, e[i + 1]), cA[i + 1], cB[i + 2]);
+    if (i > 0)
+      p[i - 1] = blend(b3, b1, cand(D[i + 2], -5.f / 6.f, e[i + 2], 1.f / 3.f, e[i + 3]), cB[i + 1], cA[i]);
+  }
 }
 
+// Godunov's one-sided slope along an axis for the sign of the normal speed
+// (level_set_utils.cpp:180-213): of (minus, plus), max(m, 0) and -min(p, 0) where the
+// speed is positive, max(-m, 0) and -min(-p, 0) where it is negative; the larger counts.
+__device__ __forceinline__ float godunov(float sign, float m, float p) {
+  return fmaxf(fmaxf(sign * m, -sign * p), 0.f);
+}
+
+// Tile rows y0 - LS_H .. , columns x0 - LS_HX ..: every index clamped into the image.
+template <int SH>
 __device__ __forceinline__ void load_tile(float (*t)[LS_SW], const float* __restrict__ phi,
-                                          int rows, int cols, int y0, int x0) {
-  // warp w loads tile rows w, w + 8, ...; each lane columns lane and lane + 32
-  const int lane = threadIdx.x & 31;
-  const int xa = min(max(x0 - LS_H + lane, 0), cols - 1);
-  const int xb = min(max(x0 - LS_H + lane + 32, 0), cols - 1);
-  for (int ty = threadIdx.x >> 5; ty < LS_SH; ty += LS_NT / 32) {
-    const float* row = phi + (size_t)min(max(y0 - LS_H + ty, 0), rows - 1) * cols;
-    t[ty][lane] = __ldg(row + xa);
-    if (lane + 32 < LS_SW) t[ty][lane + 32] = __ldg(row + xb);
+                                          int rows, int cols, int y0, int x0, bool vec4) {
+  if (vec4 && x0 >= LS_HX && x0 - LS_HX + LS_SW <= cols) {
+    constexpr int Q = LS_SW / 4;
+    const float* base = phi + x0 - LS_HX;
+#pragma unroll
+    for (int i0 = 0; i0 < SH * Q; i0 += LS_NT) {
+      const int i = i0 + (int)threadIdx.x;
+      if (i < SH * Q) {
+        const int ty = i / Q, c = 4 * (i - ty * Q);
+        const float* row = base + (size_t)min(max(y0 - LS_H + ty, 0), rows - 1) * cols;
+        *reinterpret_cast<float4*>(&t[ty][c]) = __ldg(reinterpret_cast<const float4*>(row + c));
+      }
+    }
+    return;
   }
-}
-
-// delta = Vn |grad phi|_G at tile pixel (ly, lx) (tile coordinates include the halo).
-__device__ __forceinline__ float weno_delta(const float (*t)[LS_SW], int ly, int lx, float speed,
-                                            float idx, float idy) {
-  float d[6];
+  // warp w loads tile rows w, w + 4, ...; each lane columns lane, lane + 32, lane + 64
+  const int lane = threadIdx.x & 31;
+  int xc[3];
 #pragma unroll
-  for (int q = 0; q < 6; ++q) d[q] = (t[ly][lx - 2 + q] - t[ly][lx - 3 + q]) * idx;
-  // minus: D(j-3..j+1) = d[0..4]; plus: mirrored d[5..1]; both in one packed call
-  const float2 xmp = weno5x2(make_float2(d[0], d[5]), make_float2(d[1], d[4]),
-                             make_float2(d[2], d[3]), make_float2(d[3], d[2]),
-                             make_float2(d[4], d[1]));
-#pragma unroll
-  for (int q = 0; q < 6; ++q) d[q] = (t[ly - 2 + q][lx] - t[ly - 3 + q][lx]) * idy;
-  const float2 ymp = weno5x2(make_float2(d[0], d[5]), make_float2(d[1], d[4]),
-                             make_float2(d[2], d[3]), make_float2(d[3], d[2]),
-                             make_float2(d[4], d[1]));
-  return speed * godunov(speed, xmp.x, xmp.y, ymp.x, ymp.y);
+  for (int k = 0; k < 3; ++k) xc[k] = min(max(x0 - LS_HX + lane + 32 * k, 0), cols - 1);
+  for (int ty = threadIdx.x >> 5; ty < SH; ty += LS_NT / 32) {
+    const float* row = phi + (size_t)min(max(y0 - LS_H + ty, 0), rows - 1) * cols;
+    t[ty][lane] = __ldg(row + xc[0]);
+    t[ty][lane + 32] = __ldg(row + xc[1]);
+    if (lane + 64 < LS_SW) t[ty][lane + 64] = __ldg(row + xc[2]);
+  }
 }
 
 // _gradient_1d along x (level_set_utils.cpp:228-255) at global column x of row ly.
@@ -131,30 +165,26 @@ __device__ __forceinline__ float grad_y(const float (*t)[LS_SW], int ly, int lx,
   return (t[ly + 1][lx] - t[ly - 1][lx]) * inv2d;
 }
 
-// b * kappa |grad phi| (level_set_utils.cpp:257-278) at global (y, x).
-__device__ float kappa_term(const float (*t)[LS_SW], int ly, int lx, int y, int x, int rows,
-                            int cols, float dx, float dy, float b) {
+// b kappa |grad phi| (level_set_utils.cpp:257-278) from undivided differences (px, py two
+// apart, the second ones differences of those): ix2 = 1 / (2 dx)^2, iy2 alike, kb = b ix2 iy2.
+__device__ __forceinline__ float kappa_value(float px, float py, float pxx, float pxy, float pyy,
+                                             float ix2, float iy2, float kb) {
+  const float px2 = px * px, py2 = py * py;
+  const float g2 = fmaf(px2, ix2, py2 * iy2);
+  const float num = fmaf(pyy, px2, fmaf(-2.f * px * py, pxy, pxx * py2));
+  return g2 > (float)DBL_EPSILON ? kb * num * rcp_normal(g2) : 0.f;
+}
+
+// The same at global (y, x) near the image border, where some differences are one-sided.
+__device__ __noinline__ float kappa_border(const float (*t)[LS_SW], int ly, int lx, int y, int x,
+                                           int rows, int cols, float dx, float dy, float b) {
   const float ix = 1.f / (2.f * dx), iy = 1.f / (2.f * dy);
-  float px, py, pxy, pxx, pyy;
-  if (x >= 2 && x < cols - 2 && y >= 2 && y < rows - 2) {
-    // Away from the image border every difference below is the central one: the
-    // same arithmetic as the general path, without its border tests.
-    auto cx = [&](int oy, int ox) { return (t[ly + oy][lx + ox + 1] - t[ly + oy][lx + ox - 1]) * ix; };
-    auto cy = [&](int oy) { return (t[ly + oy + 1][lx] - t[ly + oy - 1][lx]) * iy; };
-    px = cx(0, 0);
-    py = cy(0);
-    pxy = (cx(1, 0) - cx(-1, 0)) * iy;
-    pxx = (cx(0, 1) - cx(0, -1)) * ix;
-    pyy = (cy(1) - cy(-1)) * iy;
-    const float g2 = px * px + py * py;
-    const float num = pxx * py * py - 2.f * px * py * pxy + pyy * px * px;
-    return g2 > (float)DBL_EPSILON ? b * __fdividef(num, g2) : 0.f;
-  }
+  float pxy, pxx, pyy;
   // phi_x at (y, x) and its row/column neighbours used by the second derivatives.
   auto px_at = [&](int oy, int ox) { return grad_x(t, ly + oy, lx + ox, x + ox, cols, ix); };
   auto py_at = [&](int oy) { return grad_y(t, ly + oy, lx, y + oy, rows, iy); };
-  px = px_at(0, 0);
-  py = py_at(0);
+  const float px = px_at(0, 0);
+  const float py = py_at(0);
   if (y == 0) pxy = (-3.f * px + 4.f * px_at(1, 0) - px_at(2, 0)) * iy;
   else if (y == rows - 1) pxy = (3.f * px - 4.f * px_at(-1, 0) + px_at(-2, 0)) * iy;
   else pxy = (px_at(1, 0) - px_at(-1, 0)) * iy;
@@ -169,23 +199,11 @@ __device__ float kappa_term(const float (*t)[LS_SW], int ly, int lx, int y, int 
   return g2 > (float)DBL_EPSILON ? b * __fdividef(num, g2) : 0.f;
 }
 
-__device__ float block_max(float v, float* sh) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
-  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = v;
-  __syncthreads();
-  float r = 0.f;
-  if (threadIdx.x == 0)
-    for (int w = 0; w < LS_NT / 32; ++w) r = fmaxf(r, sh[w]);
-  __syncthreads();
-  return r;
-}
-
 // what: 0 = delta (+ habs), 1 = kappa term, 2 = normal = kappa - delta,
 // 3 = RK2 stage 1: out = phi0 + dt N(phi0), 4 = RK2 stage 2:
 // out = 0.5 phi0 + 0.5 (phi1 + dt N(phi1)), mask_out = out >= 0.
 struct LsArgs {
-  int rows, cols, what;
+  int rows, cols;
   const float* phi;   // field whose stencil is evaluated
   const float* phi0;  // stage 2: the step's starting phi
   const float* vn;
@@ -193,182 +211,341 @@ struct LsArgs {
   const float* dt;    // device scalar (stages)
   float* out;
   float* out2;        // habs (what 0) or mask (what 4)
-  int wy0, wy1, wx0, wx1;  // update window [wy0, wy1) x [wx0, wx1) (stages 3, 4 and what 6, 8)
   // Batched launches: image blockIdx.z of rows x cols images back to back; its dt at
-  // dt[blockIdx.z * dt_stride]; its window from wins[4 blockIdx.z ..] when wins is set.
+  // dt[blockIdx.z * dt_stride]; its update window {y0, y1, x0, x1} (stages 3, 4 and what
+  // 6, 8) at wins + 4 blockIdx.z, the whole image when wins is null.
   const int* wins;
   int dt_stride;
+  int vec4, vec2;     // 16-byte loads of phi rows; 8-byte accesses of pixel pairs elsewhere
 };
 
-// WHAT (the mode, LsArgs::what) is a template parameter so that the per-pixel loop
-// carries no mode tests.
-template <int WHAT>
-__global__ void __launch_bounds__(LS_NT) levelset_kernel(LsArgs a) {
+// Stencil modes 0-4. A CTA computes LS_TX x (LS_TY RPT) pixels from a tile in shared
+// memory, each thread RPT blocks of 2 x 2 pixels: packed FP32x2 lanes are the two rows
+// along x and the two columns along y, and neighbouring pixels of a block share their
+// smoothness indicators and candidates (weno5_chain). The stencil is bound by FP32 issue
+// (a packed instruction takes the issue port and the FMA pipe twice): 176-197 thread
+// instructions per pixel and stage, 82 of them packed, against 422-443 for one pixel per
+// thread. Stages of 16 images of 2048^2: 932 -> 486 us and 1005 -> 535 us (1.9 and 2.0 TB/s).
+// Longer strips fed by cp.async one pass ahead removed the wait for the tile but cost as
+// many instructions as they hid (1.24 against 1.23 ms per update at that stage), and scalar
+// FFMA on blocks of 2 x 4 pixels ran out of registers and instruction cache (1.6 ms).
+template <int WHAT, int RPT, bool WIN>
+__global__ void __launch_bounds__(LS_NT, RPT == 1 ? 6 : 7) levelset_kernel(LsArgs a) {
+  constexpr int SH = LS_TY * RPT + 2 * LS_H;
+  __shared__ __align__(16) float t[SH][LS_SW];
   const size_t img = (size_t)blockIdx.z * a.rows * a.cols;
   const float* phi = a.phi + img;
   float* out = a.out + img;
-  int wy0 = a.wy0, wy1 = a.wy1, wx0 = a.wx0, wx1 = a.wx1;
-  if (a.wins) {
+  int wy0 = 0, wy1 = 0, wx0 = 0, wx1 = 0;   // WIN: the image's update window
+  if (WIN) {
     const int* w = a.wins + 4 * (size_t)blockIdx.z;
     wy0 = w[0]; wy1 = w[1]; wx0 = w[2]; wx1 = w[3];
   }
-  if (WHAT >= 5) {  // elementwise modes
-    const int x = blockIdx.x * LS_TX + threadIdx.x % LS_TX;
-    for (int r = 0; r < LS_RPT; ++r) {
-      const int y = blockIdx.y * LS_TY * LS_RPT + threadIdx.x / LS_TX + r * LS_TY;
-      if (y < a.rows && x < a.cols) {
-        const size_t i = (size_t)y * a.cols + x;
-        const bool in = y >= wy0 && y < wy1 && x >= wx0 && x < wx1;
-        if (WHAT == 5)         // printed mask: phi >= 0 (LSM_Optimizer.cpp:128)
-          out[i] = phi[i] >= 0.f ? 1.f : 0.f;
-        else if (WHAT == 6)    // speed restricted to the update window
-          out[i] = in ? a.vn[img + i] : 0.f;
-        else if (WHAT == 7)    // +-0.5 sign image of phi >= 0 (full_chip_lsm.cpp:229-230)
-          out[i] = phi[i] >= 0.f ? 0.5f : -0.5f;
-        else if (WHAT == 9)    // mask - 0.5 (full_chip_lsm.cpp:143)
-          out[i] = phi[i] - 0.5f;
-        else                     // commit phi inside the window over phi0 (out may be phi0)
-          out[i] = in ? phi[i] : a.phi0[img + i];
-      }
-    }
-    return;
-  }
-  __shared__ float t[LS_SH][LS_SW];
-  const int x0 = blockIdx.x * LS_TX;
-  const int y0 = blockIdx.y * LS_TY * LS_RPT;
-  load_tile(t, phi, a.rows, a.cols, y0, x0);
-  __syncthreads();
-  const float idx = 1.f / a.dx, idy = 1.f / a.dy;
-  const float dt = (WHAT >= 3) ? a.dt[(size_t)blockIdx.z * a.dt_stride] : 0.f;
+  const int x0 = blockIdx.x * LS_TX, y0 = blockIdx.y * (LS_TY * RPT);
   const float* phi0 = a.phi0 ? a.phi0 + img : nullptr;
   const float* vn = a.vn ? a.vn + img : nullptr;
   float* out2 = a.out2 ? a.out2 + img : nullptr;
-  const int lx = threadIdx.x % LS_TX;
-  for (int r = 0; r < LS_RPT; ++r) {
-    const int ly = threadIdx.x / LS_TX + r * LS_TY;
-    const int y = y0 + ly, x = x0 + lx;
-    if (y >= a.rows || x >= a.cols) continue;
-    const size_t i = (size_t)y * a.cols + x;
-    if (WHAT >= 3 && !(y >= wy0 && y < wy1 && x >= wx0 && x < wx1)) {
-      // Outside the update window the step keeps phi (stage 1) / the starting phi (stage 2).
-      const float keep = WHAT == 3 ? t[ly + LS_H][lx + LS_H] : __ldg(phi0 + i);
-      if (WHAT == 4 && out2) out2[i] = keep >= 0.f ? 1.f : 0.f;
-      out[i] = keep;
-      continue;
-    }
-    const float speed = WHAT == 1 ? 0.f : __ldg(vn + i);
-    float v;
-    if (WHAT == 0) {
-      v = weno_delta(t, ly + LS_H, lx + LS_H, speed, idx, idy);
-      if (out2) out2[i] = fabsf(speed);
-    } else if (WHAT == 1) {
-      v = kappa_term(t, ly + LS_H, lx + LS_H, y, x, a.rows, a.cols, a.dx, a.dy, a.b);
+  const int lx = 2 * (threadIdx.x & 31), x = x0 + lx;
+  const bool pair = x + 1 < a.cols;       // both columns of the block lie in the image
+  const bool v2 = pair && a.vec2;
+  auto load2 = [&](const float* p, size_t i) -> float2 {
+    if (v2) return __ldg(reinterpret_cast<const float2*>(p + i));
+    return make_float2(__ldg(p + i), pair ? __ldg(p + i + 1) : 0.f);
+  };
+  auto store2 = [&](float* p, size_t i, float2 v) {
+    if (v2) {
+      *reinterpret_cast<float2*>(p + i) = v;
     } else {
-      const float n = kappa_term(t, ly + LS_H, lx + LS_H, y, x, a.rows, a.cols, a.dx, a.dy, a.b) -
-                      weno_delta(t, ly + LS_H, lx + LS_H, speed, idx, idy);
-      if (WHAT == 2) {
-        v = n;
-      } else if (WHAT == 3) {
-        v = t[ly + LS_H][lx + LS_H] + dt * n;
-      } else {
-        v = 0.5f * __ldg(phi0 + i) + 0.5f * (t[ly + LS_H][lx + LS_H] + dt * n);
-        if (out2) out2[i] = v >= 0.f ? 1.f : 0.f;
+      p[i] = v.x;
+      if (pair) p[i + 1] = v.y;
+    }
+  };
+  // The normal speed of a block, [row](x, x + 1), loaded one pass ahead of its use.
+  float2 sp_n[2] = {f2(0.f), f2(0.f)};
+  auto fetch = [&](int r) {
+    const int y = y0 + 2 * (threadIdx.x >> 5) + r * LS_TY;
+    const size_t i = (size_t)y * a.cols + x;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      if (x < a.cols && y + h < a.rows) {
+        if (WHAT != 1) sp_n[h] = load2(vn, i + (size_t)h * a.cols);
+        // the starting phi, read at the end of the pass: its line into L2 by then
+        if (WHAT == 4 && (threadIdx.x & 15) == 0)
+          asm volatile("prefetch.global.L2 [%0];" ::"l"(phi0 + i + (size_t)h * a.cols));
       }
     }
-    out[i] = v;
+  };
+  fetch(0);
+  load_tile<SH>(t, phi, a.rows, a.cols, y0, x0, a.vec4 != 0);
+  __syncthreads();
+  const float idx = 1.f / a.dx, idy = 1.f / a.dy;
+  const float ix2 = 0.25f * idx * idx, iy2 = 0.25f * idy * idy, kb = a.b * ix2 * iy2;
+  const float dt = (WHAT >= 3) ? a.dt[(size_t)blockIdx.z * a.dt_stride] : 0.f;
+  if (x >= a.cols) return;
+#pragma unroll 1
+  for (int r = 0; r < RPT; ++r) {
+    const int ly = 2 * (threadIdx.x >> 5) + r * LS_TY, y = y0 + ly;
+    if (y >= a.rows) break;
+    const bool two = y + 1 < a.rows;        // both rows lie in the image
+    const size_t i0 = (size_t)y * a.cols + x, i1 = i0 + a.cols;
+    float2 ph[2] = {f2(0.f), f2(0.f)};      // stage 2: the starting phi, used last
+    if (WHAT == 4) {
+      ph[0] = load2(phi0, i0);
+      if (two) ph[1] = load2(phi0, i1);
+    }
+    const float* c = &t[ly + LS_H][lx + LS_HX];   // pixel (y, x); row stride LS_SW
+    auto at2 = [&](int oy, int ox) { return *reinterpret_cast<const float2*>(c + oy * LS_SW + ox); };
+    const float2 sp[2] = {sp_n[0], sp_n[1]};
+    if (r + 1 < RPT) fetch(r + 1);
+    if (WIN && (y + 1 < wy0 || y >= wy1 || x + 1 < wx0 || x >= wx1)) {
+      // Outside the update window the step keeps phi (stage 1) / the starting phi (stage 2).
+      for (int h = 0; h < (two ? 2 : 1); ++h) {
+        const size_t i = h ? i1 : i0;
+        const float2 keep = WHAT == 3 ? at2(h, 0) : ph[h];
+        if (WHAT == 4 && out2)
+          store2(out2, i, make_float2(keep.x >= 0.f ? 1.f : 0.f, keep.y >= 0.f ? 1.f : 0.f));
+        store2(out, i, keep);
+      }
+      continue;
+    }
+    // rows y, y + 1, columns x - 4 .. x + 5
+    float ra[10], rb[10];
+#pragma unroll
+    for (int k = 0; k < 5; ++k) {
+      const float2 p = at2(0, 2 * k - 4), q = at2(1, 2 * k - 4);
+      ra[2 * k] = p.x; ra[2 * k + 1] = p.y;
+      rb[2 * k] = q.x; rb[2 * k + 1] = q.y;
+    }
+    // columns x, x + 1, rows y - 3 .. y + 4
+    float2 col[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k)
+      col[k] = k == 3 ? make_float2(ra[4], ra[5]) : k == 4 ? make_float2(rb[4], rb[5]) : at2(k - 3, 0);
+    float2 kap[2] = {f2(0.f), f2(0.f)};
+    if (WHAT != 0) {
+      if (x >= 2 && x + 1 < a.cols - 2 && y >= 2 && y + 1 < a.rows - 2) {
+        // Every difference is central. d(y, x) = phi(y, x + 1) - phi(y, x - 1) of columns x
+        // and x + 1 on the rows y - 1 .. y + 2; along x, d of x + 1 is also the step from x.
+        const float2 up = at2(-1, -2), un = at2(-1, 2), dp = at2(2, -2), dn = at2(2, 2);
+        const float2 dm = make_float2(col[2].y - up.y, un.x - col[2].x);   // row y - 1
+        const float2 da = make_float2(ra[5] - ra[3], ra[6] - ra[4]);       // row y
+        const float2 db = make_float2(rb[5] - rb[3], rb[6] - rb[4]);       // row y + 1
+        const float2 dd = make_float2(col[5].y - dp.y, dn.x - col[5].x);   // row y + 2
+        const float2 pyA = sub2(col[4], col[2]), pyB = sub2(col[5], col[3]);
+        const float2 pyyA = sub2(pyB, sub2(col[3], col[1])), pyyB = sub2(sub2(col[6], col[4]), pyA);
+        const float2 pxyA = sub2(db, dm), pxyB = sub2(dd, da);
+        const float2 pxxA = make_float2(da.y - (ra[4] - ra[2]), (ra[7] - ra[5]) - da.x);
+        const float2 pxxB = make_float2(db.y - (rb[4] - rb[2]), (rb[7] - rb[5]) - db.x);
+        kap[0].x = kappa_value(da.x, pyA.x, pxxA.x, pxyA.x, pyyA.x, ix2, iy2, kb);
+        kap[0].y = kappa_value(da.y, pyA.y, pxxA.y, pxyA.y, pyyA.y, ix2, iy2, kb);
+        kap[1].x = kappa_value(db.x, pyB.x, pxxB.x, pxyB.x, pyyB.x, ix2, iy2, kb);
+        kap[1].y = kappa_value(db.y, pyB.y, pxxB.y, pxyB.y, pyyB.y, ix2, iy2, kb);
+      } else {
+        for (int h = 0; h < (two ? 2 : 1); ++h) {
+          kap[h].x = kappa_border(t, ly + h + LS_H, lx + LS_HX, y + h, x, a.rows, a.cols, a.dx,
+                                  a.dy, a.b);
+          if (pair)
+            kap[h].y = kappa_border(t, ly + h + LS_H, lx + 1 + LS_HX, y + h, x + 1, a.rows, a.cols,
+                                    a.dx, a.dy, a.b);
+        }
+      }
+    }
+    float2 del[2] = {f2(0.f), f2(0.f)};     // Vn |grad phi|
+    if (WHAT != 1) {
+      const float2 sg0 = make_float2(sp[0].x < 0.f ? -1.f : 1.f, sp[0].y < 0.f ? -1.f : 1.f);
+      const float2 sg1 = make_float2(sp[1].x < 0.f ? -1.f : 1.f, sp[1].y < 0.f ? -1.f : 1.f);
+      float2 g[2];
+      {
+        float2 D[7];
+#pragma unroll
+        for (int k = 0; k < 7; ++k) D[k] = make_float2(ra[k + 2] - ra[k + 1], rb[k + 2] - rb[k + 1]);
+        float2 m[2], p[2];   // [column], lanes rows
+        weno5_chain<2>(D, m, p);
+        g[0] = make_float2(godunov(sg0.x, m[0].x, p[0].x) * idx, godunov(sg0.y, m[1].x, p[1].x) * idx);
+        g[1] = make_float2(godunov(sg1.x, m[0].y, p[0].y) * idx, godunov(sg1.y, m[1].y, p[1].y) * idx);
+      }
+      {
+        float2 D[7];
+#pragma unroll
+        for (int k = 0; k < 7; ++k) D[k] = sub2(col[k + 1], col[k]);
+        float2 m[2], p[2];   // [row], lanes columns
+        weno5_chain<2>(D, m, p);
+        auto length = [&](float gx, float sgn, float mi, float pl) {
+          const float gy = godunov(sgn, mi, pl) * idy;
+          return sqrt_normal(fmaf(gx, gx, gy * gy));
+        };
+        del[0] = make_float2(sp[0].x * length(g[0].x, sg0.x, m[0].x, p[0].x),
+                             sp[0].y * length(g[0].y, sg0.y, m[0].y, p[0].y));
+        del[1] = make_float2(sp[1].x * length(g[1].x, sg1.x, m[1].x, p[1].x),
+                             sp[1].y * length(g[1].y, sg1.y, m[1].y, p[1].y));
+      }
+    }
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      if (h && !two) break;
+      const size_t i = h ? i1 : i0;
+      float2 v;
+      if (WHAT == 0) {
+        v = del[h];
+        if (out2) store2(out2, i, make_float2(fabsf(sp[h].x), fabsf(sp[h].y)));
+      } else if (WHAT == 1) {
+        v = kap[h];
+      } else {
+        const float2 n = sub2(kap[h], del[h]);
+        if (WHAT == 2) {
+          v = n;
+        } else {
+          const float2 here = col[3 + h];
+          const float2 start = WHAT == 4 ? ph[h] : here;
+          v = make_float2(here.x + dt * n.x, here.y + dt * n.y);
+          if (WHAT == 4) v = make_float2(0.5f * start.x + 0.5f * v.x, 0.5f * start.y + 0.5f * v.y);
+          if (WIN) {
+            const bool in_y = y + h >= wy0 && y + h < wy1;
+            if (!(in_y && x >= wx0 && x < wx1)) v.x = start.x;
+            if (!(in_y && x + 1 >= wx0 && x + 1 < wx1)) v.y = start.y;
+          }
+          if (WHAT == 4 && out2)
+            store2(out2, i, make_float2(v.x >= 0.f ? 1.f : 0.f, v.y >= 0.f ? 1.f : 0.f));
+        }
+      }
+      store2(out, i, v);
+    }
   }
 }
 
-static dim3 ls_grid(int rows, int cols) {
-  return dim3((cols + LS_TX - 1) / LS_TX, (rows + LS_TY * LS_RPT - 1) / (LS_TY * LS_RPT));
+// Elementwise modes: 6 speed restricted to the update window, 8 phi inside the window over
+// phi0 outside (out may be phi0).
+template <int WHAT>
+__global__ void __launch_bounds__(LS_ET) window_kernel(LsArgs a) {
+  const size_t img = (size_t)blockIdx.z * a.rows * a.cols;
+  const int* w = a.wins + 4 * (size_t)blockIdx.z;
+  const int wy0 = w[0], wy1 = w[1], wx0 = w[2], wx1 = w[3];
+  const int x = blockIdx.x * 32 + threadIdx.x % 32;
+  for (int r = 0; r < 4; ++r) {
+    const int y = blockIdx.y * 32 + threadIdx.x / 32 + 8 * r;
+    if (y < a.rows && x < a.cols) {
+      const size_t i = img + (size_t)y * a.cols + x;
+      const bool in = y >= wy0 && y < wy1 && x >= wx0 && x < wx1;
+      if (WHAT == 6) a.out[i] = in ? a.vn[i] : 0.f;
+      else a.out[i] = in ? a.phi[i] : a.phi0[i];
+    }
+  }
+}
+
+template <int WHAT, int RPT>
+static void ls_launch_t(cudaStream_t s, const LsArgs& a, int nimg) {
+  const dim3 g((a.cols + LS_TX - 1) / LS_TX, (a.rows + LS_TY * RPT - 1) / (LS_TY * RPT), nimg);
+  if constexpr (WHAT >= 3) {
+    if (a.wins) {
+      levelset_kernel<WHAT, RPT, true><<<g, LS_NT, 0, s>>>(a);
+      return;
+    }
+  }
+  levelset_kernel<WHAT, RPT, false><<<g, LS_NT, 0, s>>>(a);
+}
+
+template <int WHAT>
+static void ls_launch(cudaStream_t s, const LsArgs& a, int nimg) {
+  // Tall tiles (fewer halo rows per pixel) where they fill the GPU, else one pass per CTA.
+  const long long tall = (long long)((a.cols + LS_TX - 1) / LS_TX) *
+                         ((a.rows + 4 * LS_TY - 1) / (4 * LS_TY)) * nimg;
+  if (tall >= LS_TALL_CTAS) ls_launch_t<WHAT, 4>(s, a, nimg);
+  else ls_launch_t<WHAT, 1>(s, a, nimg);
 }
 
 cudaError_t launch_levelset(cudaStream_t s, int what, int rows, int cols, const float* phi,
                             const float* phi0, const float* vn, float dx, float dy, float b,
-                            const float* dt, float* out, float* out2, const int* window,
-                            int nimg, const int* d_windows, int dt_stride) {
+                            const float* dt, float* out, float* out2, int nimg,
+                            const int* d_windows, int dt_stride) {
   if (nimg < 1 || nimg > 65535) return cudaErrorInvalidValue;
-  LsArgs a{rows, cols, what, phi, phi0, vn, dx, dy, b, dt, out, out2, 0, rows, 0, cols,
-           d_windows, dt_stride};
-  if (window) {
-    a.wy0 = window[0]; a.wy1 = window[1]; a.wx0 = window[2]; a.wx1 = window[3];
-  }
-  dim3 g = ls_grid(rows, cols);
-  g.z = nimg;
+  auto aligned = [](const void* p, size_t n) { return reinterpret_cast<uintptr_t>(p) % n == 0; };
+  LsArgs a{rows, cols, phi, phi0, vn, dx, dy, b, dt, out, out2, d_windows,
+           dt_stride, cols % 4 == 0 && aligned(phi, 16),
+           cols % 2 == 0 && aligned(phi0, 8) && aligned(vn, 8) && aligned(out, 8) && aligned(out2, 8)};
+  const dim3 flat((cols + 31) / 32, (rows + 31) / 32, nimg);
   switch (what) {
-    case 0: levelset_kernel<0><<<g, LS_NT, 0, s>>>(a); break;
-    case 1: levelset_kernel<1><<<g, LS_NT, 0, s>>>(a); break;
-    case 2: levelset_kernel<2><<<g, LS_NT, 0, s>>>(a); break;
-    case 3: levelset_kernel<3><<<g, LS_NT, 0, s>>>(a); break;
-    case 4: levelset_kernel<4><<<g, LS_NT, 0, s>>>(a); break;
-    case 5: levelset_kernel<5><<<g, LS_NT, 0, s>>>(a); break;
-    case 6: levelset_kernel<6><<<g, LS_NT, 0, s>>>(a); break;
-    case 7: levelset_kernel<7><<<g, LS_NT, 0, s>>>(a); break;
-    case 8: levelset_kernel<8><<<g, LS_NT, 0, s>>>(a); break;
-    case 9: levelset_kernel<9><<<g, LS_NT, 0, s>>>(a); break;
+    case 0: ls_launch<0>(s, a, nimg); break;
+    case 1: ls_launch<1>(s, a, nimg); break;
+    case 2: ls_launch<2>(s, a, nimg); break;
+    case 3: ls_launch<3>(s, a, nimg); break;
+    case 4: ls_launch<4>(s, a, nimg); break;
+    case 6: window_kernel<6><<<flat, LS_ET, 0, s>>>(a); break;
+    case 8: window_kernel<8><<<flat, LS_ET, 0, s>>>(a); break;
     default: return cudaErrorInvalidValue;
   }
   return cudaGetLastError();
 }
 
-// max |Vn| partials then dt = get_dt_normal_kappa (level_set_utils.cpp:280-288).
-__global__ void __launch_bounds__(LS_NT) absmax_kernel(const float* __restrict__ v, size_t n,
-                                                       float* __restrict__ part, int* bad) {
-  __shared__ float sh[LS_NT / 32];
-  v += (size_t)blockIdx.y * n;                 // image blockIdx.y of a batched launch
-  part += (size_t)blockIdx.y * gridDim.x;
-  float m = 0.f;
-  bool nonfinite = false;
-  for (size_t i = (size_t)blockIdx.x * LS_NT + threadIdx.x; i < n; i += (size_t)gridDim.x * LS_NT) {
-    const float a = v[i];
-    nonfinite |= !isfinite(a);
+// max |Vn| of image blockIdx.y and its dt = get_dt_normal_kappa (level_set_utils.cpp:280-288)
+// in one launch: vd[2 i] = max |Vn|, vd[2 i + 1] = dt. The CTAs of an image join their
+// maxima with an atomic on the float's bits (|Vn| >= 0 orders as integers), and the last of
+// them to arrive (count[i]) computes dt. vd and count start at zero. A non-finite Vn raises
+// *bad. Bound by HBM reads: four 16-byte loads in flight per thread (16 images of 2048^2:
+// 111 us with one 4-byte load each, 47 us so), and no second launch for dt.
+__global__ void __launch_bounds__(LS_ET) speed_dt_kernel(const float* __restrict__ v, size_t n, int vec,
+                                                         float dx, float dy, float cfl, float b,
+                                                         float* __restrict__ vd,
+                                                         unsigned* __restrict__ count, int* bad) {
+  __shared__ float sh[LS_ET / 32];
+  v += (size_t)blockIdx.y * n;
+  vd += 2 * (size_t)blockIdx.y;
+  float m = 0.f, chk = 0.f;   // chk stays 0 exactly while every value is finite
+  auto take = [&](float a) {
     m = fmaxf(m, fabsf(a));
+    chk = __fmaf_rn(a, 0.f, chk);
+  };
+  const size_t stride = (size_t)gridDim.x * LS_ET, i0 = (size_t)blockIdx.x * LS_ET + threadIdx.x;
+  if (vec) {
+    const float4* v4 = reinterpret_cast<const float4*>(v);
+    const size_t n4 = n / 4;
+    auto take4 = [&](float4 a) { take(a.x); take(a.y); take(a.z); take(a.w); };
+    size_t i = i0;
+    for (; i + 3 * stride < n4; i += 4 * stride) {
+      float4 a[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) a[q] = __ldg(v4 + i + q * stride);
+#pragma unroll
+      for (int q = 0; q < 4; ++q) take4(a[q]);
+    }
+    for (; i < n4; i += stride) take4(__ldg(v4 + i));
+  } else {
+    size_t i = i0;
+    for (; i + 3 * stride < n; i += 4 * stride) {
+      float a[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) a[q] = __ldg(v + i + q * stride);
+#pragma unroll
+      for (int q = 0; q < 4; ++q) take(a[q]);
+    }
+    for (; i < n; i += stride) take(__ldg(v + i));
   }
-  if (nonfinite && bad) atomicOr(bad, 1);
-  const float r = block_max(m, sh);
-  if (threadIdx.x == 0) part[blockIdx.x] = r;
-}
-
-__global__ void dt_kernel(const float* __restrict__ part, int n, float dx, float dy, float cfl,
-                          float b, float* __restrict__ vmax, float* __restrict__ dt) {
-  if (threadIdx.x != 0) return;
-  float m = 0.f;
-  for (int i = 0; i < n; ++i) m = fmaxf(m, part[i]);
-  const double normal = (double)m / dx + (double)m / dy;
-  const double kap = (double)b * (1.0 / ((double)dx * dx) + 1.0 / ((double)dy * dy)) * 2.0;
-  const double den = normal + kap;
-  *vmax = m;
-  *dt = den < 1e-9 ? 1e-3f : (float)(cfl / den);
-}
-
-// dt of every image of a batched launch: vd[2 i] = max |Vn|, vd[2 i + 1] = dt.
-__global__ void dt_batch_kernel(const float* __restrict__ part, int nb, float dx, float dy,
-                                float cfl, float b, float* __restrict__ vd) {
-  const float* p = part + (size_t)blockIdx.x * nb;
-  float m = 0.f;
-  for (int i = threadIdx.x; i < nb; i += 32) m = fmaxf(m, p[i]);
+  if (chk != 0.f) atomicOr(bad, 1);   // also true for NaN
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = m;
+  __syncthreads();
   if (threadIdx.x != 0) return;
+  for (int w = 1; w < LS_ET / 32; ++w) m = fmaxf(m, sh[w]);
+  atomicMax(reinterpret_cast<int*>(vd), __float_as_int(m));
+  __threadfence();
+  if (atomicAdd(count + blockIdx.y, 1u) != gridDim.x - 1) return;
+  __threadfence();
+  m = __int_as_float(atomicMax(reinterpret_cast<int*>(vd), 0));
   const double normal = (double)m / dx + (double)m / dy;
   const double kap = (double)b * (1.0 / ((double)dx * dx) + 1.0 / ((double)dy * dy)) * 2.0;
   const double den = normal + kap;
-  vd[2 * (size_t)blockIdx.x] = m;
-  vd[2 * (size_t)blockIdx.x + 1] = den < 1e-9 ? 1e-3f : (float)(cfl / den);
+  vd[1] = den < 1e-9 ? 1e-3f : (float)(cfl / den);
 }
 
-int dt_batch_blocks(size_t n, int nimg) {
-  const size_t want = (n + LS_NT - 1) / LS_NT;
-  const size_t cap = std::max<size_t>(1, 1184 / (size_t)std::max(nimg, 1));
-  return (int)std::max<size_t>(1, std::min(want, cap));
-}
-
-cudaError_t launch_dt_batch(cudaStream_t s, const float* vn, size_t n, int nimg, float dx,
-                            float dy, float cfl, float b, float* part, float* vd, int* bad) {
+cudaError_t launch_speed_dt(cudaStream_t s, const float* vn, size_t n, int nimg, float dx, float dy,
+                            float cfl, float b, float* vd, unsigned* count, int* bad) {
   if (nimg < 1 || nimg > 65535) return cudaErrorInvalidValue;
-  const int nb = dt_batch_blocks(n, nimg);
-  absmax_kernel<<<dim3(nb, nimg), LS_NT, 0, s>>>(vn, n, part, bad);
-  dt_batch_kernel<<<nimg, 32, 0, s>>>(part, nb, dx, dy, cfl, b, vd);
+  const int vec = n % 4 == 0 && reinterpret_cast<uintptr_t>(vn) % 16 == 0;
+  // about 16 values per thread, and at most 8 CTAs per SM in all
+  const size_t want = (n + 16 * LS_ET - 1) / (16 * LS_ET);
+  const size_t cap = std::max<size_t>(1, 1184 / (size_t)nimg);
+  const dim3 grid((unsigned)std::min(want, cap), nimg);
+  speed_dt_kernel<<<grid, LS_ET, 0, s>>>(vn, n, vec, dx, dy, cfl, b, vd, count, bad);
   return cudaGetLastError();
 }
 
@@ -438,15 +615,6 @@ cudaError_t launch_render_mask(cudaStream_t s, const float* phi, int rows, int c
     render_gray_kernel<<<nb, 256, 0, s>>>(phi, rows, cols, nimg, scale, mask);
   else
     render_binary_kernel<<<nb, 256, 0, s>>>(phi, n, mask);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_dt(cudaStream_t s, const float* vn, size_t n, float dx, float dy, float cfl,
-                      float b, float* part, float* vmax, float* dt, int* bad) {
-  int nb = (int)((n + LS_NT - 1) / LS_NT);
-  if (nb > 296) nb = 296;
-  absmax_kernel<<<nb, LS_NT, 0, s>>>(vn, n, part, bad);
-  dt_kernel<<<1, 32, 0, s>>>(part, nb, dx, dy, cfl, b, vmax, dt);
   return cudaGetLastError();
 }
 

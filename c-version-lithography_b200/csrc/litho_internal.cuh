@@ -359,22 +359,18 @@ inline bool tc2_supported(const BandGeom& g) {
 }
 
 // Level set (levelset.cu). what: 0 delta (+|Vn|), 1 kappa term, 2 normal,
-// 3 RK2 stage 1, 4 RK2 stage 2 (+ mask), 5 mask phi >= 0, 6 speed restricted to the
-// window, 7 +-0.5 sign image of phi >= 0, 8 out = phi inside the window, phi0 outside,
-// 9 phi - 0.5.
-// window (host, nullable): {y0, y1, x0, x1}; stages 3 and 4 update only inside it
-// (outside they keep phi / phi0). NULL = the whole grid.
+// 3 RK2 stage 1, 4 RK2 stage 2 (+ mask), 6 speed restricted to the window, 8 out = phi
+// inside the window, phi0 outside. nimg images back to back; d_windows (device, nullable
+// for 0-4; 4 ints per image {y0, y1, x0, x1}): stages 3 and 4 update only inside it
+// (outside they keep phi / phi0). dt of image i at dt[i dt_stride].
 cudaError_t launch_levelset(cudaStream_t s, int what, int rows, int cols, const float* phi,
                             const float* phi0, const float* vn, float dx, float dy, float b,
-                            const float* dt, float* out, float* out2,
-                            const int* window = nullptr, int nimg = 1,
+                            const float* dt, float* out, float* out2, int nimg = 1,
                             const int* d_windows = nullptr, int dt_stride = 0);
 // render_levelset_mask for nimg images of rows x cols: gray = 0 -> phi >= 0,
 // gray = 1 -> subpixel coverage of the scale-times bilinear upsampling.
 cudaError_t launch_render_mask(cudaStream_t s, const float* phi, int rows, int cols, int nimg,
                                int gray, int scale, float* mask);
-cudaError_t launch_dt(cudaStream_t s, const float* vn, size_t n, float dx, float dy, float cfl,
-                      float b, float* part, float* vmax, float* dt, int* bad);
 // Chamfer signed distance of reinit_sdf over nimg rows x cols images back to back:
 // inside = phi > level (phi >= level when inclusive); sdf must not alias phi. mask
 // (nullable): sdf >= 0. threads: CTA size of the row search (128, 256, 512 or 1024; 0: 256).
@@ -383,11 +379,10 @@ cudaError_t launch_reinit_sdf(cudaStream_t s, int rows, int cols, const float* p
                               int threads = 0);
 // Fills nimg rows x cols images with a pattern whose zero set crosses every row.
 cudaError_t launch_chamfer_probe(cudaStream_t s, float* p, int rows, int cols, int nimg);
-// max |Vn| and dt of nimg images of n pixels: vd[2 i] = max |Vn_i|, vd[2 i + 1] = dt_i;
-// part holds nimg * dt_batch_blocks(n, nimg) floats.
-int dt_batch_blocks(size_t n, int nimg);
-cudaError_t launch_dt_batch(cudaStream_t s, const float* vn, size_t n, int nimg, float dx,
-                            float dy, float cfl, float b, float* part, float* vd, int* bad);
+// max |Vn| and dt of nimg images of n pixels: vd[2 i] = max |Vn_i|, vd[2 i + 1] = dt_i; vd
+// and count (one counter per image) must be zero on entry. A non-finite Vn raises *bad.
+cudaError_t launch_speed_dt(cudaStream_t s, const float* vn, size_t n, int nimg, float dx, float dy,
+                            float cfl, float b, float* vd, unsigned* count, int* bad);
 
 // Sparse EPE at host-selected edge points (epe.cu): eps n x 2 (y, x) and weights n,
 // device FP64. signed_epe (nullable) per point; partial: 3 FP64 sums per block

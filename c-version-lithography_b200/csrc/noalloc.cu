@@ -12,10 +12,10 @@ using namespace litho_b200;
 
 namespace {
 
-// Layout of the static scratch, in floats: [0] non-finite flag (int, cleared by
-// every call), [64, 64 + 296) per-block |Vn| maxima, [360] max |Vn|, [361] dt,
-// [512, 512 + LITHO_RK2_NOALLOC_MAX_PIXELS) the first RK2 stage phi1.
-constexpr size_t kFlag = 0, kPart = 64, kVmax = 360, kDt = 361, kPhi1 = 512;
+// Layout of the static scratch, in floats: [0] non-finite flag (int), [1] CTA counter of the
+// |Vn| maximum, [2] max |Vn|, [3] dt (all cleared by every call), [64, 64 +
+// LITHO_RK2_NOALLOC_MAX_PIXELS) the first RK2 stage phi1.
+constexpr size_t kFlag = 0, kCount = 1, kVmax = 2, kDt = 3, kHead = 4, kPhi1 = 64;
 static __device__ __align__(256) float g_rk2_scratch[kPhi1 + LITHO_RK2_NOALLOC_MAX_PIXELS];
 
 constexpr int kMaxDevices = 64;
@@ -60,9 +60,9 @@ extern "C" int litho_lsm_rk2_update_noalloc(void* stream, int rows, int cols, co
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   int* flag = reinterpret_cast<int*>(base + kFlag);
   float* dt_dev = base + kDt;
-  if (cudaMemsetAsync(flag, 0, sizeof(int), s) != cudaSuccess ||
-      launch_dt(s, d_vn, n, (float)dx, (float)dy, (float)cfl, (float)b, base + kPart,
-                base + kVmax, dt_dev, flag) != cudaSuccess ||
+  if (cudaMemsetAsync(base, 0, kHead * sizeof(float), s) != cudaSuccess ||
+      launch_speed_dt(s, d_vn, n, 1, (float)dx, (float)dy, (float)cfl, (float)b, base + kVmax,
+                      reinterpret_cast<unsigned*>(base + kCount), flag) != cudaSuccess ||
       launch_levelset(s, 3, rows, cols, d_phi, nullptr, d_vn, (float)dx, (float)dy, (float)b,
                       dt_dev, base + kPhi1, nullptr) != cudaSuccess ||
       launch_levelset(s, 4, rows, cols, base + kPhi1, d_phi, d_vn, (float)dx, (float)dy,
@@ -70,7 +70,7 @@ extern "C" int litho_lsm_rk2_update_noalloc(void* stream, int rows, int cols, co
     cudaGetLastError();
     return LITHO_ERR_CUDA;
   }
-  float head[kDt + 1];
+  float head[kHead];
   if (cudaMemcpyAsync(head, base, sizeof(head), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
       cudaStreamSynchronize(s) != cudaSuccess) {
     cudaGetLastError();
