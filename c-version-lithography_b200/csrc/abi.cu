@@ -2415,21 +2415,26 @@ int litho_exchange_compute_epe(litho_ctx* ctx, const litho_partition* cp, const 
     LITHO_CUDA_TRY(ctx, cudaMemcpyAsync(ep_in + 2 * (size_t)e.n_eps, e.weights,
                                         (size_t)e.n_eps * sizeof(double), cudaMemcpyHostToDevice, s));
   }
-  st = check_launch(ctx, launch_tiles_extract(s, d_global_target, p->height, p->width, n,
-                                              p->d_meta + p->off_origin, ts, targets),
-                    "target extraction");
   const bool pe_epe = o.loss_type == LITHO_MICRO_LOSS_PE_EPE;
+  // The persistent fused kernel reads the layout itself and forms the windows from the loss
+  // region; EP work, Core metrics and the other schedules take them as images.
+  const bool on_chip = batched && !eval_epe && tc3_fused_supported(cache->g.kp_rows, cache->g.Nc, cache->g.Nr) &&
+                       ctx->tc_persistent(ts, group) &&
+                       (n % group == 0 || ctx->tc_persistent(ts, n % group));
+  const int* region_meta = p->d_meta + (guard_region ? p->off_update : p->off_core_l);
+  if (!on_chip)
+    st = check_launch(ctx, launch_tiles_extract(s, d_global_target, p->height, p->width, n,
+                                                p->d_meta + p->off_origin, ts, targets),
+                      "target extraction");
   if (!st && pe_epe)
     st = check_launch(ctx, launch_dilate_main(s, targets, n, ts, e.main_region_dilation_pixels,
                                               dil_tmp, main_dil),
                       "main-region dilation");
-  if (!st)
-    st = check_launch(ctx, launch_loss_windows(s, targets, n, ts,
-                                               p->d_meta + (guard_region ? p->off_update : p->off_core_l),
-                                               o.loss_type, pe_epe ? main_dil : nullptr, pe_w, pen_w,
-                                               epe_w),
+  if (!st && !on_chip)
+    st = check_launch(ctx, launch_loss_windows(s, targets, n, ts, region_meta, o.loss_type,
+                                               pe_epe ? main_dil : nullptr, pe_w, pen_w, epe_w),
                       "loss windows");
-  ctx->launches += 2 + (pe_epe ? 2 : 0);
+  ctx->launches += (on_chip ? 0 : 2) + (pe_epe ? 2 : 0);
   // micro_loss_weights (micro_gradient_exchange.cpp:95-99).
   const double wpe = o.loss_type == LITHO_MICRO_LOSS_EPE ? 0.0 : o.pe_weight;
   const double wepe = epe_terms ? e.epe_weight : 0.0;
@@ -2511,6 +2516,9 @@ int litho_exchange_compute_epe(litho_ctx* ctx, const litho_partition* cp, const 
   // With an EPE gradient the adjoint needs dL/dI after the EP scatter, so the resist
   // synthesis stores it; otherwise it stays on chip (fused adjoint tile analysis).
   const bool fuse = !epe_grad;
+  const bool copy_in_synth = batched && tc3_synth_supported(cache->g.kp_rows) &&
+                             ctx->tc_persistent(ts, group) &&
+                             (n % group == 0 || ctx->tc_persistent(ts, n % group));
   for (int t0 = 0; batched && t0 < n && !st; t0 += group) {
     // Tiles t0 .. t0 + B - 1 in one pass: windows and penalty in the resist epilogue,
     // raw gradients straight to their slots, per-tile {PE, penalty} sums to the
@@ -2526,9 +2534,18 @@ int litho_exchange_compute_epe(litho_ctx* ctx, const litho_partition* cp, const 
     ep.alpha = (float)alpha;
     ep.aerial = eval_epe ? aerial : nullptr;
     ep.wafer = core ? wafer : nullptr;
-    ep.target = targets + t0 * tt;
-    ep.pe_window = pe_w + t0 * tt;
-    ep.pen_window = pen_w + t0 * tt;
+    if (on_chip) {
+      ep.region = region_meta + 4 * t0;
+      ep.region_main = o.loss_type == LITHO_MICRO_LOSS_PE_PENALTY;
+      ep.layout = d_global_target;
+      ep.layout_h = p->height;
+      ep.layout_w = p->width;
+      ep.origins = p->d_meta + p->off_origin + 2 * t0;
+    } else {
+      ep.target = targets + t0 * tt;
+      ep.pe_window = pe_w + t0 * tt;
+      ep.pen_window = pen_w + t0 * tt;
+    }
     ep.pe_weight = (float)wpe;
     ep.penalty = (float)wpen;
     ep.pen_thr = (float)o.penalty_threshold;
@@ -2570,6 +2587,8 @@ int litho_exchange_compute_epe(litho_ctx* ctx, const litho_partition* cp, const 
                    fuse ? nullptr : dldi_group + b * tt, false);
     GradEpilogue gp{};
     gp.grad_mask = raw + t0 * tt;
+    // the exchanged gradients start as the raw ones
+    if (copy_in_synth) gp.grad_copy = d_grad + t0 * tt;
     if (!st)
       st = run_adjoint(ctx, *cache, fb, L, fuse ? nullptr : dldi_group, adj_scale, gp, &nb2, fuse, B);
   }
@@ -2600,7 +2619,7 @@ int litho_exchange_compute_epe(litho_ctx* ctx, const litho_partition* cp, const 
     int nb2 = 0;
     if (!st) st = run_adjoint(ctx, *cache, f, L, dldi, adj_scale, gp, &nb2);
   }
-  if (!st)
+  if (!st && !copy_in_synth)
     LITHO_CUDA_TRY(ctx, cudaMemcpyAsync(d_grad, raw, n * tt * sizeof(float),
                                         cudaMemcpyDeviceToDevice, s));
   if (!st)

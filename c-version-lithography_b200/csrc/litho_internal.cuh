@@ -270,9 +270,20 @@ struct ResistEpilogue {
   // even when penalty is 0 (it then adds nothing to dL/dI), for the loss the
   // reference's LSM loop tracks (LSM_Optimizer.cpp:87-90).
   int loss_penalty_term;
+  // Full-chip micro tiles, for the persistent fused kernel only (launch_loss_windows and
+  // launch_tiles_extract otherwise): with region set (4 ints {y0, y1, x0, x1} per image) the
+  // windows are those of build_micro_loss_windows inside it, pe = region_main ? [T > 0.5] : 1
+  // and pen = [T < 0.5]; with layout set (layout_h x layout_w, periodic) the target of image
+  // z is its window at origins[2 z], origins[2 z + 1] instead of target + z N N.
+  const int* region;
+  int region_main;
+  const float* layout;
+  const int* origins;
+  int layout_h, layout_w;
 };
 struct GradEpilogue {
   float* grad_mask;         // nullable
+  float* grad_copy;         // nullable: a second copy of grad_mask (persistent synthesis only)
   const float* theta;       // nullable: theta chain when set
   float* grad_theta;        // with theta
   double* norm_partial;     // with theta: per-block partial of sum grad_theta^2

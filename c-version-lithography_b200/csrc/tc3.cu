@@ -27,6 +27,8 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include <type_traits>
+
 #include "device_common.cuh"
 #include "tc_ptx.cuh"
 #include "tc_split2.cuh"
@@ -135,6 +137,12 @@ __device__ __forceinline__ bool epi_take(const EpiSums<NV>& sh, uint32_t red_bar
     for (int w = 0; w < nw; ++w) out[k] += sh.v[b][w][k];
   }
   return true;
+}
+
+// i modulo n for any i (the periodic layout).
+__device__ __forceinline__ int wrapped(int i, int n) {
+  i %= n;
+  return i < 0 ? i + n : i;
 }
 
 // L2 prefetch of the row segment of this lane for a later item: the line holding row
@@ -607,15 +615,16 @@ struct S3Resist {
     }
     return s * W * (1.f - W);
   }
-  __device__ __forceinline__ bool plain() const {
+  __host__ __device__ __forceinline__ bool plain() const {
     return p.pe_window == nullptr && p.pen_window == nullptr && p.penalty == 0.f &&
            !p.loss_penalty_term;
   }
 };
 
 // =============================================================== row synthesis
-// out[y][x] = sum_f AY[y][f] Bt[x][f] with the theta-chain (KIND 0, GradEpilogue) or
-// the resist (KIND 1, ResistEpilogue) epilogue, as launch_synth_grad_tc2 /
+// out[y][x] = sum_f AY[y][f] Bt[x][f] with the theta-chain (KIND 0, GradEpilogue), the
+// resist (KIND 1, ResistEpilogue) or the plain (KIND 2, GradEpilogue without theta: dPE/dM
+// stored once or twice) epilogue, as launch_synth_grad_tc2 /
 // launch_synth_resist_tc2, from a persistent pipeline:
 //   warp 16      (one thread) copies the AY tile (per yt), double-buffers the band
 //                operand tile Bt (per image and xt) and issues D[x][y] into acc[j & 1];
@@ -667,10 +676,10 @@ synth_tc3_kernel(const uint8_t* __restrict__ Aimg, const uint8_t* __restrict__ B
     pdl_wait();
     const int q = warp & 3, h = warp >> 2;
     const uint32_t lane_addr = (uint32_t)(32 * q) << 16;
-    const float* src = KIND == 0 ? g.theta : (r.p.mode == 1 ? r.p.target : nullptr);
+    const float* src = KIND == 0 ? g.theta : KIND == 1 && r.p.mode == 1 ? r.p.target : nullptr;
     const bool plain = KIND == 1 && r.plain();
     // theta chain without the dPE/dM output: the CTM evaluation
-    const bool lean = KIND == 0 && g.theta != nullptr && g.grad_mask == nullptr;
+    const bool lean = KIND == 0 && g.grad_mask == nullptr;
     // per-pixel input, coalesced along x: rows e0 .. e0 + 15 of item j into pre[]
     float pre[32];
     auto load_rows = [&](const Item& it, int e0) {
@@ -695,7 +704,7 @@ synth_tc3_kernel(const uint8_t* __restrict__ Aimg, const uint8_t* __restrict__ B
       load_rows(it, 16);
     }
     if (n > 1) prefetch_item(item_next(it, T, B));
-    const bool sums = KIND == 0 ? g.theta != nullptr : r.p.mode == 1;
+    const bool sums = KIND == 0 || (KIND == 1 && r.p.mode == 1);
     // the partial sums of item i: the squared norm (KIND 0) or the two loss terms
     auto sums_out = [&](const Item& i) {
       const size_t bid = ((size_t)i.z * T + i.yt) * T + i.xt;
@@ -721,7 +730,28 @@ synth_tc3_kernel(const uint8_t* __restrict__ Aimg, const uint8_t* __restrict__ B
       float s0 = 0.f, s1 = 0.f;
       // rows e0 .. e0 + 15; the inputs of the next item load into the rows just used
       auto rows = [&](int e0) {
-        if (lean && full) {
+        if (KIND == 2) {
+          // dPE/dM alone (the second copy is the full chip's raw gradient)
+          float* gp = g.grad_mask + base + (size_t)yb * N + x;
+          float* cp = g.grad_copy ? g.grad_copy + base + (size_t)yb * N + x : nullptr;
+          const int ny = xin ? N - yb : 0;
+          if (full) {
+#pragma unroll
+            for (int e = e0; e < e0 + 16; ++e) gp[e * N] = d[e];
+            if (cp) {
+#pragma unroll
+              for (int e = e0; e < e0 + 16; ++e) cp[e * N] = d[e];
+            }
+          } else {
+#pragma unroll
+            for (int e = e0; e < e0 + 16; ++e) {
+              if (e < ny) {
+                gp[e * N] = d[e];
+                if (cp) cp[e * N] = d[e];
+              }
+            }
+          }
+        } else if (lean && full) {
           float* gp = g.grad_theta + base + (size_t)yb * N + x;
 #pragma unroll
           for (int e = e0; e < e0 + 16; ++e) {
@@ -738,7 +768,7 @@ synth_tc3_kernel(const uint8_t* __restrict__ Aimg, const uint8_t* __restrict__ B
             if (KIND == 0) {
               const float G = d[e];
               if (in && g.grad_mask) g.grad_mask[i] = G;
-              if (g.theta && in) {
+              if (in) {
                 // pixels past the image edge are left out: the band operand's rows there
                 // are not part of the image and may hold anything
                 const float gt = -0.5f * G * fast_sin(pre[e]);
@@ -845,6 +875,8 @@ bool tc3_synth_supported(int kp) { return kp % 16 == 0 && kp <= 128; }
 cudaError_t launch_synth_grad_tc3(cudaStream_t s, const void* Aimg, const void* Bimg, int N,
                                   int kp, const GradEpilogue& ep, int* err, int* nblocks,
                                   int batch) {
+  if (!ep.theta)
+    return synth_tc3_t<2>(s, Aimg, Bimg, N, kp, ep, ResistEpilogue{}, err, nblocks, batch);
   return synth_tc3_t<0>(s, Aimg, Bimg, N, kp, ep, ResistEpilogue{}, err, nblocks, batch);
 }
 
@@ -878,7 +910,11 @@ __host__ __device__ constexpr uint32_t f3_x_bytes(uint32_t tb) {
                                                           : 2 * tb;
 }
 
-template <int BN>
+// MODE 0: no window, no penalty, no image output (the CTM evaluation); 1: windows and
+// penalty; 2: aerial / wafer outputs too. 16 micro tiles of 1280^2 with windows: 435 us when
+// one epilogue served all modes and loaded each pixel's windows in turn, 151 us so; 12 tiles
+// of 1266^2 (19 % of the tiles ragged) 137 -> 116 us with the edge in the packed arithmetic.
+template <int BN, int MODE>
 __global__ void __launch_bounds__(F3_NT, 1)
 fused_tc3_kernel(const uint8_t* __restrict__ Aimg, const uint8_t* __restrict__ Bimg, int N,
                  int kp, int T, int B, S3Resist r, Tc2Analysis a,
@@ -933,8 +969,6 @@ fused_tc3_kernel(const uint8_t* __restrict__ Aimg, const uint8_t* __restrict__ B
     const int lane_base = 32 * q;
     const uint32_t lane_addr = (uint32_t)lane_base << 16;
     const int xl = lane_base + lane;
-    // no window, no penalty, no aerial / wafer output: the CTM evaluation
-    const bool lean = r.plain() && r.p.aerial == nullptr && r.p.wafer == nullptr;
     const int count = a.nrows_out * a.ncols;
     // this thread's four 16-byte chunks of sA (rows y = 32 h + 8 c .. + 7 of column xl)
     uint32_t aoff[4];
@@ -943,17 +977,35 @@ fused_tc3_kernel(const uint8_t* __restrict__ Aimg, const uint8_t* __restrict__ B
     float pre[32];
     auto prefetch = [&](const Item& it) {
       const int x = it.xt * 128 + xl, yb = it.yt * 128 + 32 * h;
-      const float* tp = r.p.target + (size_t)it.z * N * N + (size_t)yb * N + x;
-      if (x < N && yb + 31 < N) {
+      const float* tp;
+      size_t step = N;
+      int wrap = 32;   // row of the segment from which the layout starts again
+      if (r.p.layout) {
+        const int H = r.p.layout_h, W = r.p.layout_w;
+        const int gy = wrapped(__ldg(r.p.origins + 2 * it.z) + yb, H);
+        tp = r.p.layout + (size_t)gy * W + wrapped(__ldg(r.p.origins + 2 * it.z + 1) + x, W);
+        step = W;
+        wrap = H - gy;
+      } else {
+        tp = r.p.target + (size_t)it.z * N * N + (size_t)yb * N + x;
+      }
+      if (x < N && yb + 31 < N && wrap >= 32) {
 #pragma unroll
-        for (int e = 0; e < 32; ++e) pre[e] = __ldg(tp + e * N);
+        for (int e = 0; e < 32; ++e) pre[e] = __ldg(tp + e * step);
+      } else if (r.p.layout) {
+        const int H = r.p.layout_h;
+#pragma unroll
+        for (int e = 0; e < 32; ++e)
+          pre[e] = (x < N && yb + e < N)
+                       ? __ldg(tp + ((ptrdiff_t)e - (ptrdiff_t)((e + H - wrap) / H) * H) * (ptrdiff_t)step)
+                       : 0.f;
       } else {
 #pragma unroll
-        for (int e = 0; e < 32; ++e) pre[e] = (x < N && yb + e < N) ? __ldg(tp + e * N) : 0.f;
+        for (int e = 0; e < 32; ++e) pre[e] = (x < N && yb + e < N) ? __ldg(tp + e * step) : 0.f;
       }
     };
     // the target rows of item i + 2 are fetched into L2 during item i
-    const bool pf = N % 4 == 0 && reinterpret_cast<uintptr_t>(r.p.target) % 16 == 0;
+    const bool pf = !r.p.layout && N % 4 == 0 && reinterpret_cast<uintptr_t>(r.p.target) % 16 == 0;
     Item it = item_at(lo, T, B), ip = it;   // items j and j - 1
     if (n > 0) prefetch(it);
     for (int j = 0; j < n; ++j, ip = it, it = item_next(it, T, B)) {
@@ -976,42 +1028,96 @@ fused_tc3_kernel(const uint8_t* __restrict__ Aimg, const uint8_t* __restrict__ B
       // d[e] becomes dL/dI at (yb + e, x), 0 outside the image.
       float s0 = 0.f, s1 = 0.f;
       bool bad;
-      if (lean && xin && yb + 31 < N) {
+      const int ny = xin ? N - yb : 0;   // rows e < ny lie in the image
+      constexpr bool OUT = MODE == 2;
+      if (MODE == 0) {
         // The window-free arithmetic of S3Resist::dldi on pixel pairs in packed FP32x2
         // (each lane rounded as the scalar operation, in the scalar order, so dL/dI is
         // the per-tile kernels' bit for bit; __expf and the reciprocal stay per lane).
         // Every dL/dI is non-finite exactly when its r is, and then so is the product
-        // with 0 in chk. The loss terms are summed in two interleaved FP32 chains.
+        // with 0 in chk. The loss terms are summed in two interleaved FP32 chains. Past
+        // the image edge r is taken as 0, and with it dL/dI and the loss term.
         float2 chk = make_float2(0.f, 0.f), se = chk;
         const float2 na = make_float2(-r.p.alpha, -r.p.alpha);
         const float2 nt = make_float2(-r.p.thr, -r.p.thr);
         const float2 one = make_float2(1.f, 1.f), pw = make_float2(r.p.pe_weight, r.p.pe_weight);
+        auto pixels = [&](auto edge) {
 #pragma unroll
-        for (int e = 0; e < 32; e += 2) {
-          const float2 z = __fmul2_rn(na, __fadd2_rn(make_float2(d[e], d[e + 1]), nt));
-          const float2 den = __fadd2_rn(one, make_float2(__expf(z.x), __expf(z.y)));
-          const float2 W = make_float2(__fdividef(1.f, den.x), __fdividef(1.f, den.y));
-          const float2 rr = __fadd2_rn(W, make_float2(-pre[e], -pre[e + 1]));
-          se = __ffma2_rn(rr, rr, se);
-          const float2 g = __fmul2_rn(__fmul2_rn(__fmul2_rn(pw, rr), W),
-                                      __fadd2_rn(one, make_float2(-W.x, -W.y)));
-          chk = __ffma2_rn(g, make_float2(0.f, 0.f), chk);
-          d[e] = g.x;
-          d[e + 1] = g.y;
-        }
+          for (int e = 0; e < 32; e += 2) {
+            const float2 z = __fmul2_rn(na, __fadd2_rn(make_float2(d[e], d[e + 1]), nt));
+            const float2 den = __fadd2_rn(one, make_float2(__expf(z.x), __expf(z.y)));
+            float2 W = make_float2(__fdividef(1.f, den.x), __fdividef(1.f, den.y));
+            float2 rr = __fadd2_rn(W, make_float2(-pre[e], -pre[e + 1]));
+            if (decltype(edge)::value) {
+              // the accumulator there may hold anything
+              if (e >= ny) rr.x = W.x = 0.f;
+              if (e + 1 >= ny) rr.y = W.y = 0.f;
+            }
+            se = __ffma2_rn(rr, rr, se);
+            const float2 g = __fmul2_rn(__fmul2_rn(__fmul2_rn(pw, rr), W),
+                                        __fadd2_rn(one, make_float2(-W.x, -W.y)));
+            chk = __ffma2_rn(g, make_float2(0.f, 0.f), chk);
+            d[e] = g.x;
+            d[e + 1] = g.y;
+          }
+        };
+        if (ny >= 32) pixels(std::false_type{});
+        else pixels(std::true_type{});
         s0 = se.x + se.y;
         bad = chk.x + chk.y != 0.f;
       } else {
-        const bool plain = r.plain();
-        bad = false;
-#pragma unroll
-        for (int e = 0; e < 32; ++e) {
-          const int y = yb + e;
-          float gd = 0.f;
-          if (xin && y < N) gd = r.dldi(base + (size_t)y * N + x, d[e], pre[e], plain, s0, s1);
-          bad |= !isfinite(gd);
-          d[e] = gd;
+        // Windows, penalty or image outputs: the scalar arithmetic, eight rows at a time so
+        // that their window loads are in flight together.
+        float chk = 0.f;
+        int ry0 = 0, ry1 = 0;   // the rows e of the loss region
+        if (r.p.region) {
+          const int* R = r.p.region + 4 * it.z;
+          const int x0 = __ldg(R + 2), x1 = __ldg(R + 3);
+          ry0 = __ldg(R) - yb;
+          ry1 = x >= x0 && x < x1 ? __ldg(R + 1) - yb : ry0;
         }
+        const bool pen_on = r.p.penalty != 0.f || r.p.loss_penalty_term;
+        const size_t i0 = base + (size_t)yb * N + x;
+        const float* pwp = r.p.pe_window ? r.p.pe_window + i0 : nullptr;
+        const float* qwp = r.p.pen_window ? r.p.pen_window + i0 : nullptr;
+#pragma unroll
+        for (int e0 = 0; e0 < 32; e0 += 8) {
+          float pw[8], qw[8];
+#pragma unroll
+          for (int e = 0; e < 8; ++e) {
+            if (r.p.region) {
+              const bool in = e0 + e >= ry0 && e0 + e < ry1;
+              pw[e] = in && (!r.p.region_main || pre[e0 + e] > 0.5f) ? 1.f : 0.f;
+              qw[e] = in ? 1.f : 0.f;   // used where T < 0.5
+            } else {
+              pw[e] = pwp && e0 + e < ny ? __ldg(pwp + (e0 + e) * N) : 1.f;
+              qw[e] = qwp && e0 + e < ny ? __ldg(qwp + (e0 + e) * N) : pw[e];
+            }
+          }
+#pragma unroll
+          for (int e = 0; e < 8; ++e) {
+            const float I = d[e0 + e], T = pre[e0 + e];
+            const float W = r.sigmoid(I);
+            const float rr = W - T;
+            float sum = r.p.pe_weight * rr * pw[e], pe = rr * rr * pw[e], pen = 0.f;
+            if (pen_on && T < 0.5f) {
+              const float ex = fmaxf(W - r.p.pen_thr, 0.f);
+              pen = ex * ex * qw[e];
+              sum += r.p.penalty * ex * qw[e];
+            }
+            float g = sum * W * (1.f - W);
+            if (e0 + e >= ny) pe = pen = g = 0.f;   // the accumulator there may hold anything
+            if (OUT && e0 + e < ny) {
+              if (r.p.aerial) r.p.aerial[i0 + (size_t)(e0 + e) * N] = I;
+              if (r.p.wafer) r.p.wafer[i0 + (size_t)(e0 + e) * N] = W;
+            }
+            s0 += pe;
+            s1 += pen;
+            chk = __fmaf_rn(g, 0.f, chk);
+            d[e0 + e] = g;
+          }
+        }
+        bad = chk != 0.f;
       }
       // rows 8 c .. 8 c + 7 of column xl: one 16-byte chunk of hi, one of lo
 #pragma unroll
@@ -1150,24 +1256,34 @@ fused_tc3_kernel(const uint8_t* __restrict__ Aimg, const uint8_t* __restrict__ B
   if (warp == F3_MMAW) tc::tmem_dealloc(tmem, 512);
 }
 
-template <int BN>
-static cudaError_t fused_tc3_t(cudaStream_t s, const void* Aimg, const void* Bimg, int N, int kp,
+template <int BN, int MODE>
+static cudaError_t fused_tc3_m(cudaStream_t s, const void* Aimg, const void* Bimg, int N, int kp,
                                const ResistEpilogue& e, const Tc2Analysis& a, const void* tx,
                                const void* ty, int* err, int* nblocks, int batch) {
   const uint32_t tb = s2_tile_bytes(128, kp);
   const size_t smem = (size_t)f3_x_bytes<BN>(tb) + A2_A_BYTES + s2_tile_bytes(BN, 128) + 1024;
   if (smem > 232448 - 512) return cudaErrorInvalidValue;
-  cudaError_t r = cudaFuncSetAttribute(fused_tc3_kernel<BN>,
+  cudaError_t r = cudaFuncSetAttribute(fused_tc3_kernel<BN, MODE>,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (r != cudaSuccess) return r;
   const int T = (N + 127) / 128;
   const int items = T * T * batch;
   const int grid = items < sm_count() ? items : sm_count();
   *nblocks = T * T;
-  return launch_pdl(fused_tc3_kernel<BN>, dim3(grid), dim3(F3_NT), smem, s,
+  return launch_pdl(fused_tc3_kernel<BN, MODE>, dim3(grid), dim3(F3_NT), smem, s,
                     static_cast<const uint8_t*>(Aimg), static_cast<const uint8_t*>(Bimg), N, kp, T,
                     batch, S3Resist{e}, a, static_cast<const uint8_t*>(tx),
                     static_cast<const uint8_t*>(ty), err);
+}
+template <int BN>
+static cudaError_t fused_tc3_t(cudaStream_t s, const void* Aimg, const void* Bimg, int N, int kp,
+                               const ResistEpilogue& e, const Tc2Analysis& a, const void* tx,
+                               const void* ty, int* err, int* nblocks, int batch) {
+  const bool out = e.aerial || e.wafer;
+  const bool plain = S3Resist{e}.plain() && !e.region;
+  return out ? fused_tc3_m<BN, 2>(s, Aimg, Bimg, N, kp, e, a, tx, ty, err, nblocks, batch)
+         : plain ? fused_tc3_m<BN, 0>(s, Aimg, Bimg, N, kp, e, a, tx, ty, err, nblocks, batch)
+                 : fused_tc3_m<BN, 1>(s, Aimg, Bimg, N, kp, e, a, tx, ty, err, nblocks, batch);
 }
 
 bool tc3_fused_supported(int kp, int ncols, int nr) {
