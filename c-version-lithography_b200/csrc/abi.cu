@@ -76,8 +76,8 @@ Layout make_layout(const BandGeom& g, int batch = 1, bool own_field = false) {
   L.gh = take(B * (2 * g.Nr - 1) * g.Nc * sizeof(float2));
   L.ik = take(B * g.K * g.Pr * g.Pc * sizeof(float));
   L.iP = take(B * g.Pr * g.Pc * sizeof(float));
-  L.Ut = take(B * N * g.kp_rows * sizeof(float));
-  L.Vt = take(B * N * g.kp_rows * sizeof(float));
+  L.Ut = take(B * synth_ld(N) * g.kp_rows * sizeof(float));
+  L.Vt = take(B * synth_ld(N) * g.kp_rows * sizeof(float));
   L.dldi = take((size_t)N * N * sizeof(float));
   L.gam = take(B * g.Pr * g.Pc * sizeof(float));
   L.Zk = take(B * g.K * g.Nr * g.Nc * sizeof(float2));
@@ -387,17 +387,18 @@ int litho_cache_create_band(litho_ctx* ctx, int N, int K, int Nr, int Nc, int ro
       TXDc[(size_t)cidx * N + x] = make_float2((float)re, (float)im);
     }
   std::vector<float2> TYS((size_t)Nr * N), TYD((size_t)Nr * N);
-  std::vector<float> AYS((size_t)N * g.kp_rows, 0.f), AYD((size_t)N * g.kp_rows, 0.f);
+  const size_t ld = (size_t)synth_ld(N);
+  std::vector<float> AYS(ld * g.kp_rows, 0.f), AYD(ld * g.kp_rows, 0.f);
   for (int r = 0; r < Nr; ++r)
     for (int y = 0; y < N; ++y) {
       twiddle(row0 + r, y, N, -1.0, &re, &im);
       TYS[(size_t)r * N + y] = make_float2((float)re, (float)im);
-      AYS[(size_t)y * g.kp_rows + 2 * r] = (float)re;
-      AYS[(size_t)y * g.kp_rows + 2 * r + 1] = (float)im;
+      AYS[2 * r * ld + y] = (float)re;
+      AYS[(2 * r + 1) * ld + y] = (float)im;
       twiddle(r, y, N, -1.0, &re, &im);
       TYD[(size_t)r * N + y] = make_float2((float)re, (float)im);
-      AYD[(size_t)y * g.kp_rows + 2 * r] = (float)re;
-      AYD[(size_t)y * g.kp_rows + 2 * r + 1] = (float)im;
+      AYD[2 * r * ld + y] = (float)re;
+      AYD[(2 * r + 1) * ld + y] = (float)im;
     }
   std::vector<float2> ESr_t((size_t)Nr * g.Pr), ESc_t((size_t)Nc * g.Pc), ESc((size_t)g.Pc * Nc);
   std::vector<float2> EDr_t((size_t)(2 * Nr - 1) * g.Pr), EDc_t((size_t)(2 * Nc - 1) * g.Pc);
@@ -687,7 +688,7 @@ int run_forward(Context* ctx, const Cache& c, Field& f, const Layout& L, int inp
                                                      g.kp_rows, ep, err, nblocks, batch),
                         "tensor-core row synthesis");
   } else {
-    st = check_launch(ctx, launch_synth_resist(s, c.AYD, at<float>(ctx, L.Ut), g.N, g.kp_rows, ep,
+    st = check_launch(ctx, launch_synth_resist(s, c.AYD, at<float>(ctx, L.Ut), g.N, 2 * g.Nr, ep,
                                                nblocks),
                       "row synthesis");
   }
@@ -755,7 +756,7 @@ int run_adjoint(Context* ctx, const Cache& c, const Field& f, const Layout& L, c
                                                    g.kp_rows, ep, err, nblocks, batch),
                         "tensor-core adjoint row synthesis");
   } else {
-    st = check_launch(ctx, launch_synth_grad(s, c.AYS, at<float>(ctx, L.Vt), g.N, g.kp_rows, ep,
+    st = check_launch(ctx, launch_synth_grad(s, c.AYS, at<float>(ctx, L.Vt), g.N, 2 * g.Nr, ep,
                                              nblocks),
                       "adjoint row synthesis");
   }
@@ -769,8 +770,8 @@ int prepare(Context* ctx, const Cache& c, Layout* L, int batch = 1, bool own_fie
   *L = make_layout(c.g, batch, own_field);
   int st = ctx->ensure_scratch(L->total);
   if (st) return st;
-  const int blocks = ((c.g.N + 127) / 128) * ((c.g.N + 127) / 128);
-  st = ctx->ensure_red(RED_PART + (3 * (size_t)blocks + 3) * batch + 1200);
+  // three partial sums per tile of an image: 64 x 64 (FP32 syntheses) at most
+  st = ctx->ensure_red(RED_PART + (3 * (size_t)synth_blocks(c.g.N) + 3) * batch + 1200);
   if (st) return st;
   LITHO_CUDA_TRY(ctx, cudaMemsetAsync(ctx->d_red, 0, RED_PART * sizeof(double), ctx->stream));
   return LITHO_OK;

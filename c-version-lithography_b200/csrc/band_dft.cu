@@ -27,208 +27,236 @@
 
 namespace litho_b200 {
 
-// ---------------------------------------------------------------- GEMM main loop
-// acc[i][j] += sum_{k in [kbeg, kend)} A(m0 + ty*TM + i, k) * B[(n0 + tx + j*BNT) * ldb + k]
-// with 256 threads (BMT x BNT), A produced by a functor (load4 of 4 consecutive k),
-// shared tiles As[BK][BM + 4] (transposed, float4 reads) and Bs[BK][BN + 1].
-template <int BMT, int BNT, int TM, int TN, int BK, class ALoad>
-__device__ __forceinline__ void gemm_mainloop(ALoad& aload, const float* __restrict__ B, int ldb,
-                                              int Nn, int m0, int n0, int kbeg, int kend,
-                                              float* As, float* Bs, float (&acc)[TM][TN]) {
-  constexpr int BM = BMT * TM, BN = BNT * TN, NT = BMT * BNT;
-  constexpr int AS = BM + 4, BS = BN + 1;
-  const int tid = threadIdx.x, tx = tid % BNT, ty = tid / BNT;
-  for (int kt = kbeg; kt < kend; kt += BK) {
-    for (int e = tid; e < BM * (BK / 4); e += NT) {
-      const int mm = e / (BK / 4);
-      const int kq = (e % (BK / 4)) * 4;
-      float v[4];
-      aload.load4(m0 + mm, kt + kq, kend, v);
-#pragma unroll
-      for (int q = 0; q < 4; ++q) As[(kq + q) * AS + mm] = v[q];
-    }
-    for (int e = tid; e < BN * BK; e += NT) {
-      const int nn = e / BK, kk = e % BK;
-      const int gn = n0 + nn, gk = kt + kk;
-      Bs[kk * BS + nn] = (gn < Nn && gk < kend) ? __ldg(B + (size_t)gn * ldb + gk) : 0.f;
-    }
-    __syncthreads();
-#pragma unroll 4
-    for (int kk = 0; kk < BK; ++kk) {
-      float a[TM];
-#pragma unroll
-      for (int i = 0; i < TM; i += 4) {
-        const float4 t = *reinterpret_cast<const float4*>(&As[kk * AS + ty * TM + i]);
-        a[i] = t.x; a[i + 1] = t.y; a[i + 2] = t.z; a[i + 3] = t.w;
-      }
-      float b[TN];
-#pragma unroll
-      for (int j = 0; j < TN; ++j) b[j] = Bs[kk * BS + tx + j * BNT];
-#pragma unroll
-      for (int i = 0; i < TM; ++i)
-#pragma unroll
-        for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
-    }
-    __syncthreads();
-  }
+// Asynchronous copies into shared memory (cp.async); ok = false zero-fills.
+template <int BYTES>
+__device__ __forceinline__ void cp_async(void* dst, const void* src, bool ok) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;" ::"r"(
+                   static_cast<uint32_t>(__cvta_generic_to_shared(dst))),
+               "l"(src), "n"(BYTES), "r"(ok ? BYTES : 0)
+               : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int LEFT>
+__device__ __forceinline__ void cp_async_wait() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(LEFT) : "memory");
 }
 
 // ---------------------------------------------------------------- tile analysis
-// mode 0: A = in;  mode 1: A = (1 + cos(in))/2 (theta -> mask), optional mask_out.
-// Non-finite inputs raise flag[0].
-struct ImageLoad {
-  const float* in;
-  float* mask_out;
-  int* flag;
-  int N;
-  int mode;
-  int vec4;  // rows are 16-byte aligned (N % 4 == 0 and an aligned base pointer)
-  __device__ __forceinline__ void load4(int m, int k, int kend, float* v) {
-    if (vec4 && m < N && k + 3 < kend) {
-      const float4 t = __ldg(reinterpret_cast<const float4*>(in + (size_t)m * N + k));
-      v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w;
-    } else {
-#pragma unroll
-      for (int q = 0; q < 4; ++q)
-        v[q] = (m < N && k + q < kend) ? __ldg(in + (size_t)m * N + k + q) : 0.f;
-    }
-    bool bad = false;
-#pragma unroll
-    for (int q = 0; q < 4; ++q)
-      if (m < N && k + q < kend) bad |= !isfinite(v[q]);
-    if (bad) atomicOr(flag, 1);
-    if (mode == 1) {
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const bool in_range = m < N && k + q < kend;
-        v[q] = in_range ? 0.5f * (1.f + cosf(v[q])) : 0.f;
-        if (mask_out && in_range) mask_out[(size_t)m * N + k + q] = v[q];
-      }
-    }
-  }
-};
-
-constexpr int AT_BMT = 16, AT_BNT = 16, AT_TM = 8, AT_BK = 32, AT_NT = 256;
-constexpr int AT_TILE = AT_BMT * AT_TM;  // 128 rows, and 128 columns of x per tile
-constexpr int AT_RC = 16;                // band rows staged per chunk in phase 2
+// For every 128 x 128 tile: R[y][f] = sum_x A[y][x] tw[f][x] (phase 1, f the real columns
+// Re, Im of the column twiddles), then P[r][c] = sum_y T(r, y) R[y][c] (phase 2), each sum
+// in increasing x or y with fmaf.
+//
+// Both phases are FP32 FMA work (about 120 per pixel and direction at a 35 x 35 band); what
+// bounded them was latency: two CTAs per SM that loaded, waited and computed in turn (FMA
+// pipe 30 % busy). The image block and twiddles of the next 32 columns are now fetched into
+// registers while the current ones are multiplied (two shared buffers, one barrier per
+// block), the row twiddles of phase 2 are copied asynchronously during phase 1 and kept for
+// all rows, and phase 2 gives every thread RPT rows (with their conjugates when sym) x 2
+// columns: 62 and 72 us (forward, adjoint) -> 45 and 45 at 2048^2.
+constexpr int AT_NT = 256, AT_TM = 8, AT_BK = 32;
+constexpr int AT_TILE = 128;             // rows, and columns of x per tile
+constexpr int AT_AS = AT_TILE + 4;       // row stride of an image block [BK][128]
 
 struct AnalysisArgs {
-  ImageLoad ld;
+  const float* in;     // mode 0: A = in;  mode 1: A = (1 + cos(in)) / 2 (theta -> mask)
+  float* mask_out;     // nullable (mode 1)
+  int* flag;           // non-finite inputs raise flag[0]
+  int N, mode;
+  int vec4;            // rows are 16-byte aligned (N % 4 == 0 and an aligned base pointer)
   const float* tw;     // [2 * ncols][N] real rows (Re, Im of the column twiddles)
-  int N, ncols;
+  int ncols;
   const float2* TY;    // [nr][N] row twiddles
   int nrows_out, nr, sym;
   float2* part;        // [tiles][nrows_out][ncols]
 };
 
-template <int BN>
-__device__ void analysis_phase2(float* smem, const AnalysisArgs& a, int y0, int f0, int tile);
+// Row twiddles per shared row [y][ts]: every thread's RPT rows, an odd count (the copies of
+// 32 consecutive y then fall into different banks).
+__host__ __device__ constexpr int at_ts(int nr, int rpt) { return (nr + rpt - 1) / rpt * rpt | 1; }
 
-template <int TN>
-__global__ void __launch_bounds__(AT_NT)
+template <int TN, int RPT>
+__global__ void __launch_bounds__(AT_NT, 2)
 analysis_tile_kernel(AnalysisArgs a) {
   extern __shared__ __align__(16) float smem[];
-  constexpr int BN = AT_BNT * TN;   // real columns (2 per complex frequency)
-  float* As = smem;
-  float* Bs = smem + AT_BK * (AT_TILE + 4);
-  const int tid = threadIdx.x, tx = tid % AT_BNT, ty = tid / AT_BNT;
+  constexpr int BN = 16 * TN;              // real columns of this CTA
+  constexpr int BS = BN + 1, RS = BN + 4;
+  float* As = smem;                                    // [2][BK][AS]
+  float* Bs = smem + 2 * AT_BK * AT_AS;                // [2][BK][BS]
+  float* R = smem;                                     // [128][RS] (after phase 1)
+  constexpr int P1 = 2 * AT_BK * (AT_AS + BS), P2 = AT_TILE * RS;
+  float2* TYs = reinterpret_cast<float2*>(smem + ((P1 > P2 ? P1 : P2) + 3) / 4 * 4);   // [128][ts]
+  const int ts = at_ts(a.nr, RPT);
+  const int tid = threadIdx.x, tx = tid % 16, ty = tid / 16;
   const int x0 = blockIdx.x * AT_TILE, y0 = blockIdx.y * AT_TILE;
   const int f0 = blockIdx.z * BN;
-  const int Nn = 2 * a.ncols;
-  ImageLoad ld = a.ld;
+  const int Nn = 2 * a.ncols, N = a.N;
+  const int nkt = (min(N - x0, AT_TILE) + AT_BK - 1) / AT_BK;
   pdl_trigger();
+  // the row twiddles (constant tables), ready long before phase 2
+  for (int e = tid; e < AT_TILE * ts; e += AT_NT) {
+    const int yy = e % AT_TILE, r = e / AT_TILE;
+    const bool ok = r < a.nr && y0 + yy < N;
+    cp_async<8>(TYs + yy * ts + r, a.TY + (ok ? (size_t)r * N + y0 + yy : 0), ok);
+  }
+  cp_async_commit();
+  float va[16], vb[2 * TN];
+  // image block kt: rows (tid >> 3) + 32 q, columns 4 (tid & 7) ..; twiddle block kt: column
+  // tid % 32 of the rows f tid / 32 + 8 q
+  auto fetch_b = [&](int kt) {
+    const int x = x0 + kt * AT_BK + (tid & 31);
+#pragma unroll
+    for (int q = 0; q < 2 * TN; ++q) {
+      const int f = f0 + (tid >> 5) + 8 * q;
+      vb[q] = f < Nn && x < N ? __ldg(a.tw + (size_t)f * N + x) : 0.f;
+    }
+  };
+  auto fetch_a = [&](int kt) {
+    const int x = x0 + kt * AT_BK + 4 * (tid & 7);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int y = y0 + (tid >> 3) + 32 * q;
+      const float* p = a.in + (size_t)y * N + x;
+      if (a.vec4 && y < N && x + 3 < N) {
+        const float4 t = __ldg(reinterpret_cast<const float4*>(p));
+        va[4 * q] = t.x; va[4 * q + 1] = t.y; va[4 * q + 2] = t.z; va[4 * q + 3] = t.w;
+      } else {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) va[4 * q + e] = (y < N && x + e < N) ? __ldg(p + e) : 0.f;
+      }
+    }
+  };
+  auto store_blocks = [&](int kt) {
+    float* as = As + (kt & 1) * AT_BK * AT_AS;
+    float* bs = Bs + (kt & 1) * AT_BK * BS;
+    const int x = x0 + kt * AT_BK + 4 * (tid & 7);
+    bool bad = false;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int yy = (tid >> 3) + 32 * q, y = y0 + yy;
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        float v = va[4 * q + e];
+        const bool in_range = y < N && x + e < N;
+        bad |= !isfinite(v);   // 0 outside the image
+        if (a.mode == 1) {
+          v = in_range ? 0.5f * (1.f + cosf(v)) : 0.f;
+          if (a.mask_out && in_range && blockIdx.z == 0) a.mask_out[(size_t)y * N + x + e] = v;
+        }
+        as[(4 * (tid & 7) + e) * AT_AS + yy] = v;
+      }
+    }
+    if (bad) atomicOr(a.flag, 1);
+#pragma unroll
+    for (int q = 0; q < 2 * TN; ++q) bs[(tid & 31) * BS + (tid >> 5) + 8 * q] = vb[q];
+  };
+  fetch_b(0);
   pdl_wait();
-
-  // Phase 1: R[y][f] = sum_{x in tile} A[y][x] tw[f][x]  (128 rows x BN real columns).
+  fetch_a(0);
   float acc[AT_TM][TN];
 #pragma unroll
   for (int i = 0; i < AT_TM; ++i)
 #pragma unroll
     for (int j = 0; j < TN; ++j) acc[i][j] = 0.f;
-  gemm_mainloop<AT_BMT, AT_BNT, AT_TM, TN, AT_BK>(ld, a.tw, a.N, Nn, y0, f0, x0,
-                                                  min(a.N, x0 + AT_TILE), As, Bs, acc);
-  // Phase 2 input: R staged as [128][BN + 4] floats.
-  constexpr int RS = BN + 4;
+  store_blocks(0);
+  __syncthreads();
+#pragma unroll 1
+  for (int kt = 0; kt < nkt; ++kt) {
+    if (kt + 1 < nkt) {
+      fetch_a(kt + 1);
+      fetch_b(kt + 1);
+    }
+    const float* as = As + (kt & 1) * AT_BK * AT_AS + ty * AT_TM;
+    const float* bs = Bs + (kt & 1) * AT_BK * BS + tx;
+#pragma unroll 4
+    for (int kk = 0; kk < AT_BK; ++kk) {
+      float av[AT_TM], bv[TN];
+#pragma unroll
+      for (int i = 0; i < AT_TM; i += 4) {
+        const float4 t = *reinterpret_cast<const float4*>(as + kk * AT_AS + i);
+        av[i] = t.x; av[i + 1] = t.y; av[i + 2] = t.z; av[i + 3] = t.w;
+      }
+#pragma unroll
+      for (int j = 0; j < TN; ++j) bv[j] = bs[kk * BS + 16 * j];
+#pragma unroll
+      for (int i = 0; i < AT_TM; ++i)
+#pragma unroll
+        for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(av[i], bv[j], acc[i][j]);
+    }
+    if (kt + 1 < nkt) store_blocks(kt + 1);   // the other buffer: read before the last barrier
+    __syncthreads();
+  }
 #pragma unroll
   for (int i = 0; i < AT_TM; ++i)
 #pragma unroll
-    for (int j = 0; j < TN; ++j) smem[(ty * AT_TM + i) * RS + tx + j * AT_BNT] = acc[i][j];
-  analysis_phase2<BN>(smem, a, y0, f0, blockIdx.y * gridDim.x + blockIdx.x);
-}
-
-// Phase 2 of a tile analysis: P[r][c] = sum_{y in tile} T(r, y) R[y][c] for the
-// tile's rows, R given in smem as [128][BN + 4] floats (complex column c at
-// floats 2c, 2c + 1), as a register-tiled complex product: each thread owns 2
-// band rows x 2 columns. Every thread of the CTA (AT_NT) must call it; it
-// begins with a barrier, so the caller's writes of R need no extra one.
-template <int BN>
-__device__ void analysis_phase2(float* smem, const AnalysisArgs& a, int y0, int f0, int tile) {
-  constexpr int BNC = BN / 2;
-  constexpr int RS = BN + 4;                         // keeps float4 alignment of R rows
-  const float* Rs = smem;                            // [128][RS]
-  float2* TYs = reinterpret_cast<float2*>(smem + AT_TILE * RS);  // [RC][128]
-  const int tid = threadIdx.x;
-  constexpr int CP = BNC / 2;                        // column pairs
-  const int cp = tid % CP, rp = tid / CP;            // rows 2rp, 2rp+1 of each chunk
-  const bool active = rp < AT_RC / 2;
-  const int c0g = f0 / 2 + 2 * cp;                   // first of the two global columns
-  for (int r0 = 0; r0 < a.nrows_out; r0 += AT_RC) {
-    __syncthreads();
-    for (int e = tid; e < AT_RC * AT_TILE; e += AT_NT) {
-      const int r = e / AT_TILE, yy = e % AT_TILE;
-      const int row = r0 + r, y = y0 + yy;
-      float2 t = make_float2(0.f, 0.f);
-      if (row < a.nrows_out && y < a.N) {
-        if (!a.sym) {
-          t = a.TY[(size_t)row * a.N + y];
-        } else {
-          const int d = row - (a.nr - 1);
-          t = d >= 0 ? a.TY[(size_t)d * a.N + y] : conjf2(a.TY[(size_t)(-d) * a.N + y]);
-        }
-      }
-      TYs[r * AT_TILE + yy] = t;
-    }
-    __syncthreads();
-    if (active && r0 + 2 * rp < a.nrows_out) {
-      float2 p00 = make_float2(0.f, 0.f), p01 = p00, p10 = p00, p11 = p00;
-      const float2* t0 = TYs + (2 * rp) * AT_TILE;
-      const float2* t1 = t0 + AT_TILE;
+    for (int j = 0; j < TN; ++j) R[(ty * AT_TM + i) * RS + tx + 16 * j] = acc[i][j];
+  cp_async_wait<0>();
+  __syncthreads();
+  // Phase 2: item (row group, column pair).
+  const int c0 = f0 / 2, npairs = (min(BN / 2, a.ncols - c0) + 1) / 2;
+  const int items = (a.nr + RPT - 1) / RPT * npairs;
+  float2* out = a.part + (size_t)(blockIdx.y * gridDim.x + blockIdx.x) * a.nrows_out * a.ncols;
+  for (int it = tid; it < items; it += AT_NT) {
+    const int r0 = it / npairs * RPT, cp = it % npairs, c = c0 + 2 * cp;
+    float2 p[RPT][2], m[RPT][2];   // rows r, and (sym) their conjugates' rows -r
+#pragma unroll
+    for (int i = 0; i < RPT; ++i) p[i][0] = p[i][1] = m[i][0] = m[i][1] = make_float2(0.f, 0.f);
+    const float2* t0 = TYs + r0;
+    const float* rr = R + 4 * cp;
+    if (!a.sym) {
 #pragma unroll 4
       for (int yy = 0; yy < AT_TILE; ++yy) {
-        const float4 rv = *reinterpret_cast<const float4*>(&Rs[yy * RS + 4 * cp]);
+        const float4 rv = *reinterpret_cast<const float4*>(rr + yy * RS);
         const float2 ra = make_float2(rv.x, rv.y), rb = make_float2(rv.z, rv.w);
-        const float2 ta = t0[yy], tb = t1[yy];
-        cfma(p00, ta, ra);
-        cfma(p01, ta, rb);
-        cfma(p10, tb, ra);
-        cfma(p11, tb, rb);
+#pragma unroll
+        for (int i = 0; i < RPT; ++i) {
+          const float2 t = t0[yy * ts + i];
+          cfma(p[i][0], t, ra);
+          cfma(p[i][1], t, rb);
+        }
       }
-      const int row0 = r0 + 2 * rp;
-      float2* out0 = a.part + ((size_t)tile * a.nrows_out + row0) * a.ncols;  // [tile][row][c]
-      if (c0g < a.ncols) out0[c0g] = p00;
-      if (c0g + 1 < a.ncols) out0[c0g + 1] = p01;
-      if (row0 + 1 < a.nrows_out) {
-        float2* out1 = out0 + a.ncols;
-        if (c0g < a.ncols) out1[c0g] = p10;
-        if (c0g + 1 < a.ncols) out1[c0g + 1] = p11;
+    } else {
+#pragma unroll 2
+      for (int yy = 0; yy < AT_TILE; ++yy) {
+        const float4 rv = *reinterpret_cast<const float4*>(rr + yy * RS);
+        const float2 ra = make_float2(rv.x, rv.y), rb = make_float2(rv.z, rv.w);
+#pragma unroll
+        for (int i = 0; i < RPT; ++i) {
+          const float2 t = t0[yy * ts + i], tc = conjf2(t);
+          cfma(p[i][0], t, ra);
+          cfma(p[i][1], t, rb);
+          cfma(m[i][0], tc, ra);
+          cfma(m[i][1], tc, rb);
+        }
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < RPT; ++i) {
+      const int r = r0 + i;
+      if (r >= a.nr) break;
+      float2* o = out + (size_t)(a.sym ? a.nr - 1 + r : r) * a.ncols + c;
+      o[0] = p[i][0];
+      if (c + 1 < a.ncols) o[1] = p[i][1];
+      if (a.sym && r > 0) {
+        o = out + (size_t)(a.nr - 1 - r) * a.ncols + c;
+        o[0] = m[i][0];
+        if (c + 1 < a.ncols) o[1] = m[i][1];
       }
     }
   }
 }
 
-template <int TN>
+template <int TN, int RPT>
 static cudaError_t analysis_tile_t(cudaStream_t s, const AnalysisArgs& a) {
-  constexpr int BN = AT_BNT * TN;
-  const size_t p1 = (size_t)(AT_BK * (AT_TILE + 4) + AT_BK * (BN + 1)) * sizeof(float);
-  const size_t p2 = (size_t)AT_TILE * (BN + 4) * sizeof(float) +
-                    (size_t)AT_RC * AT_TILE * sizeof(float2);
-  const size_t smem = p1 > p2 ? p1 : p2;
-  cudaError_t e = cudaFuncSetAttribute(analysis_tile_kernel<TN>,
+  constexpr int BN = 16 * TN;
+  constexpr size_t p1 = 2 * AT_BK * (AT_AS + BN + 1), p2 = AT_TILE * (BN + 4);
+  const size_t smem = ((p1 > p2 ? p1 : p2) + 3) / 4 * 4 * sizeof(float) +
+                      (size_t)AT_TILE * at_ts(a.nr, RPT) * sizeof(float2);
+  cudaError_t e = cudaFuncSetAttribute(analysis_tile_kernel<TN, RPT>,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   const int t = (a.N + AT_TILE - 1) / AT_TILE;
   dim3 grid(t, t, (2 * a.ncols + BN - 1) / BN);
-  return launch_pdl(analysis_tile_kernel<TN>, grid, dim3(AT_NT), smem, s, a);
+  return launch_pdl(analysis_tile_kernel<TN, RPT>, grid, dim3(AT_NT), smem, s, a);
 }
 
 int analysis_tiles(int N) {
@@ -239,19 +267,25 @@ int analysis_tiles(int N) {
 // Tile partials of sum_{y, x} T(a, y) A[y][x] tw(c, x) for every 128 x 128 tile:
 // part[tile][a][c], tiles in row-major order of the tile grid (each tile's partials
 // contiguous, so that the tensor-core epilogue writes them as one coalesced block).
+// Tiles below which the columns are split over more CTAs, 8 columns each (256^2: 4 tiles,
+// 76 us per imaging call, 86 with 16 columns each and 90 unsplit), or 16 (1001^2: 64 tiles,
+// forward and adjoint 197 us per gradient call, 211 and 198); 2048^2 has 256 tiles, and there
+// the split repeats the loads and cosines for nothing (276 us against 215 per evaluation).
+constexpr int AT_SMALL = 32, AT_MID = 96;
 cudaError_t launch_analysis(cudaStream_t s, int mode, const float* in, float* mask_out,
                             int* flag, const float* tw, int N, int ncols, const float2* TY,
                             int nrows_out, int nr, int sym, float2* part) {
   const int vec4 = (N % 4 == 0) && (reinterpret_cast<uintptr_t>(in) % 16 == 0);
-  AnalysisArgs a{ImageLoad{in, mask_out, flag, N, mode, vec4}, tw, N, ncols, TY, nrows_out,
-                 nr, sym, part};
-  const int n2 = 2 * ncols;
-  if (n2 <= 32) return analysis_tile_t<2>(s, a);
-  if (n2 <= 48) return analysis_tile_t<3>(s, a);
-  if (n2 <= 64) return analysis_tile_t<4>(s, a);
-  if (n2 <= 80) return analysis_tile_t<5>(s, a);
-  if (n2 <= 96) return analysis_tile_t<6>(s, a);
-  return analysis_tile_t<8>(s, a);
+  const AnalysisArgs a{in, mask_out, flag, N, mode, vec4, tw, ncols, TY, nrows_out, nr, sym, part};
+  const int n2 = 2 * ncols, tiles = analysis_tiles(N);
+  if (tiles < AT_SMALL) return analysis_tile_t<1, 1>(s, a);
+  if (tiles < AT_MID) return analysis_tile_t<2, 2>(s, a);
+  if (n2 <= 32) return analysis_tile_t<2, 2>(s, a);
+  if (n2 <= 48) return analysis_tile_t<3, 3>(s, a);
+  if (n2 <= 64) return analysis_tile_t<4, 3>(s, a);
+  if (n2 <= 80) return analysis_tile_t<5, 3>(s, a);
+  if (n2 <= 96) return analysis_tile_t<6, 3>(s, a);
+  return analysis_tile_t<8, 3>(s, a);
 }
 
 // out[o] = scale * sum_t part[t][o] in a fixed order: RT_G tile groups (group g sums
@@ -300,99 +334,118 @@ cudaError_t launch_reduce_tiles(cudaStream_t s, const float2* part, int tiles, i
 }
 
 // ---------------------------------------------------------------- row synthesis
-// out[y][x] = sum_f AY[y][f] * Bt[x][f] (K = kp) with the epilogue applied to the
-// tile through shared memory in two halves, so that every global access of the
-// epilogue is a coalesced float4 (or scalar at ragged edges).
-struct AYLoad {
-  const float* AY;
-  int N, kp;
-  __device__ __forceinline__ void load4(int m, int k, int kend, float* v) {
-    if (m < N && k + 3 < kend) {
-      const float4 t = __ldg(reinterpret_cast<const float4*>(AY + (size_t)m * kp + k));
-      v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w;
-    } else {
-#pragma unroll
-      for (int q = 0; q < 4; ++q) v[q] = (m < N && k + q < kend) ? AY[(size_t)m * kp + k + q] : 0.f;
-    }
-  }
-};
-
-constexpr int SY_BMT = 16, SY_BNT = 16, SY_TM = 8, SY_TN = 8, SY_BK = 16;
-constexpr int SY_NT = SY_BMT * SY_BNT;
-constexpr int SY_TILE = 128;
-constexpr int SY_SS = SY_TILE + 4;  // staging row stride
+// out[y][x] = sum_f AYt[f][y] * Bt[f][x], f < nf in order with fmaf, from operands stored
+// with f as the slow index (row stride ld, a multiple of 4): 64 x 64 tiles, 4 x 4 pixels per
+// thread. The whole inner dimension of both operands is copied asynchronously in two halves:
+// one wait per half, no other barrier in the product, and several CTAs per SM overlap their
+// copies, products and epilogues. The tile then goes through shared memory, so that every
+// global access of the epilogue is a row of float4 and its code exists once. Half of the
+// kernel's issue slots are the epilogue's (expf, division, sinf, FP64 sums), so the many
+// warps of small thread tiles count for more than the FMAs per operand byte of large ones
+// (8 x 8 pixels per thread: a 2048^2 CTM evaluation 215 us against 206). With 128 x 128 tiles
+// and two barriers per 16 inner columns the two syntheses of 2048^2 took 48 and 47 us (FMA
+// pipe 25 % busy), now 33 and 29; of 256^2 23 us, now 7.
+constexpr int SF_T = 64, SF_NT = 256, SF_SS = SF_T + 4;
 
 template <class Epi>
-__global__ void __launch_bounds__(SY_NT)
-synth_kernel(const float* __restrict__ AY, const float* __restrict__ Bt, int N, int kp, Epi epi) {
-  __shared__ __align__(16) float As[SY_BK * (SY_TILE + 4)];
-  __shared__ float Bs[SY_BK * (SY_TILE + 1)];
-  extern __shared__ __align__(16) float stage[];  // [64][SY_SS]
-  const int tid = threadIdx.x, tx = tid % SY_BNT, ty = tid / SY_BNT;
-  const int m0 = blockIdx.y * SY_TILE, n0 = blockIdx.x * SY_TILE;
+__global__ void __launch_bounds__(SF_NT)
+synth_kernel(const float* __restrict__ AYt, const float* __restrict__ Bt, int N, int ld, int nf,
+             Epi epi) {
+  extern __shared__ __align__(16) float sf[];
+  float* As = sf;                   // [nf][64]
+  float* Bs = sf + nf * SF_T;       // [nf][64]
+  const int tid = threadIdx.x, tx = tid % 16, ty = tid / 16;
+  const int m0 = blockIdx.y * SF_T, n0 = blockIdx.x * SF_T;
+  const int half = (nf + 1) / 2;
+  // rows f0 .. f1 - 1 of an operand, 64 floats from `first`: zeros past the row stride
+  auto copy = [&](float* dst, const float* src, int f0, int f1, int first) {
+    const int c = 4 * (tid % 16);
+    const bool ok = first + c < ld;
+    for (int f = f0 + tid / 16; f < f1; f += SF_NT / 16)
+      cp_async<16>(dst + f * SF_T + c, ok ? src + (size_t)f * ld + first + c : src, ok);
+  };
   pdl_trigger();
-  pdl_wait();
-  float acc[SY_TM][SY_TN];
-#pragma unroll
-  for (int i = 0; i < SY_TM; ++i)
-#pragma unroll
-    for (int j = 0; j < SY_TN; ++j) acc[i][j] = 0.f;
-  AYLoad ld{AY, N, kp};
-  gemm_mainloop<SY_BMT, SY_BNT, SY_TM, SY_TN, SY_BK>(ld, Bt, kp, N, m0, n0, 0, kp, As, Bs, acc);
-  for (int h = 0; h < 2; ++h) {
-    __syncthreads();
-    if (ty / 8 == h) {
-#pragma unroll
-      for (int i = 0; i < SY_TM; ++i)
-#pragma unroll
-        for (int j = 0; j < SY_TN; ++j)
-          stage[(ty * SY_TM + i - 64 * h) * SY_SS + tx + j * SY_BNT] = acc[i][j];
-    }
-    __syncthreads();
-    for (int e = tid; e < 64 * (SY_TILE / 4); e += SY_NT) {
-      const int r = e / (SY_TILE / 4), c4 = (e % (SY_TILE / 4)) * 4;
-      const int m = m0 + 64 * h + r, n = n0 + c4;
-      if (m >= N || n >= N) continue;
-      const float4 v = *reinterpret_cast<const float4*>(&stage[r * SY_SS + c4]);
-      epi.store4(m, n, v, min(4, N - n));
-    }
+  copy(As, AYt, 0, half, m0);
+  pdl_wait();   // the band operand comes from the previous kernel
+  copy(Bs, Bt, 0, half, n0);
+  cp_async_commit();
+  copy(As, AYt, half, nf, m0);
+  copy(Bs, Bt, half, nf, n0);
+  cp_async_commit();
+  // the epilogue's input lines into L2
+  if (const float* img = epi.input()) {
+    const int m = m0 + tid / 2, n = n0 + 32 * (tid % 2);
+    if (tid < 2 * SF_T && m < N && n < N)
+      asm volatile("prefetch.global.L2 [%0];" ::"l"(img + (size_t)m * N + n));
   }
-  epi.finish();
+  float acc[4][4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
+  auto multiply = [&](int f0, int f1) {
+#pragma unroll 4
+    for (int f = f0; f < f1; ++f) {
+      const float4 a = *reinterpret_cast<const float4*>(As + f * SF_T + 4 * ty);
+      const float4 b = *reinterpret_cast<const float4*>(Bs + f * SF_T + 4 * tx);
+      const float av[4] = {a.x, a.y, a.z, a.w}, bv[4] = {b.x, b.y, b.z, b.w};
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(av[i], bv[j], acc[i][j]);
+    }
+  };
+  cp_async_wait<1>();
+  __syncthreads();
+  multiply(0, half);
+  cp_async_wait<0>();
+  __syncthreads();
+  multiply(half, nf);
+  __syncthreads();
+  float* stage = sf;   // [64][SS], over the operands
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+    *reinterpret_cast<float4*>(stage + (4 * ty + i) * SF_SS + 4 * tx) =
+        make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+  __syncthreads();
+#pragma unroll 2
+  for (int e = tid; e < SF_T * (SF_T / 4); e += SF_NT) {
+    const int r = e / (SF_T / 4), c = 4 * (e % (SF_T / 4)), m = m0 + r, n = n0 + c;
+    if (m < N && n < N)
+      epi.store4(m, n, *reinterpret_cast<const float4*>(stage + r * SF_SS + c), min(4, N - n));
+  }
+  epi.template finish<SF_NT>();
 }
 
-static dim3 synth_grid(int N) {
-  const int t = (N + SY_TILE - 1) / SY_TILE;
-  return dim3(t, t, 1);
-}
+int synth_ld(int N) { return (N + 3) / 4 * 4; }
+int synth_blocks(int N) { return ((N + SF_T - 1) / SF_T) * ((N + SF_T - 1) / SF_T); }
 
 template <class Epi>
-static cudaError_t launch_synth(cudaStream_t s, const float* AY, const float* Bt, int N, int kp,
-                                const Epi& e) {
-  const int smem = 64 * SY_SS * sizeof(float);
+static cudaError_t launch_synth(cudaStream_t s, const float* AYt, const float* Bt, int N, int nf,
+                                const Epi& e, int* nblocks) {
+  const size_t smem = std::max((size_t)2 * nf * SF_T, (size_t)SF_T * SF_SS) * sizeof(float);
   cudaError_t err = cudaFuncSetAttribute(synth_kernel<Epi>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (err != cudaSuccess) return err;
-  return launch_pdl(synth_kernel<Epi>, synth_grid(N), dim3(SY_NT), smem, s, AY, Bt, N, kp, e);
+  const int t = (N + SF_T - 1) / SF_T;
+  *nblocks = t * t;
+  return launch_pdl(synth_kernel<Epi>, dim3(t, t, 1), dim3(SF_NT), smem, s, AYt, Bt, N, synth_ld(N),
+                    nf, e);
 }
 
-
-cudaError_t launch_synth_resist(cudaStream_t s, const float* AY, const float* Bt, int N, int kp,
+cudaError_t launch_synth_resist(cudaStream_t s, const float* AYt, const float* Bt, int N, int nf,
                                 const ResistEpilogue& ep, int* nblocks) {
-  const dim3 grid = synth_grid(N);
-  *nblocks = grid.x * grid.y;
   const int vec = N % 4 == 0 && aligned16(ep.aerial) && aligned16(ep.wafer) &&
                   aligned16(ep.target) && aligned16(ep.pe_window) && aligned16(ep.pen_window) &&
                   aligned16(ep.dldi);
-  return launch_synth(s, AY, Bt, N, kp, ResistEpi{ep, N, vec, 0.0, 0.0});
+  return launch_synth(s, AYt, Bt, N, nf, ResistEpi{ep, N, vec, 0.0, 0.0}, nblocks);
 }
 
-cudaError_t launch_synth_grad(cudaStream_t s, const float* AY, const float* Bt, int N, int kp,
+cudaError_t launch_synth_grad(cudaStream_t s, const float* AYt, const float* Bt, int N, int nf,
                               const GradEpilogue& ep, int* nblocks) {
-  const dim3 grid = synth_grid(N);
-  *nblocks = grid.x * grid.y;
   const int vec = N % 4 == 0 && aligned16(ep.grad_mask) && aligned16(ep.theta) &&
                   aligned16(ep.grad_theta);
-  return launch_synth(s, AY, Bt, N, kp, GradEpi{ep, N, vec, 0.0});
+  return launch_synth(s, AYt, Bt, N, nf, GradEpi{ep, N, vec, 0.0}, nblocks);
 }
 
 // ---------------------------------------------------------------- small-grid band stage
@@ -822,12 +875,12 @@ static size_t chat_smem(const BandGeom& g) {
   return (size_t)(g.Pc + g.Pr + g.Pc * nd) * sizeof(float2) + (size_t)g.Pr * g.Pc * sizeof(float);
 }
 
-// Band -> image columns: Ut[x][2a + {0,1}] = kappa(a) sum_c coef[a][c] phase(c, x) for
+// Band -> image columns: Ut[2a + {0,1}][x] = kappa(a) sum_c coef[a][c] phase(c, x) for
 // a 64-column x strip and 8 band rows per CTA (coefficients and phases staged).
 // mode 0 (band S): phase = conj(TX[c][x]) (TX = e^{-2 pi i s_c x/N}), kappa = 1.
 // mode 1 (difference set D, c in [0, 2nc-1), d = c - (nc-1)):
 //   phase = d >= 0 ? conj(TX[d][x]) : TX[-d][x], kappa(a) = a > 0 ? 2 : 1 (Hermitian half).
-// Columns 2*nrows .. kp-1 of Ut are zero.
+// Rows 2*nrows .. kp-1 of Ut are zero.
 // With img set (tensor-core path) the result goes
 // straight into the split-BF16 operand image of the row synthesis instead of Ut:
 // x tile x / 128 at img + (x / 128) * img_tile_bytes, hi of column f at
@@ -843,6 +896,8 @@ static size_t chat_smem(const BandGeom& g) {
 // its terms in j order as fma(D, u, fma(S, t, acc)) per component, in every kernel
 // below, so the batched and per-image expansions give bit-identical results.
 constexpr int EX_X = 64, EX_NT = 256;
+// Row stride of Ut ([kp][ut_ld], synth_ld).
+__host__ __device__ __forceinline__ size_t ut_ld(int N) { return (size_t)((N + 3) / 4 * 4); }
 
 // S_j and D_j of band row coef_row for phase row j, as (S.x, S.y, D.x, D.y).
 __device__ __forceinline__ float4 expand_sd(const float2* __restrict__ coef_row, int mode, int nc,
@@ -909,7 +964,11 @@ __device__ __forceinline__ void expand_store(const float4* sd, const float2* ph,
       *reinterpret_cast<uint2*>(tile + sw128_offset(128, x % 128, f0)) = hw;
       *reinterpret_cast<uint2*>(tile + sw128_offset(128, x % 128, kp + f0)) = lw;
     } else {
-      *reinterpret_cast<float4*>(Ut + (size_t)x * kp + f0) = v;
+      float* o = Ut + (size_t)f0 * ut_ld(N) + x;
+      o[0] = v.x;
+      o[ut_ld(N)] = v.y;
+      o[2 * ut_ld(N)] = v.z;
+      o[3 * ut_ld(N)] = v.w;
     }
   }
   // Columns past the last row group are zero.
@@ -920,7 +979,7 @@ __device__ __forceinline__ void expand_store(const float4* sd, const float2* ph,
         *reinterpret_cast<uint2*>(tile + sw128_offset(128, x % 128, f)) = make_uint2(0u, 0u);
         *reinterpret_cast<uint2*>(tile + sw128_offset(128, x % 128, kp + f)) = make_uint2(0u, 0u);
       } else {
-        *reinterpret_cast<float4*>(Ut + (size_t)x * kp + f) = make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int q = 0; q < 4; ++q) Ut[(size_t)(f + q) * ut_ld(N) + x] = 0.f;
       }
     }
   }
@@ -941,7 +1000,7 @@ expand_kernel(const float2* __restrict__ coef, int nrows, int ncoef, int ld,
     const size_t b = blockIdx.z;
     coef += b * nrows * ld;
     if (img) img += b * ((N + 127) / 128) * (size_t)img_tile_bytes;
-    else Ut += b * N * kp;
+    else Ut += b * ut_ld(N) * kp;
   }
   pdl_trigger();
   fill_batched<EX_NT>(ph, nph * EX_X, [&](int i) {
@@ -980,7 +1039,7 @@ expand_rows_kernel(const float2* __restrict__ coef, int nrows, int ncoef, int ld
     const size_t b = blockIdx.z;
     coef += b * nrows * ld;
     if (img) img += b * ((N + 127) / 128) * (size_t)img_tile_bytes;
-    else Ut += b * N * kp;
+    else Ut += b * ut_ld(N) * kp;
   }
   pdl_trigger();
   fill_batched<EXR_NT>(ph, nph * EXR_X, [&](int i) {
@@ -1048,7 +1107,11 @@ expand_rows_kernel(const float2* __restrict__ coef, int nrows, int ncoef, int ld
         *reinterpret_cast<uint2*>(tile + sw128_offset(128, x % 128, f0)) = hw;
         *reinterpret_cast<uint2*>(tile + sw128_offset(128, x % 128, kp + f0)) = lw;
       } else {
-        *reinterpret_cast<float4*>(Ut + (size_t)x * kp + f0) = v;
+        float* o = Ut + (size_t)f0 * ut_ld(N) + x;
+      o[0] = v.x;
+      o[ut_ld(N)] = v.y;
+      o[2 * ut_ld(N)] = v.z;
+      o[3 * ut_ld(N)] = v.w;
       }
     }
     // Columns past the last row group are zero.
@@ -1059,7 +1122,7 @@ expand_rows_kernel(const float2* __restrict__ coef, int nrows, int ncoef, int ld
           *reinterpret_cast<uint2*>(tile + sw128_offset(128, x % 128, f)) = make_uint2(0u, 0u);
           *reinterpret_cast<uint2*>(tile + sw128_offset(128, x % 128, kp + f)) = make_uint2(0u, 0u);
         } else {
-          *reinterpret_cast<float4*>(Ut + (size_t)x * kp + f) = make_float4(0.f, 0.f, 0.f, 0.f);
+          for (int q = 0; q < 4; ++q) Ut[(size_t)(f + q) * ut_ld(N) + x] = 0.f;
         }
       }
     }

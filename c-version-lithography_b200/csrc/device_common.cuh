@@ -66,7 +66,7 @@ __device__ __forceinline__ void st4(float* p, size_t i, float4 v, int vec, int n
   if (nvalid > 3) p[i + 3] = v.w;
 }
 
-constexpr int EPI_NT = 256;  // threads of every CTA that runs a synthesis epilogue
+constexpr int EPI_NT = 256;  // threads of a per-tile tensor-core CTA that runs a synthesis epilogue
 
 // sin / cos for the split-BF16 tensor-core path: Cody-Waite reduction of x by
 // 2 pi with a two-term constant (6.28125, exact in 9 bits so that k * 6.28125 is
@@ -128,7 +128,9 @@ struct ResistEpiT {
       }
       return;
     }
-    st4(p.dldi, i, dldi4(m, n, I, T, nvalid), vec, nvalid);
+    // four pixels without windows and penalty: the same values without their loads
+    st4(p.dldi, i, nvalid == 4 && plain() ? plain4(m, n, I, T) : dldi4(m, n, I, T, nvalid), vec,
+        nvalid);
   }
   // Mode 1 without the dL/dI store: aerial / wafer stores and loss terms as in
   // store4p, dL/dI returned (0 in lanes past nvalid).
@@ -169,12 +171,15 @@ struct ResistEpiT {
     return p.pe_window == nullptr && p.pen_window == nullptr && p.penalty == 0.f &&
            !p.loss_penalty_term;
   }
-  // All EPI_NT threads of the CTA must call finish.
+  // The per-pixel input of store4 (nullable).
+  __device__ __forceinline__ const float* input() const { return p.mode == 1 ? p.target : nullptr; }
+  // All NT threads of the CTA must call finish.
+  template <int NT = EPI_NT>
   __device__ __forceinline__ void finish() {
     if (p.mode != 1) return;
-    __shared__ double sh[EPI_NT / 32];
-    const double a = block_sum<EPI_NT>(pe, sh);
-    const double b = block_sum<EPI_NT>(pen, sh);
+    __shared__ double sh[NT / 32];
+    const double a = block_sum<NT>(pe, sh);
+    const double b = block_sum<NT>(pen, sh);
     if (threadIdx.x == 0) {
       const size_t bid = ((size_t)blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;
       p.loss_partial[2 * bid] = a;
@@ -222,10 +227,12 @@ struct GradEpiT {
     }
     st4(p.grad_theta, i, gt, vec, nvalid);
   }
+  __device__ __forceinline__ const float* input() const { return p.theta; }
+  template <int NT = EPI_NT>
   __device__ __forceinline__ void finish() {
     if (!p.theta) return;
-    __shared__ double sh[EPI_NT / 32];
-    const double a = block_sum<EPI_NT>(nrm, sh);
+    __shared__ double sh[NT / 32];
+    const double a = block_sum<NT>(nrm, sh);
     if (threadIdx.x == 0)   // [image][tile] over a batched launch
       p.norm_partial[((size_t)blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x] = a;
   }

@@ -54,8 +54,8 @@ struct Cache {
   float* TXD = nullptr;   // [2Nc][N]: same for d_c = 0..Nc-1
   float2* TYS = nullptr;  // [Nr][N]: e^{-2 pi i s_r y / N}
   float2* TYD = nullptr;  // [Nr][N]: e^{-2 pi i d_r y / N}, d_r = 0..Nr-1
-  float* AYS = nullptr;   // [N][kp_rows]: (Re, Im) of TYS[r][y] interleaved per y
-  float* AYD = nullptr;   // [N][kp_rows]: (Re, Im) of TYD[d][y] interleaved per y
+  float* AYS = nullptr;   // [kp_rows][synth_ld(N)]: rows 2r, 2r + 1 = Re, Im of TYS[r][y]
+  float* AYD = nullptr;   // [kp_rows][synth_ld(N)]: rows 2d, 2d + 1 = Re, Im of TYD[d][y]
   float2* TXSc = nullptr; // [Nc][N]: e^{-2 pi i s_c x / N} (complex rows)
   float2* TXDc = nullptr; // [Nc][N]: e^{-2 pi i d_c x / N}
   // Small-grid tables (Pr x Pc grid, P >= 2 * band - 1):
@@ -254,7 +254,7 @@ cudaError_t launch_band_adjoint(cudaStream_t s, const Cache& c, const Field& f, 
                                 double scale, float* gam, float2* Zk, float2* X, float* Vt,
                                 void* img, int batch = 1, int width = 0);
 
-// Row synthesis: out[y][x] = sum_f AY[y][f] * Bt[x][f] with a fused epilogue.
+// Row synthesis: out[y][x] = sum_f AY[y][f] * B[x][f] with a fused epilogue.
 struct ResistEpilogue {
   int mode;                 // 0: image only; 1: resist + loss + dL/dI
   float thr, alpha;
@@ -288,9 +288,13 @@ struct GradEpilogue {
   float* grad_theta;        // with theta
   double* norm_partial;     // with theta: per-block partial of sum grad_theta^2
 };
-cudaError_t launch_synth_resist(cudaStream_t s, const float* AY, const float* Bt, int N, int kp,
+// FP32 row syntheses: AYt and Bt have the inner index f (nf of them) as the slow one, rows of
+// synth_ld(N) floats; one loss / norm partial per 64 x 64 tile (synth_blocks(N)).
+int synth_ld(int N);
+int synth_blocks(int N);
+cudaError_t launch_synth_resist(cudaStream_t s, const float* AYt, const float* Bt, int N, int nf,
                                 const ResistEpilogue& ep, int* nblocks);
-cudaError_t launch_synth_grad(cudaStream_t s, const float* AY, const float* Bt, int N, int kp,
+cudaError_t launch_synth_grad(cudaStream_t s, const float* AYt, const float* Bt, int N, int nf,
                               const GradEpilogue& ep, int* nblocks);
 cudaError_t launch_sum_partials(cudaStream_t s, const double* part, int n, int stride,
                                 double* out);
@@ -322,7 +326,7 @@ cudaError_t launch_analysis_tc2(cudaStream_t s, int mode, const float* in, float
                                 int* flag, int N, int ncols, int nrows_out, int nr, int sym,
                                 float2* part, const void* tx_img, const void* ty_img, int* err,
                                 int batch = 1);
-// Row synthesis: Aimg = image of AY ([N][kp], launch_pack_tc2_rows), Bimg = image
+// Row synthesis: Aimg = image of AY (AYS or AYD, launch_pack_tc2_rows), Bimg = image
 // of the band operand Bt ([N][kp]); kp % 16 == 0 and kp <= 128.
 size_t tc2_rows_image_bytes(int N, int kp);
 cudaError_t launch_pack_tc2_rows(cudaStream_t s, const float* src, int N, int kp, void* dst);

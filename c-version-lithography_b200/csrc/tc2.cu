@@ -33,7 +33,8 @@ __device__ __forceinline__ size_t img_row(int N, int m) {
 // ---------------------------------------------------------------- image packing
 // Logical real matrix of a pack source: kind 0 reads src[row * ld + col];
 // kind 1 reads the complex src2[(row / 2) * ld + col] and gives its real part
-// for even rows, its imaginary part for odd rows. Outside rows x cols it is 0.
+// for even rows, its imaginary part for odd rows; kind 2 reads src[col * ld + row].
+// Outside rows x cols it is 0.
 struct Split2Src {
   const float* src;
   int kind;
@@ -43,6 +44,7 @@ struct Split2Src {
 __device__ __forceinline__ float s2_value(const Split2Src& s, int row, int col) {
   if (row >= s.rows || col >= s.cols) return 0.f;
   if (s.kind == 0) return s.src[(size_t)row * s.ld + col];
+  if (s.kind == 2) return s.src[(size_t)col * s.ld + row];
   const float2 z = reinterpret_cast<const float2*>(s.src)[(size_t)(row >> 1) * s.ld + col];
   return (row & 1) ? z.y : z.x;
 }
@@ -509,7 +511,7 @@ static cudaError_t launch_tc2(cudaStream_t s, const void* Aimg, const void* Bimg
 size_t tc2_rows_image_bytes(int N, int kp) { return split2_image_bytes((N + 127) / 128, 128, 1, kp); }
 
 cudaError_t launch_pack_tc2_rows(cudaStream_t s, const float* src, int N, int kp, void* dst) {
-  return launch_pack_split2(s, src, 0, N, kp, kp, 128, kp, (N + 127) / 128, 1, dst);
+  return launch_pack_split2(s, src, 2, N, kp, synth_ld(N), 128, kp, (N + 127) / 128, 1, dst);
 }
 
 cudaError_t launch_synth_resist_tc2(cudaStream_t s, const void* Aimg, const void* Bimg, int N,
