@@ -1035,8 +1035,9 @@ fused_tc3_kernel(const uint8_t* __restrict__ Aimg, const uint8_t* __restrict__ B
         // (each lane rounded as the scalar operation, in the scalar order, so dL/dI is
         // the per-tile kernels' bit for bit; __expf and the reciprocal stay per lane).
         // Every dL/dI is non-finite exactly when its r is, and then so is the product
-        // with 0 in chk. The loss terms are summed in two interleaved FP32 chains. Past
-        // the image edge r is taken as 0, and with it dL/dI and the loss term.
+        // with 0 in chk. The loss terms are summed in two interleaved FP32 chains, at the
+        // image edge in one of rounded squares (the FP64 losses of ragged images depend on
+        // it in the ninth digit); past it r is 0, and with it dL/dI and the loss term.
         float2 chk = make_float2(0.f, 0.f), se = chk;
         const float2 na = make_float2(-r.p.alpha, -r.p.alpha);
         const float2 nt = make_float2(-r.p.thr, -r.p.thr);
@@ -1053,7 +1054,10 @@ fused_tc3_kernel(const uint8_t* __restrict__ Aimg, const uint8_t* __restrict__ B
               if (e >= ny) rr.x = W.x = 0.f;
               if (e + 1 >= ny) rr.y = W.y = 0.f;
             }
-            se = __ffma2_rn(rr, rr, se);
+            if (decltype(edge)::value)
+              se.x = __fadd_rn(__fadd_rn(se.x, __fmul_rn(rr.x, rr.x)), __fmul_rn(rr.y, rr.y));
+            else
+              se = __ffma2_rn(rr, rr, se);
             const float2 g = __fmul2_rn(__fmul2_rn(__fmul2_rn(pw, rr), W),
                                         __fadd2_rn(one, make_float2(-W.x, -W.y)));
             chk = __ffma2_rn(g, make_float2(0.f, 0.f), chk);
@@ -1099,20 +1103,19 @@ fused_tc3_kernel(const uint8_t* __restrict__ Aimg, const uint8_t* __restrict__ B
             const float I = d[e0 + e], T = pre[e0 + e];
             const float W = r.sigmoid(I);
             const float rr = W - T;
-            float sum = r.p.pe_weight * rr * pw[e], pe = rr * rr * pw[e], pen = 0.f;
+            const bool in = e0 + e < ny;   // the accumulator past the edge may hold anything
+            float sum = r.p.pe_weight * rr * pw[e];
+            if (in) s0 += rr * rr * pw[e];
             if (pen_on && T < 0.5f) {
               const float ex = fmaxf(W - r.p.pen_thr, 0.f);
-              pen = ex * ex * qw[e];
+              if (in) s1 += ex * ex * qw[e];
               sum += r.p.penalty * ex * qw[e];
             }
-            float g = sum * W * (1.f - W);
-            if (e0 + e >= ny) pe = pen = g = 0.f;   // the accumulator there may hold anything
-            if (OUT && e0 + e < ny) {
+            const float g = in ? sum * W * (1.f - W) : 0.f;
+            if (OUT && in) {
               if (r.p.aerial) r.p.aerial[i0 + (size_t)(e0 + e) * N] = I;
               if (r.p.wafer) r.p.wafer[i0 + (size_t)(e0 + e) * N] = W;
             }
-            s0 += pe;
-            s1 += pen;
             chk = __fmaf_rn(g, 0.f, chk);
             d[e0 + e] = g;
           }
