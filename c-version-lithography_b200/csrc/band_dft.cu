@@ -568,28 +568,48 @@ band_fields_kernel(const float2* __restrict__ H, const float2* __restrict__ mban
 }
 
 // C = A B over operands in shared memory: each thread owns an RT x 2 block of C (rows
-// m0 .. m0 + RT - 1, columns 2p and 2p + 1) and adds the terms in k order with cfma,
-// the operand order and summation order of the chunked kernels, so every element is
+// m0 .. m0 + RT - 1, columns 2p and 2p + 1) and adds the terms in k order with cfma, the
+// operand order and summation order of the chunked kernels, so every element is
 // bit-identical to theirs. Work items run pair-fastest: a warp's B loads are adjacent
-// 16-byte words and its A loads mostly one broadcast address. a(m, k) returns A[m][k];
-// B[k][n] is at B + k ldb + n (ldb even, B 16-byte aligned).
-template <int RT, int NT, class ALoad, class Store>
-__device__ __forceinline__ void cgemm_rt2(int M, int npairs, int Kd, ALoad a,
+// 16-byte words and its A loads one or two broadcast addresses. Column 2p takes A0, column
+// 2p + 1 takes A1 (the same operand, or the two classes of a folded transform). The operands
+// are read two k at a time, 16 bytes each: the shared-memory wavefronts, about as many as
+// the FMAs with 8-byte A loads, are what bounds these products. A[m][k] is at A + m lda + k,
+// B[k][n] at B + k ldb + n; lda and ldb even, all bases 16-byte aligned.
+template <int RT, int NT, class Store>
+__device__ __forceinline__ void cgemm_rt2(int M, int npairs, int Kd, const float2* __restrict__ A0,
+                                          const float2* __restrict__ A1, int lda,
                                           const float2* __restrict__ B, int ldb, Store store) {
   const int rblocks = (M + RT - 1) / RT;
   for (int it = threadIdx.x; it < rblocks * npairs; it += NT) {
     const int m0 = (it / npairs) * RT, p = it % npairs;
+    const float2* bp = B + 2 * p;
+    int ro[RT];
+#pragma unroll
+    for (int i = 0; i < RT; ++i) ro[i] = min(m0 + i, M - 1) * lda;
     float2 acc[RT][2];
 #pragma unroll
     for (int i = 0; i < RT; ++i) acc[i][0] = acc[i][1] = make_float2(0.f, 0.f);
-    for (int k = 0; k < Kd; ++k) {
-      const float4 b = *reinterpret_cast<const float4*>(B + (size_t)k * ldb + 2 * p);
-      const float2 b0 = make_float2(b.x, b.y), b1 = make_float2(b.z, b.w);
+    int k = 0;
+    for (; k + 1 < Kd; k += 2) {
+      const float4 b = *reinterpret_cast<const float4*>(bp + k * ldb);
+      const float4 c = *reinterpret_cast<const float4*>(bp + (k + 1) * ldb);
 #pragma unroll
       for (int i = 0; i < RT; ++i) {
-        const float2 av = a(min(m0 + i, M - 1), k);
-        cfma(acc[i][0], av, b0);
-        cfma(acc[i][1], av, b1);
+        const float4 a = *reinterpret_cast<const float4*>(A0 + ro[i] + k);
+        cfma(acc[i][0], make_float2(a.x, a.y), make_float2(b.x, b.y));
+        cfma(acc[i][0], make_float2(a.z, a.w), make_float2(c.x, c.y));
+        const float4 d = A1 == A0 ? a : *reinterpret_cast<const float4*>(A1 + ro[i] + k);
+        cfma(acc[i][1], make_float2(d.x, d.y), make_float2(b.z, b.w));
+        cfma(acc[i][1], make_float2(d.z, d.w), make_float2(c.z, c.w));
+      }
+    }
+    if (k < Kd) {
+      const float4 b = *reinterpret_cast<const float4*>(bp + k * ldb);
+#pragma unroll
+      for (int i = 0; i < RT; ++i) {
+        cfma(acc[i][0], A0[ro[i] + k], make_float2(b.x, b.y));
+        cfma(acc[i][1], A1[ro[i] + k], make_float2(b.z, b.w));
       }
     }
 #pragma unroll
@@ -605,38 +625,39 @@ __device__ __forceinline__ void cgemm_rt2(int M, int npairs, int Kd, ALoad a,
 // C = A B folded over the output rows (the transform over P = 2 M outputs): output rows
 // m and m + M of each column pair from Ev = sum over k of the parity class k0, k0 + 2,
 // ... and Od = sum over the other class, each in increasing k with cfma, stored as
-// Ev + Od (row m) and Ev - Od (row m + M). Each thread owns RT rows x 2 columns.
-template <int RT, int NT, class ALoad, class Store>
-__device__ __forceinline__ void fold_rows(int M, int npairs, int Kd, int k0, ALoad a,
-                                          const float2* __restrict__ B, int ldb, Store store) {
-  const int rblocks = (M + RT - 1) / RT;
+// Ev + Od (row m) and Ev - Od (row m + M). Each thread owns four rows x 2 columns. A[m][k] is
+// at A + k lda + m (lda even): its four rows are two 16-byte words.
+template <int NT, class Store>
+__device__ __forceinline__ void fold_rows4(int M, int npairs, int Kd, int k0, const float2* __restrict__ A,
+                                           int lda, const float2* __restrict__ B, int ldb, Store store) {
+  const int rblocks = (M + 3) / 4;
   for (int it = threadIdx.x; it < rblocks * npairs; it += NT) {
-    const int m0 = (it / npairs) * RT, p = it % npairs;
-    float2 ev[RT][2], od[RT][2];
+    const int m0 = (it / npairs) * 4, p = it % npairs;
+    float2 ev[4][2], od[4][2];
 #pragma unroll
-    for (int i = 0; i < RT; ++i) ev[i][0] = ev[i][1] = od[i][0] = od[i][1] = make_float2(0.f, 0.f);
-    for (int k = k0; k < Kd; k += 2) {
-      const float4 b = *reinterpret_cast<const float4*>(B + (size_t)k * ldb + 2 * p);
-      const float2 b0 = make_float2(b.x, b.y), b1 = make_float2(b.z, b.w);
+    for (int i = 0; i < 4; ++i) ev[i][0] = ev[i][1] = od[i][0] = od[i][1] = make_float2(0.f, 0.f);
+    auto term = [&](float2 (&acc)[4][2], int k) {
+      const float4 b = *reinterpret_cast<const float4*>(B + k * ldb + 2 * p);
+      const float4 a01 = *reinterpret_cast<const float4*>(A + k * lda + m0);
+      const float4 a23 = *reinterpret_cast<const float4*>(A + k * lda + m0 + 2);
+      const float2 av[4] = {make_float2(a01.x, a01.y), make_float2(a01.z, a01.w),
+                            make_float2(a23.x, a23.y), make_float2(a23.z, a23.w)};
 #pragma unroll
-      for (int i = 0; i < RT; ++i) {
-        const float2 av = a(min(m0 + i, M - 1), k);
-        cfma(ev[i][0], av, b0);
-        cfma(ev[i][1], av, b1);
+      for (int i = 0; i < 4; ++i) {
+        cfma(acc[i][0], av[i], make_float2(b.x, b.y));
+        cfma(acc[i][1], av[i], make_float2(b.z, b.w));
       }
+    };
+    // k0 = 1: the first term belongs to the odd class
+    int k = 0;
+    if (k0) term(od, k++);
+    for (; k + 1 < Kd; k += 2) {
+      term(ev, k);
+      term(od, k + 1);
     }
-    for (int k = 1 - k0; k < Kd; k += 2) {
-      const float4 b = *reinterpret_cast<const float4*>(B + (size_t)k * ldb + 2 * p);
-      const float2 b0 = make_float2(b.x, b.y), b1 = make_float2(b.z, b.w);
+    if (k < Kd) term(ev, k);
 #pragma unroll
-      for (int i = 0; i < RT; ++i) {
-        const float2 av = a(min(m0 + i, M - 1), k);
-        cfma(od[i][0], av, b0);
-        cfma(od[i][1], av, b1);
-      }
-    }
-#pragma unroll
-    for (int i = 0; i < RT; ++i) {
+    for (int i = 0; i < 4; ++i) {
       if (m0 + i < M) {
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
@@ -651,17 +672,17 @@ __device__ __forceinline__ void fold_rows(int M, int npairs, int Kd, int k0, ALo
 // Forward 1, whole small grid per CTA: grid (K, 1, batch), CTA (k, b) computes all of
 // e_k = ESr (A ESc^T) (Pr x Pc) and ik = w_k |e_k|^2 for image b, every table staged
 // once per CTA instead of once per column chunk. Same arithmetic as
-// band_fields_kernel (bit-identical results), register-blocked: 5 rows x 2 columns of
-// T and, folded over the row parity classes, 5 row pairs (jr, jr + Nr) x 2 columns of
+// band_fields_kernel (bit-identical results), register-blocked: 4 rows x 2 columns of
+// T and, folded over the row parity classes, 4 row pairs (jr, jr + Nr) x 2 columns of
 // e_k per thread.
-constexpr int BG_NT = 256;
+constexpr int BG_NT = 320;
 __global__ void __launch_bounds__(BG_NT)
 band_fields_whole_kernel(const float2* __restrict__ H, const float2* __restrict__ mband,
                          const float* __restrict__ w, int Nr, int Nc, int Pr, int Pc, int row0,
                          const float2* __restrict__ ESc_t, const float2* __restrict__ ESr_t,
                          float2* __restrict__ e, float* __restrict__ ik) {
   extern __shared__ __align__(16) float2 sm2[];
-  const int k = blockIdx.x;
+  const int k = blockIdx.x, NcE = even_up(Nc);
   {  // image b of a batch
     const size_t b = blockIdx.z;
     mband += b * Nr * Nc;
@@ -669,31 +690,33 @@ band_fields_whole_kernel(const float2* __restrict__ H, const float2* __restrict_
     ik += b * gridDim.x * Pr * Pc;
   }
   float2* esc = sm2;                    // [Nc][Pc]
-  float2* esr = esc + Nc * Pc;          // [Nr][Pr]
-  float2* T = esr + Nr * Pr;            // [Nr][Pc]
-  float2* A = T + Nr * Pc;              // [Nr][Nc]
+  float2* esr = esc + Nc * Pc;          // [Nr][Pr] (+ 2: the last rows' 16-byte reads)
+  float2* T = esr + Nr * Pr + 2;        // [Nr][Pc]
+  float2* A = T + Nr * Pc;              // [Nr][NcE]
   pdl_trigger();
   fill_batched<BG_NT>(esc, Nc * Pc, [&](int i) { return ESc_t[i]; });
   fill_batched<BG_NT>(esr, Nr * Pr, [&](int i) { return ESr_t[i]; });
   pdl_wait();
-  fill_batched<BG_NT>(A, Nr * Nc, [&](int i) { return cmul(H[(size_t)k * Nr * Nc + i], mband[i]); });
+  fill_batched<BG_NT>(A, Nr * NcE, [&](int i) {
+    const int r = i / NcE, c = i - r * NcE, o = r * Nc + min(c, Nc - 1);
+    return cmul(H[(size_t)k * Nr * Nc + o], mband[o]);
+  });
   __syncthreads();
-  cgemm_rt2<5, BG_NT>(Nr, Pc / 2, Nc, [&](int r, int c) { return A[r * Nc + c]; }, esc, Pc,
+  cgemm_rt2<4, BG_NT>(Nr, Pc / 2, Nc, A, A, NcE, esc, Pc,
                       [&](int r, int j, float2 v) { T[r * Pc + j] = v; });
   __syncthreads();
   const float wk = w[k];
   float2* ek = e + (size_t)k * Pr * Pc;
   float* ikk = ik + (size_t)k * Pr * Pc;
-  fold_rows<5, BG_NT>(Nr, Pc / 2, Nr, row0 & 1, [&](int jr, int r) { return esr[r * Pr + jr]; }, T,
-                      Pc, [&](int jr, int j, float2 v) {
-                        const size_t o = (size_t)jr * Pc + j;
-                        ek[o] = v;
-                        ikk[o] = wk * (v.x * v.x + v.y * v.y);
-                      });
+  fold_rows4<BG_NT>(Nr, Pc / 2, Nr, row0 & 1, esr, Pr, T, Pc, [&](int jr, int j, float2 v) {
+    const size_t o = (size_t)jr * Pc + j;
+    ek[o] = v;
+    ikk[o] = wk * (v.x * v.x + v.y * v.y);
+  });
 }
 
 static size_t fields_whole_smem(const BandGeom& g) {
-  return (size_t)(g.Nc * g.Pc + g.Nr * g.Pr + g.Nr * g.Pc + g.Nr * g.Nc) * sizeof(float2);
+  return (size_t)(g.Nc * g.Pc + g.Nr * g.Pr + 2 + g.Nr * g.Pc + g.Nr * even_up(g.Nc)) * sizeof(float2);
 }
 
 template <int W>
@@ -786,18 +809,25 @@ __device__ __forceinline__ float2 sum4(const float2 (&a)[4]) {
   return make_float2((a[0].x + a[1].x) + (a[2].x + a[3].x), (a[0].y + a[1].y) + (a[2].y + a[3].y));
 }
 
-// Forward 3 with BC_DR band rows per CTA: grid (ceil(Nr / BC_DR), batch). The tables and
+// Forward 3 with up to BC_DR band rows (per) per CTA: grid (ceil(Nr / per), batch). The tables and
 // the image's small-grid intensity are staged once per BC_DR rows instead of once per
 // row; one thread per pair of outputs keeps the four interleaved partial sums of
 // band_chat_kernel and adds them in its order, so the results are bit-identical.
 constexpr int BC_DR = 5;
+// Rows per CTA of the row-grouped small-grid kernels: few enough for BAND_CTAS CTAs, two per
+// SM. Staging is shared by the rows of a CTA, but a grid below that leaves SMs idle.
+constexpr int BAND_CTAS = 296;
+static int rows_per_cta(int rows, int batch, int most) {
+  const long long per = ((long long)rows * batch + BAND_CTAS - 1) / BAND_CTAS;
+  return (int)std::max<long long>(1, std::min<long long>(per, most));
+}
 __global__ void __launch_bounds__(256)
 band_chat_rows_kernel(const float* __restrict__ iP, int Nr, int Nc, int Pr, int Pc,
                       const float2* __restrict__ EDr_t, const float2* __restrict__ EDc, float inv,
-                      float2* __restrict__ chat) {
+                      int per, float2* __restrict__ chat) {
   extern __shared__ __align__(16) float2 sb[];
   const int nd = 2 * Nc - 1, ndE = even_up(nd);
-  const int dr0 = blockIdx.x * BC_DR, nr = min(BC_DR, Nr - dr0);
+  const int dr0 = blockIdx.x * per, nr = min(per, Nr - dr0);
   iP += (size_t)blockIdx.y * Pr * Pc;   // image b of a batch
   chat += (size_t)blockIdx.y * Nr * nd;
   float2* edc = sb;                                    // [Pc][ndE] (column nd zero)
@@ -1219,9 +1249,10 @@ cudaError_t launch_band_forward(cudaStream_t s, const Cache& c, Field& f, float*
     err = cudaFuncSetAttribute(band_chat_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                (int)smc);
     if (err != cudaSuccess) return err;
-    err = launch_pdl(band_chat_rows_kernel, dim3((g.Nr + BC_DR - 1) / BC_DR, batch), dim3(256),
+    const int per = rows_per_cta(g.Nr, batch, BC_DR);
+    err = launch_pdl(band_chat_rows_kernel, dim3((g.Nr + per - 1) / per, batch), dim3(256),
                      smc, s, static_cast<const float*>(iP), g.Nr, g.Nc, g.Pr, g.Pc, c.EDr_t, c.EDc,
-                     1.f / ((float)g.Pr * (float)g.Pc), chat);
+                     1.f / ((float)g.Pr * (float)g.Pc), per, chat);
   } else {
     const size_t smc = chat_smem(g);
     err = cudaFuncSetAttribute(band_chat_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1283,18 +1314,18 @@ band_gamma_kernel(const float2* __restrict__ gh, int Nr, int Nc, int Pr, int Pc,
   }
 }
 
-// Adjoint 1 with BG_JR small-grid rows per CTA: grid (ceil(Pr / BG_JR), batch). The
+// Adjoint 1 with up to BG_JR small-grid rows (per) per CTA: grid (ceil(Pr / per), batch). The
 // tables and the image's g' are staged once per BG_JR rows; one thread per output (wv)
 // or pair of outputs (gamma) keeps the four interleaved partial sums of
 // band_gamma_kernel and adds them in its order, so the results are bit-identical.
 constexpr int BG_JR = 10;
 __global__ void __launch_bounds__(256)
 band_gamma_rows_kernel(const float2* __restrict__ gh, int Nr, int Nc, int Pr, int Pc,
-                       const float2* __restrict__ EDr_t, const float2* __restrict__ EDc_t,
+                       const float2* __restrict__ EDr_t, const float2* __restrict__ EDc_t, int per,
                        float* __restrict__ gam) {
   extern __shared__ __align__(16) float2 sg[];
   const int na = 2 * Nr - 1;
-  const int jr0 = blockIdx.x * BG_JR, nj = min(BG_JR, Pr - jr0);
+  const int jr0 = blockIdx.x * per, nj = min(per, Pr - jr0);
   gh += (size_t)blockIdx.y * na * Nc;   // image b of a batch
   gam += (size_t)blockIdx.y * Pr * Pc;
   float2* edc = sg;                  // [Nc][Pc] rows Nc-1 .. 2Nc-2 of EDc_t
@@ -1405,38 +1436,6 @@ __device__ __forceinline__ void z_fold_inplace(float2* q, int Pr, int Nc, int Pc
   }
 }
 
-// C = A B with a separate A operand per column of each pair (the transform over P = 2 n
-// inputs, folded: column 2p reads a0, column 2p + 1 reads a1), K = Kd in increasing
-// order with cfma; each thread owns RT rows x 2 columns.
-template <int RT, int NT, class ALoad0, class ALoad1, class Store>
-__device__ __forceinline__ void fold_cols_in(int M, int npairs, int Kd, ALoad0 a0, ALoad1 a1,
-                                             const float2* __restrict__ B, int ldb, Store store) {
-  const int rblocks = (M + RT - 1) / RT;
-  for (int it = threadIdx.x; it < rblocks * npairs; it += NT) {
-    const int m0 = (it / npairs) * RT, p = it % npairs;
-    float2 acc[RT][2];
-#pragma unroll
-    for (int i = 0; i < RT; ++i) acc[i][0] = acc[i][1] = make_float2(0.f, 0.f);
-    for (int k = 0; k < Kd; ++k) {
-      const float4 b = *reinterpret_cast<const float4*>(B + (size_t)k * ldb + 2 * p);
-      const float2 b0 = make_float2(b.x, b.y), b1 = make_float2(b.z, b.w);
-#pragma unroll
-      for (int i = 0; i < RT; ++i) {
-        const int m = min(m0 + i, M - 1);
-        cfma(acc[i][0], a0(m, k), b0);
-        cfma(acc[i][1], a1(m, k), b1);
-      }
-    }
-#pragma unroll
-    for (int i = 0; i < RT; ++i) {
-      if (m0 + i < M) {
-        store(m0 + i, 2 * p, acc[i][0]);
-        store(m0 + i, 2 * p + 1, acc[i][1]);
-      }
-    }
-  }
-}
-
 // Adjoint 2: grid (K, band column chunks of W, batch). CTA (k, q) owns band columns
 // uc in [q W, q W + W): q_k = e_k gamma (Pr x Pc, staged), Z1 = q_k conj(ESc)
 // restricted to those columns (Pr x W), Zk = conj(ESr_t) Z1 / (Pr Pc) (Nr x W); four
@@ -1526,7 +1525,8 @@ band_z_kernel(const float2* __restrict__ e, const float* __restrict__ gam, int N
 // Zk for image b, every table staged once. Same arithmetic as band_z_kernel
 // (bit-identical results); the band columns are padded to an even count with zero
 // table columns, whose outputs are not stored.
-__global__ void __launch_bounds__(BG_NT)
+constexpr int BZ_NT = 256;
+__global__ void __launch_bounds__(BZ_NT)
 band_z_whole_kernel(const float2* __restrict__ e, const float* __restrict__ gam, int Nr, int Nc,
                     int Pr, int Pc, int col0, const float2* __restrict__ ESc,
                     const float2* __restrict__ ESr_t, float inv, float2* __restrict__ Zk) {
@@ -1539,38 +1539,62 @@ band_z_whole_kernel(const float2* __restrict__ e, const float* __restrict__ gam,
     gam += b * Pr * Pc;
     Zk += b * gridDim.x * Nr * Nc;
   }
-  float2* esc = sz;                   // [Pc][NcE]
-  float2* esr = esc + Pc * NcE;       // [Nr][Pr]
-  float2* q = esr + Nr * Pr;          // [Pr][Pc]
-  float2* Z1 = q + Pr * Pc;           // [Pr][NcE]
+  // The second transform's table takes the place of the folded input, which is dead by
+  // then: three CTAs per SM instead of two (384 CTAs for 16 images and 24 kernels fit at once).
+  float2* esc = sz;                   // [Nc][NcE]
+  float2* Z1 = esc + Nc * NcE;        // [Pr][NcE]
+  float2* q = Z1 + Pr * NcE;          // [Pr][2][NcE]: folded sums, differences
+  float2* esr = q;                    // [Nr][Pr]
   const float2* ek = e + (size_t)k * Pr * Pc;
   pdl_trigger();
-  fill_batched<BG_NT>(esc, Nc * NcE, [&](int i) {
+  fill_batched<BZ_NT>(esc, Nc * NcE, [&](int i) {
     const int jc = i / NcE, u = i % NcE;
     return u < Nc ? conjf2(ESc[(size_t)jc * Nc + u]) : make_float2(0.f, 0.f);
   });
-  fill_batched<BG_NT>(esr, Nr * Pr, [&](int i) { return ESr_t[i]; });
   pdl_wait();
-  fill_batched<BG_NT>(q, Pr * Pc, [&](int i) { return z_product(ek, gam, i); });
-  __syncthreads();
-  z_fold_inplace<BG_NT>(q, Pr, Nc, Pc);
+  // q = e_k gamma (products rounded on their own) folded as it is read: column jc of row jr
+  // holds q(jr, jc) + q(jr, jc + Nc), and NcE further on the difference.
+  for (int base = threadIdx.x; base < Pr * Nc; base += BZ_NT * 4) {
+    float2 t0[4], t1[4];
+    float g0[4], g1[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int i = base + u * BZ_NT;
+      if (i < Pr * Nc) {
+        const int o = i / Nc * Pc + i % Nc;
+        t0[u] = ek[o]; t1[u] = ek[o + Nc];
+        g0[u] = gam[o]; g1[u] = gam[o + Nc];
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int i = base + u * BZ_NT;
+      if (i < Pr * Nc) {
+        const float2 a = make_float2(__fmul_rn(t0[u].x, g0[u]), __fmul_rn(t0[u].y, g0[u]));
+        const float2 b = make_float2(__fmul_rn(t1[u].x, g1[u]), __fmul_rn(t1[u].y, g1[u]));
+        float2* row = q + i / Nc * 2 * NcE + i % Nc;
+        row[0] = fold_sum(a, b);
+        row[NcE] = fold_diff(a, b);
+      }
+    }
+  }
   __syncthreads();
   // Column 2p has the parity of col0: sums for an even class, differences for an odd one.
-  const int off0 = (col0 & 1) ? Nc : 0, off1 = Nc - off0;
-  fold_cols_in<5, BG_NT>(Pr, NcE / 2, Nc, [&](int jr, int jc) { return q[jr * Pc + off0 + jc]; },
-                         [&](int jr, int jc) { return q[jr * Pc + off1 + jc]; }, esc, NcE,
-                         [&](int jr, int u, float2 v) { Z1[jr * NcE + u] = v; });
+  const int off0 = (col0 & 1) ? NcE : 0;
+  cgemm_rt2<5, BZ_NT>(Pr, NcE / 2, Nc, q + off0, q + NcE - off0, 2 * NcE, esc, NcE,
+                      [&](int jr, int u, float2 v) { Z1[jr * NcE + u] = v; });
+  __syncthreads();
+  fill_batched<BZ_NT>(esr, Nr * Pr, [&](int i) { return conjf2(ESr_t[i]); });
   __syncthreads();
   float2* zk = Zk + (size_t)k * Nr * Nc;
-  cgemm_rt2<3, BG_NT>(Nr, NcE / 2, Pr, [&](int ur, int jr) { return conjf2(esr[ur * Pr + jr]); },
-                      Z1, NcE, [&](int ur, int u, float2 v) {
-                        if (u < Nc) zk[(size_t)ur * Nc + u] = make_float2(v.x * inv, v.y * inv);
-                      });
+  cgemm_rt2<3, BZ_NT>(Nr, NcE / 2, Pr, esr, esr, Pr, Z1, NcE, [&](int ur, int u, float2 v) {
+    if (u < Nc) zk[(size_t)ur * Nc + u] = make_float2(v.x * inv, v.y * inv);
+  });
 }
 
 static size_t z_whole_smem(const BandGeom& g) {
   const int NcE = even_up(g.Nc);
-  return (size_t)(g.Pc * NcE + g.Nr * g.Pr + g.Pr * g.Pc + g.Pr * NcE) * sizeof(float2);
+  return (size_t)(g.Nc * NcE + g.Pr * NcE + std::max(g.Pr * 2 * NcE, g.Nr * g.Pr)) * sizeof(float2);
 }
 
 // Adjoint 3: X[u] = scale sum_k w_k conj(H_k(u)) Z_k(u). Four lanes per u: lane j
@@ -1629,8 +1653,9 @@ cudaError_t launch_band_adjoint(cudaStream_t s, const Cache& c, const Field& f, 
     e0 = cudaFuncSetAttribute(band_gamma_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                               (int)smg);
     if (e0 != cudaSuccess) return e0;
-    e0 = launch_pdl(band_gamma_rows_kernel, dim3((g.Pr + BG_JR - 1) / BG_JR, batch), dim3(256),
-                    smg, s, gh, g.Nr, g.Nc, g.Pr, g.Pc, c.EDr_t, c.EDc_t, gam);
+    const int per = rows_per_cta(g.Pr, batch, BG_JR);
+    e0 = launch_pdl(band_gamma_rows_kernel, dim3((g.Pr + per - 1) / per, batch), dim3(256),
+                    smg, s, gh, g.Nr, g.Nc, g.Pr, g.Pc, c.EDr_t, c.EDc_t, per, gam);
   } else {
     const size_t smg = gamma_smem(g);
     e0 = cudaFuncSetAttribute(band_gamma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1660,7 +1685,7 @@ cudaError_t launch_band_adjoint(cudaStream_t s, const Cache& c, const Field& f, 
     err = cudaFuncSetAttribute(band_z_whole_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                (int)smw);
     if (err == cudaSuccess)
-      err = launch_pdl(band_z_whole_kernel, dim3(g.K, 1, batch), dim3(BG_NT), smw, s,
+      err = launch_pdl(band_z_whole_kernel, dim3(g.K, 1, batch), dim3(BZ_NT), smw, s,
                        static_cast<const float2*>(f.e), static_cast<const float*>(gam), g.Nr,
                        g.Nc, g.Pr, g.Pc, g.col0, c.ESc, c.ESr_t, 1.f / ((float)g.Pr * (float)g.Pc),
                        Zk);
