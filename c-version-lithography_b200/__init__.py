@@ -217,6 +217,9 @@ def _f32(t, torch, shape=None, name="array"):
     """Contiguous float32 CUDA tensor view of t (copies host data to the device)."""
     if t is None:
         return None
+    if (isinstance(t, torch.Tensor) and t.dtype is torch.float32 and t.is_cuda
+            and t.is_contiguous() and (shape is None or t.shape == shape)):
+        return t
     if not isinstance(t, torch.Tensor):
         t = torch.as_tensor(np.asarray(t))
     if t.device.type != "cuda":

@@ -108,6 +108,7 @@ constexpr int RED_FLAG = 0;
 constexpr int RED_COUNT = 1;  // CTA counter of the single-image dt
 constexpr int RED_SUM = 2;    // summed results (up to 4 doubles)
 constexpr int RED_PART = 8;   // per-block partials
+constexpr int HOST_MORE = 8;  // per-image results in ctx->h_red
 
 }  // namespace
 
@@ -152,6 +153,23 @@ int Context::ensure_red(size_t n) {
     return fail(LITHO_ERR_OOM, "reduction buffer allocation failed");
   }
   red_cap = n;
+  red_clean = false;
+  return LITHO_OK;
+}
+
+int Context::ensure_host(size_t n) {
+  if (h_cap >= n) return LITHO_OK;
+  double* p = nullptr;
+  if (cudaMallocHost(reinterpret_cast<void**>(&p), n * sizeof(double)) != cudaSuccess) {
+    cudaGetLastError();
+    return fail(LITHO_ERR_OOM, "pinned result buffer allocation failed");
+  }
+  if (h_red) {
+    cudaStreamSynchronize(stream);
+    cudaFreeHost(h_red);
+  }
+  h_red = p;
+  h_cap = n;
   return LITHO_OK;
 }
 
@@ -213,7 +231,7 @@ int litho_ctx_create(int device, void* stream, litho_ctx** out) {
     }
     c->own_stream = true;
   }
-  if (cudaMallocHost(reinterpret_cast<void**>(&c->h_red), 64 * sizeof(double)) != cudaSuccess) {
+  if (c->ensure_host(64) != LITHO_OK) {
     if (c->own_stream) cudaStreamDestroy(c->stream);
     delete c;
     return LITHO_ERR_OOM;
@@ -765,23 +783,32 @@ int run_adjoint(Context* ctx, const Cache& c, const Field& f, const Layout& L, c
   return st;
 }
 
-int prepare(Context* ctx, const Cache& c, Layout* L, int batch = 1, bool own_field = false) {
-  if (cudaSetDevice(ctx->device) != cudaSuccess) return ctx->fail(LITHO_ERR_CUDA, "cudaSetDevice");
-  *L = make_layout(c.g, batch, own_field);
-  int st = ctx->ensure_scratch(L->total);
-  if (st) return st;
-  // three partial sums per tile of an image: 64 x 64 (FP32 syntheses) at most
-  st = ctx->ensure_red(RED_PART + (3 * (size_t)synth_blocks(c.g.N) + 3) * batch + 1200);
-  if (st) return st;
-  LITHO_CUDA_TRY(ctx, cudaMemsetAsync(ctx->d_red, 0, RED_PART * sizeof(double), ctx->stream));
+// A zero reduction header (status, counters, sums) at the start of a call.
+int begin_red(Context* ctx) {
+  if (!ctx->red_clean)
+    LITHO_CUDA_TRY(ctx, cudaMemsetAsync(ctx->d_red, 0, RED_PART * sizeof(double), ctx->stream));
+  ctx->red_clean = false;
   return LITHO_OK;
 }
 
-// Copies n summed doubles (and the flag) back to the host and waits.
-int fetch(Context* ctx, int n) {
-  LITHO_CUDA_TRY(ctx, cudaMemcpyAsync(ctx->h_red, ctx->d_red, (RED_SUM + n) * sizeof(double),
-                                      cudaMemcpyDeviceToHost, ctx->stream));
+int reserve(Context* ctx, const Cache& c, Layout* L, int batch = 1, bool own_field = false) {
+  if (cudaSetDevice(ctx->device) != cudaSuccess) return ctx->fail(LITHO_ERR_CUDA, "cudaSetDevice");
+  *L = make_layout(c.g, batch, own_field);
+  const int st = ctx->ensure_scratch(L->total);
+  if (st) return st;
+  // three partial sums per tile of an image: 64 x 64 (FP32 syntheses) at most
+  return ctx->ensure_red(RED_PART + (3 * (size_t)synth_blocks(c.g.N) + 3) * batch + 1200);
+}
+
+int prepare(Context* ctx, const Cache& c, Layout* L, int batch = 1, bool own_field = false) {
+  const int st = reserve(ctx, c, L, batch, own_field);
+  return st ? st : begin_red(ctx);
+}
+
+// Waits for a call whose last kernel has handed its results to ctx->h_red.
+int wait_results(Context* ctx) {
   LITHO_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
+  ctx->red_clean = true;
   ctx->collect_stages();
   int tc_err;
   std::memcpy(&tc_err, reinterpret_cast<const char*>(ctx->h_red + RED_FLAG) + sizeof(int),
@@ -792,17 +819,30 @@ int fetch(Context* ctx, int n) {
   return LITHO_OK;
 }
 
-int* flag_word(const Context* ctx) { return reinterpret_cast<int*>(ctx->d_red + RED_FLAG); }
+// Hands the reduction header and nmore further doubles (to h_red + HOST_MORE, whose room the
+// caller has ensured) to the host and waits.
+int fetch(Context* ctx, const double* more = nullptr, int nmore = 0) {
+  const int st = check_launch(ctx, launch_publish(ctx->stream, ctx->d_red, RED_PART, ctx->h_red,
+                                                  more, nmore, ctx->h_red + HOST_MORE),
+                              "results");
+  ctx->launches += 1;
+  return st ? st : wait_results(ctx);
+}
 
-// deferred[0] |= the call's non-finite flag; deferred[1] keeps the first wait code.
-__global__ void merge_deferred_kernel(const int* __restrict__ flag, int* __restrict__ deferred) {
+// deferred[0] |= the call's non-finite flag; deferred[1] keeps the first wait code. The
+// reduction header is cleared: a caller's graph may replay this call between calls that
+// expect it zero.
+__global__ void merge_deferred_kernel(double* red, int* __restrict__ deferred) {
+  const int* flag = reinterpret_cast<const int*>(red + RED_FLAG);
   if (threadIdx.x == 0) {
     if (flag[0]) deferred[0] = 1;
     if (flag[1] && !deferred[1]) deferred[1] = flag[1];
   }
+  __syncwarp();
+  if (threadIdx.x < RED_PART) red[threadIdx.x] = 0.0;
 }
-cudaError_t launch_merge_deferred(cudaStream_t s, const int* flag, int* deferred) {
-  merge_deferred_kernel<<<1, 32, 0, s>>>(flag, deferred);
+cudaError_t launch_merge_deferred(cudaStream_t s, double* red, int* deferred) {
+  merge_deferred_kernel<<<1, 32, 0, s>>>(red, deferred);
   return cudaGetLastError();
 }
 
@@ -888,7 +928,7 @@ int litho_imaging_compute(litho_ctx* ctx, const litho_cache* cache, const float*
   ep.wafer = d_wafer;
   int nb = 0;
   st = run_forward(ctx, *cache, *f, L, 0, d_mask, nullptr, ep, &nb);
-  if (!st) st = fetch(ctx, 0);
+  if (!st) st = fetch(ctx);
   if (st) return st;
   if (flag_set(ctx)) {
     f->valid = false;
@@ -909,7 +949,7 @@ int litho_backpropagate(litho_ctx* ctx, const litho_field* field, const float* d
   ep.grad_mask = d_grad;
   int nb = 0;
   st = run_adjoint(ctx, c, *field, L, d_dLdI, output_scale, ep, &nb);
-  if (!st) st = fetch(ctx, 0);
+  if (!st) st = fetch(ctx);
   if (st) return st;
   if (flag_set(ctx)) return ctx->fail(LITHO_ERR_NONFINITE, "Gradient: dLdI must be finite");
   return LITHO_OK;
@@ -921,6 +961,7 @@ int litho_pe_loss(litho_ctx* ctx, const float* d_wafer, const float* d_target, i
     return LITHO_ERR_INVALID_ARGUMENT;
   if (cudaSetDevice(ctx->device) != cudaSuccess) return LITHO_ERR_CUDA;
   int st = ctx->ensure_red(RED_PART + 2 * 600);
+  if (!st) st = begin_red(ctx);
   if (st) return st;
   litho_pe_options o{nullptr, nullptr, 1.0, 0.0, 0.01};
   if (opt) o = *opt;
@@ -936,7 +977,7 @@ int litho_pe_loss(litho_ctx* ctx, const float* d_wafer, const float* d_target, i
                     "sum");
   if (st) return st;
   ctx->launches += 2;
-  st = fetch(ctx, 2);
+  st = fetch(ctx);
   if (st) return st;
   // pe_weight * Loss::pe_loss + penalty * Loss::background_penalty_loss; with
   // pe_weight 1 this is Loss::pe_loss_with_penalty (loss.cpp:25-51).
@@ -973,7 +1014,7 @@ int litho_pe_gradient(litho_ctx* ctx, const litho_field* field, const float* d_w
   ep.grad_mask = d_grad;
   int nb2 = 0;
   st = run_adjoint(ctx, c, *field, L, at<float>(ctx, L.dldi), 4.0 * alpha, ep, &nb2);
-  if (!st) st = fetch(ctx, 2);
+  if (!st) st = fetch(ctx);
   if (st) return st;
   if (loss) *loss = o.pe_weight * ctx->h_red[RED_SUM] + o.penalty * ctx->h_red[RED_SUM + 1];
   return LITHO_OK;
@@ -1028,11 +1069,12 @@ static int ctm_evaluate_impl(litho_ctx* ctx, const litho_cache* cache, litho_fie
     if (!r)
       r = run_adjoint(ctx, *cache, *f, L, at<float>(ctx, L.dldi), 4.0 * alpha, gp, &nb2, fuse);
     // Both FP64 sums (loss terms and the gradient norm) in one launch at the end, off
-    // the path between the forward and the adjoint.
+    // the path between the forward and the adjoint; it hands the results to the host.
     if (!r)
       r = check_launch(ctx, launch_sum_partials2(ctx->stream, ctx->d_red + RED_PART, nb, 2,
-                                                 ctx->d_red + RED_SUM, gp.norm_partial, nb2, 1,
-                                                 ctx->d_red + RED_SUM + 2),
+                                                 ctx->h_red + RED_SUM, gp.norm_partial, nb2, 1,
+                                                 ctx->h_red + RED_SUM + 2,
+                                                 ctx->d_red + RED_FLAG, ctx->h_red + RED_FLAG),
                        "sum");
     ctx->launches += 1;
     return r;
@@ -1040,14 +1082,15 @@ static int ctm_evaluate_impl(litho_ctx* ctx, const litho_cache* cache, litho_fie
   // Repeated evaluations on the same buffers replay a CUDA graph of the chain.
   const BandGeom& g = cache->g;
   EvalKey key;
-  const void* ptrs[16] = {cache,       f->e,          f->mband,          d_theta,
+  const void* ptrs[17] = {cache,       f->e,          f->mband,          d_theta,
                           d_target,    d_mask,        d_aerial,          d_wafer,
                           d_grad_mask, d_grad_theta,  ctx->scratch.base, ctx->d_red,
                           cache->H,    cache->AYD_img, cache->TXS,
                           reinterpret_cast<const void*>(
                               (uintptr_t)ctx->precision |
-                              ((uintptr_t)ctx->tc_persistent(cache->g.N, 1) << 4))};
-  for (int i = 0; i < 16; ++i) key.ptr[i] = ptrs[i];
+                              ((uintptr_t)ctx->tc_persistent(cache->g.N, 1) << 4)),
+                          ctx->h_red};
+  for (int i = 0; i < 17; ++i) key.ptr[i] = ptrs[i];
   const int geom[6] = {g.N, g.K, g.Nr, g.Nc, g.row0, g.col0};
   for (int i = 0; i < 6; ++i) key.geom[i] = geom[i];
   key.thr = threshold;
@@ -1091,7 +1134,7 @@ static int ctm_evaluate_impl(litho_ctx* ctx, const litho_cache* cache, litho_fie
   }
   ctx->eval_last_key = key;
   ctx->eval_last_valid = graphable;
-  if (!st) st = fetch(ctx, 3);
+  if (!st) st = wait_results(ctx);
   if (st) return st;
   if (flag_set(ctx)) {
     f->valid = false;
@@ -1113,12 +1156,13 @@ int litho_ctm_evaluate(litho_ctx* ctx, const litho_cache* cache, litho_field* fi
 }
 
 // The batched tensor-core chain on ctx->stream, without a host round trip: per
-// image {PE, penalty term, ||dPE/dtheta||^2} into d_sums ([batch][3], device). L
+// image {PE, penalty term, ||dPE/dtheta||^2} into sums ([batch][3]; device memory, or with
+// `last` pinned host memory, to which the call's status goes too). L
 // comes from prepare(ctx, c, &L, batch, true) (band state of every image included;
 // batch > 1 includes it anyway); the partials use the reduction area.
 static int ctm_batch_chain(Context* ctx, const Cache& c, const Layout& L, int batch,
                            const float* d_theta, const float* d_target, double threshold,
-                           double alpha, float* d_grad_theta, double* d_sums) {
+                           double alpha, float* d_grad_theta, double* sums, bool last = false) {
   Field f;
   f.cache = &c;
   f.e = at<float2>(ctx, L.fe);
@@ -1141,7 +1185,9 @@ static int ctm_batch_chain(Context* ctx, const Cache& c, const Layout& L, int ba
   if (!st) st = run_adjoint(ctx, c, f, L, nullptr, 4.0 * alpha, gp, &nb2, true, batch);
   if (!st)
     st = check_launch(ctx, launch_sum_partials_batch(ctx->stream, ctx->d_red + RED_PART, nb, 2,
-                                                     gp.norm_partial, nb2, 1, d_sums, batch),
+                                                     gp.norm_partial, nb2, 1, sums, 3, batch,
+                                                     last ? ctx->d_red + RED_FLAG : nullptr,
+                                                     ctx->h_red + RED_FLAG),
                       "sum");
   ctx->launches += 1;
   return st;
@@ -1171,23 +1217,25 @@ int litho_ctm_evaluate_batch(litho_ctx* ctx, const litho_cache* cache, int batch
     return LITHO_OK;
   }
   Layout L;
-  int st = prepare(ctx, *cache, &L, batch);
+  int st = ctx->ensure_host(HOST_MORE + 3 * (size_t)batch);
+  if (!st) st = prepare(ctx, *cache, &L, batch);
   if (st) return st;
-  double* d_sums = ctx->d_red + RED_PART + 3 * (size_t)L.tiles * batch;
+  const double* sums = ctx->h_red + HOST_MORE;
   auto chain = [&]() {
     return ctm_batch_chain(ctx, *cache, L, batch, d_theta, d_target, threshold, alpha,
-                           d_grad_theta, d_sums);
+                           d_grad_theta, ctx->h_red + HOST_MORE, true);
   };
   // Repeated calls on the same buffers replay a CUDA graph of the chain (captured on
   // the second consecutive call with the same key), as the single-image evaluation does.
   EvalKey key;
-  const void* ptrs[16] = {cache, d_theta, d_target, d_grad_theta, ctx->scratch.base, ctx->d_red,
+  const void* ptrs[17] = {cache, d_theta, d_target, d_grad_theta, ctx->scratch.base, ctx->d_red,
                           cache->H, cache->AYD_img, cache->TXS_img, cache->TXD_img,
                           reinterpret_cast<const void*>((uintptr_t)batch),
                           reinterpret_cast<const void*>(
                               (uintptr_t)ctx->precision | ((uintptr_t)ctx->tc_persistent(g.N, batch) << 4) |
-                              ((uintptr_t)ctx->band_width(g.N, batch) << 8))};
-  for (int i = 0; i < 16; ++i) key.ptr[i] = ptrs[i];
+                              ((uintptr_t)ctx->band_width(g.N, batch) << 8)),
+                          ctx->h_red};
+  for (int i = 0; i < 17; ++i) key.ptr[i] = ptrs[i];
   const int geom[6] = {g.N, g.K, g.Nr, g.Nc, g.row0, g.col0};
   for (int i = 0; i < 6; ++i) key.geom[i] = geom[i];
   key.thr = threshold;
@@ -1229,11 +1277,7 @@ int litho_ctm_evaluate_batch(litho_ctx* ctx, const litho_cache* cache, int batch
   }
   ctx->batch_last_key = key;
   ctx->batch_last_valid = graphable;
-  std::vector<double> sums(3 * (size_t)batch);
-  if (!st)
-    LITHO_CUDA_TRY(ctx, cudaMemcpyAsync(sums.data(), d_sums, sums.size() * sizeof(double),
-                                        cudaMemcpyDeviceToHost, ctx->stream));
-  if (!st) st = fetch(ctx, 0);
+  if (!st) st = wait_results(ctx);
   if (st) return st;
   if (flag_set(ctx)) return ctx->fail(LITHO_ERR_NONFINITE, "theta must be finite");
   for (int b = 0; b < batch; ++b) {
@@ -1258,8 +1302,12 @@ static int pe_gradient_batch_impl(litho_ctx* ctx, const litho_cache* cache, int 
   const BandGeom& g = cache->g;
   const size_t px = (size_t)g.N * g.N;
   const bool tc = ctx->precision == LITHO_PRECISION_BF16X3 && cache->TXD_img != nullptr;
+  const bool device_out = d_losses != nullptr;
   Layout L;
-  int st = prepare(ctx, *cache, &L, tc ? batch : 1, true);
+  int st = device_out ? LITHO_OK : ctx->ensure_host(HOST_MORE + 2 * (size_t)batch);
+  // a caller's graph that captures the device-resident call carries its own clear
+  if (device_out) ctx->red_clean = false;
+  if (!st) st = prepare(ctx, *cache, &L, tc ? batch : 1, true);
   if (st) return st;
   Field f;
   f.cache = cache;
@@ -1276,7 +1324,6 @@ static int pe_gradient_batch_impl(litho_ctx* ctx, const litho_cache* cache, int 
   ep.loss_partial = ctx->d_red + RED_PART;
   GradEpilogue gp{};
   cudaStream_t s = ctx->stream;
-  const bool device_out = d_losses != nullptr;
   if (device_out) {
     st = ctx->ensure_deferred();
     if (st) return st;
@@ -1288,25 +1335,20 @@ static int pe_gradient_batch_impl(litho_ctx* ctx, const litho_cache* cache, int 
     int nb = 0, nb2 = 0;
     st = run_forward(ctx, *cache, f, L, 0, d_masks, nullptr, ep, &nb, nullptr, true, batch);
     if (!st) st = run_adjoint(ctx, *cache, f, L, nullptr, 4.0 * alpha, gp, &nb2, true, batch);
-    double* d_sums = ctx->d_red + RED_PART + 2 * (size_t)nb * batch;
+    double* sums = device_out ? d_losses : ctx->h_red + HOST_MORE;
     if (!st)
-      st = check_launch(ctx, launch_sum_partials_batch(s, ctx->d_red + RED_PART, nb, 2,
-                                                       ctx->d_red + RED_PART, 0, 0, d_sums, batch),
+      st = check_launch(ctx, launch_sum_partials_batch(
+                                 s, ctx->d_red + RED_PART, nb, 2, ctx->d_red + RED_PART, 0, 0,
+                                 sums, 2, batch, device_out ? nullptr : ctx->d_red + RED_FLAG,
+                                 ctx->h_red + RED_FLAG),
                         "sum");
     ctx->launches += 1;
     if (device_out) {
-      if (!st)
-        LITHO_CUDA_TRY(ctx, cudaMemcpyAsync(d_losses, d_sums, 2 * (size_t)batch * sizeof(double),
-                                            cudaMemcpyDeviceToDevice, s));
-      if (!st) st = check_launch(ctx, launch_merge_deferred(s, flag_word(ctx), ctx->d_deferred),
+      if (!st) st = check_launch(ctx, launch_merge_deferred(s, ctx->d_red, ctx->d_deferred),
                                  "deferred status");
       return st;
     }
-    std::vector<double> sums(2 * (size_t)batch);
-    if (!st)
-      LITHO_CUDA_TRY(ctx, cudaMemcpyAsync(sums.data(), d_sums, sums.size() * sizeof(double),
-                                          cudaMemcpyDeviceToHost, s));
-    if (!st) st = fetch(ctx, 0);
+    if (!st) st = wait_results(ctx);
     if (st) return st;
     if (flag_set(ctx)) return ctx->fail(LITHO_ERR_NONFINITE, "mask must be finite");
     for (int b = 0; b < batch && losses; ++b) losses[b] = sums[2 * (size_t)b];
@@ -1315,6 +1357,8 @@ static int pe_gradient_batch_impl(litho_ctx* ctx, const litho_cache* cache, int 
   // FP32: one image after another through the same chain with dL/dI stored between
   // the resist synthesis and the adjoint.
   for (int b = 0; b < batch; ++b) {
+    if (!device_out) st = begin_red(ctx);
+    if (st) return st;
     ep.target = d_targets + b * px;
     ep.dldi = at<float>(ctx, L.dldi);
     gp.grad_mask = d_grad_masks + b * px;
@@ -1333,13 +1377,13 @@ static int pe_gradient_batch_impl(litho_ctx* ctx, const litho_cache* cache, int 
       if (st) return st;
       continue;
     }
-    if (!st) st = fetch(ctx, 2);
+    if (!st) st = fetch(ctx);
     if (st) return st;
     if (flag_set(ctx)) return ctx->fail(LITHO_ERR_NONFINITE, "mask must be finite");
     if (losses) losses[b] = ctx->h_red[RED_SUM];
   }
   if (device_out)
-    return check_launch(ctx, launch_merge_deferred(s, flag_word(ctx), ctx->d_deferred),
+    return check_launch(ctx, launch_merge_deferred(s, ctx->d_red, ctx->d_deferred),
                         "deferred status");
   return LITHO_OK;
 }
@@ -1479,8 +1523,10 @@ int litho_ctm_evaluate_host_batch(litho_ctx* ctx, const litho_cache* cache, int 
     }
   }
   Layout L;
-  int st = prepare(ctx, *cache, &L, G, true);   // with the band state of G images
+  int st = ctx->ensure_host(HOST_MORE + 3 * (size_t)batch);
+  if (!st) st = prepare(ctx, *cache, &L, G, true);   // with the band state of G images
   if (st) return st;
+  const double* sums = ctx->h_red + HOST_MORE;
   float* base = static_cast<float*>(ctx->pipe_stage.base);
   double* d_sums = reinterpret_cast<double*>(base + 2 * slot_floats);
   cudaStream_t up = ctx->aux, cp = ctx->stream, dn = ctx->dn;
@@ -1518,15 +1564,11 @@ int litho_ctm_evaluate_host_batch(litho_ctx* ctx, const litho_cache* cache, int 
          cudaEventRecord(ev[DN], dn) == cudaSuccess;
     if (!ok) st = ctx->fail(LITHO_ERR_CUDA, "host batch: download failed");
   }
-  std::vector<double> sums(3 * (size_t)batch);
-  if (!st)
-    LITHO_CUDA_TRY(ctx, cudaMemcpyAsync(sums.data(), d_sums, sums.size() * sizeof(double),
-                                        cudaMemcpyDeviceToHost, cp));
   if (cudaStreamSynchronize(dn) != cudaSuccess && !st)
     st = ctx->fail(LITHO_ERR_CUDA, "download stream synchronize failed");
   if (cudaStreamSynchronize(up) != cudaSuccess && !st)
     st = ctx->fail(LITHO_ERR_CUDA, "upload stream synchronize failed");
-  if (!st) st = fetch(ctx, 0);
+  if (!st) st = fetch(ctx, d_sums, 3 * batch);
   if (st) return st;
   if (flag_set(ctx)) return ctx->fail(LITHO_ERR_NONFINITE, "theta must be finite");
   for (int b = 0; b < batch; ++b) {
@@ -1595,8 +1637,8 @@ static size_t dt_slots(int n) { return (size_t)n + ((size_t)n + 1) / 2; }
 static int ls_dt(litho_ctx* ctx, int rows, int cols, const float* d_vn, double dx, double dy,
                  double cfl, double b, float** dt_dev) {
   int st = ctx->ensure_red(RED_PART + 2 * 600);
+  if (!st) st = begin_red(ctx);
   if (st) return st;
-  LITHO_CUDA_TRY(ctx, cudaMemsetAsync(ctx->d_red, 0, RED_PART * sizeof(double), ctx->stream));
   float* vd = reinterpret_cast<float*>(ctx->d_red + RED_SUM);   // max |Vn|, dt
   st = check_launch(ctx, launch_speed_dt(ctx->stream, d_vn, (size_t)rows * cols, 1, (float)dx,
                                          (float)dy, (float)cfl, (float)b, vd,
@@ -1621,7 +1663,7 @@ int litho_evolution_term(litho_ctx* ctx, int rows, int cols, const float* d_phi,
                                          (float)dx, (float)dy, (float)b, dtd, d_normal, nullptr),
                     "evolution");
   ctx->launches += 1;
-  if (!st) st = fetch(ctx, 1);
+  if (!st) st = fetch(ctx);
   if (st) return st;
   if (flag_set(ctx)) return ctx->fail(LITHO_ERR_NONFINITE, "normal speed must be finite");
   float h[2];
@@ -1898,7 +1940,7 @@ int litho_lsm_rk2_update(litho_ctx* ctx, int rows, int cols, const float* d_phi,
                       "rk2 stage 2");
   ctx->stage_end(8);
   ctx->launches += 2;
-  if (!st) st = fetch(ctx, 1);
+  if (!st) st = fetch(ctx);
   if (st) return st;
   if (flag_set(ctx)) return ctx->fail(LITHO_ERR_NONFINITE, "normal speed must be finite");
   float h[2];
@@ -1922,7 +1964,9 @@ static int rk2_update_batch_impl(litho_ctx* ctx, int batch, int rows, int cols,
   if (st) return st;
   // The per-image (max |Vn|, dt) pairs and CTA counters, cleared with the header.
   st = ctx->ensure_red(RED_PART + dt_slots(batch));
+  if (!st && !device_out) st = ctx->ensure_host(HOST_MORE + (size_t)batch);
   if (st) return st;
+  ctx->red_clean = false;
   LITHO_CUDA_TRY(ctx, cudaMemsetAsync(ctx->d_red, 0, (RED_PART + dt_slots(batch)) * sizeof(double),
                                       ctx->stream));
   float* phi1 = static_cast<float*>(ctx->scratch.base);
@@ -1951,16 +1995,13 @@ static int rk2_update_batch_impl(litho_ctx* ctx, int batch, int rows, int cols,
       st = check_launch(ctx, cudaGetLastError(), "dt export");
       ctx->launches += 1;
     }
-    if (!st) st = check_launch(ctx, launch_merge_deferred(s, bad, ctx->d_deferred), "deferred status");
+    if (!st) st = check_launch(ctx, launch_merge_deferred(s, ctx->d_red, ctx->d_deferred), "deferred status");
     return st;
   }
-  std::vector<float> h(2 * (size_t)batch);
-  if (!st)
-    LITHO_CUDA_TRY(ctx, cudaMemcpyAsync(h.data(), vd, h.size() * sizeof(float),
-                                        cudaMemcpyDeviceToHost, s));
-  if (!st) st = fetch(ctx, 0);
+  if (!st) st = fetch(ctx, ctx->d_red + RED_PART, batch);
   if (st) return st;
   if (flag_set(ctx)) return ctx->fail(LITHO_ERR_NONFINITE, "normal speed must be finite");
+  const float* h = reinterpret_cast<const float*>(ctx->h_red + HOST_MORE);
   for (int i = 0; i < batch && dts; ++i) dts[i] = h[2 * (size_t)i + 1];
   return LITHO_OK;
 }
@@ -2043,7 +2084,6 @@ struct litho_partition {
   double* d_loss = nullptr;
   double* d_xpart = nullptr;   // exchange partial sums: ntiles * kMaxRel * 32
 
-  std::vector<double> h_loss;
   // EPE work, allocated when an EPE term or the Core metrics are asked for: EPE
   // windows, the PE_EPE main region and its row-pass temporary (ntiles * ts * ts
   // each), then one tile each of aerial and wafer image.
@@ -2318,7 +2358,7 @@ int litho_exchange_compute_epe(litho_ctx* ctx, const litho_partition* cp, const 
                        n > 1;
   const int group = batched ? exchange_group(ctx, cache->g, n) : 1;
   Layout L;
-  int st = prepare(ctx, *cache, &L, group, batched);
+  int st = reserve(ctx, *cache, &L, group, batched);
   if (st) return st;
   const bool guard_region = o.loss_region == LITHO_MICRO_REGION_CORE_GUARD;
   const int periods = guard_region ? 1 : 0;
@@ -2333,7 +2373,6 @@ int litho_exchange_compute_epe(litho_ctx* ctx, const litho_partition* cp, const 
       cudaGetLastError();
       return ctx->fail(LITHO_ERR_OOM, "full-chip work allocation failed");
     }
-    p->h_loss.assign((size_t)(S + 1) * n, 0.0);
   }
   // EP work: EPE window, main region, dilation scratch (n tiles each), then the
   // aerial and wafer images and the dL/dI of a group of tiles.
@@ -2390,8 +2429,9 @@ int litho_exchange_compute_epe(litho_ctx* ctx, const litho_partition* cp, const 
   st = ctx->ensure_red(RED_PART + std::max<size_t>(3 * (size_t)std::max(epe_blocks, 64) + 8,
                                                    6 * ((size_t)rect_losses_batch_blocks(ts) + 1) *
                                                            group + 8));
+  if (!st) st = ctx->ensure_host(HOST_MORE + (size_t)(S + 1) * n);
+  if (!st) st = begin_red(ctx);
   if (st) return st;
-  LITHO_CUDA_TRY(ctx, cudaMemsetAsync(ctx->d_red, 0, RED_PART * sizeof(double), ctx->stream));
   float* targets = p->d_work;
   float* pe_w = targets + n * tt;
   float* pen_w = pe_w + n * tt;
@@ -2494,7 +2534,7 @@ int litho_exchange_compute_epe(litho_ctx* ctx, const litho_partition* cp, const 
                        "region and core losses");
       if (!r)
         r = check_launch(ctx, launch_sum_partials_batch(s, part, rect_losses_batch_blocks(ts), 6,
-                                                        part, 0, 0, slot + 5, 1),
+                                                        part, 0, 0, slot + 5, S, 1),
                          "sum");
       ctx->launches += 2;
     }
@@ -2554,20 +2594,16 @@ int litho_exchange_compute_epe(litho_ctx* ctx, const litho_partition* cp, const 
     ep.loss_partial = part;
     int nb = 0, nb2 = 0;
     st = run_forward(ctx, *cache, fb, L, 0, d_masks + t0 * tt, nullptr, ep, &nb, nullptr, fuse, B);
-    double* sums = part + 2 * (size_t)nb * B;
     if (!st)
-      st = check_launch(ctx, launch_sum_partials_batch(s, part, nb, 2, part, 0, 0, sums, B), "sum");
+      st = check_launch(ctx, launch_sum_partials_batch(s, part, nb, 2, part, 0, 0,
+                                                       p->d_loss + (size_t)S * t0, S, B),
+                        "sum");
     ctx->launches += 1;
-    if (!st)
-      LITHO_CUDA_TRY(ctx, cudaMemcpy2DAsync(p->d_loss + (size_t)S * t0, S * sizeof(double), sums,
-                                            2 * sizeof(double), 2 * sizeof(double), B,
-                                            cudaMemcpyDeviceToDevice, s));
     if (!st && zero_pe_dldi)
       LITHO_CUDA_TRY(ctx, cudaMemsetAsync(dldi_group, 0, B * tt * sizeof(float), s));
     if (!st && core) {
       // Loss-region and Core sums of the group's tiles in one launch, to slots 5..10.
       const int nbr = rect_losses_batch_blocks(ts);
-      double* sums6 = part + 6 * (size_t)nbr * B;
       st = check_launch(ctx, launch_rect_losses_batch(
                                  s, wafer, targets + t0 * tt, pe_w + t0 * tt, pen_w + t0 * tt, ts,
                                  p->d_meta + (guard_region ? p->off_update : p->off_core_l) + 4 * t0,
@@ -2575,12 +2611,9 @@ int litho_exchange_compute_epe(litho_ctx* ctx, const litho_partition* cp, const 
                                  part, B),
                         "region and core losses");
       if (!st)
-        st = check_launch(ctx, launch_sum_partials_batch(s, part, nbr, 6, part, 0, 0, sums6, B),
+        st = check_launch(ctx, launch_sum_partials_batch(s, part, nbr, 6, part, 0, 0,
+                                                         p->d_loss + (size_t)S * t0 + 5, S, B),
                           "sum");
-      if (!st)
-        LITHO_CUDA_TRY(ctx, cudaMemcpy2DAsync(p->d_loss + (size_t)S * t0 + 5, S * sizeof(double),
-                                              sums6, 6 * sizeof(double), 6 * sizeof(double), B,
-                                              cudaMemcpyDeviceToDevice, s));
       ctx->launches += 2;
     }
     for (int b = 0; eval_epe && b < B && !st; ++b)
@@ -2629,22 +2662,19 @@ int litho_exchange_compute_epe(litho_ctx* ctx, const litho_partition* cp, const 
                                            d_grad, p->d_loss + (size_t)S * n, p->d_xpart),
                       "micro-gradient exchange");
   ctx->launches += 1;
-  if (!st)
-    LITHO_CUDA_TRY(ctx, cudaMemcpyAsync(p->h_loss.data(), p->d_loss,
-                                        (size_t)(S + 1) * n * sizeof(double),
-                                        cudaMemcpyDeviceToHost, s));
-  if (!st) st = fetch(ctx, 0);
+  if (!st) st = fetch(ctx, p->d_loss, (S + 1) * n);
   if (st) return st;
   if (flag_set(ctx)) return ctx->fail(LITHO_ERR_NONFINITE, "Imaging: mask, threshold, and alpha must be finite");
+  const double* h_loss = ctx->h_red + HOST_MORE;
   double tot[3] = {0.0, 0.0, 0.0};
   const bool report_bg = o.loss_type == LITHO_MICRO_LOSS_PE_PENALTY || core;
   for (int t = 0; t < n; ++t) {
-    const double* h = &p->h_loss[(size_t)S * t];
+    const double* h = h_loss + (size_t)S * t;
     // With the wafer image at hand the loss-region sums come from it; otherwise from
     // the resist epilogue (whose background sum runs only under a penalty).
     const double pe = core ? h[5] : h[0];
     const double bg = core ? h[6] : h[1];
-    const double cept = p->h_loss[(size_t)S * n + t];
+    const double cept = h_loss[(size_t)S * n + t];
     const double epe_loss = eval_epe ? h[2] : 0.0;
     const double data = wpe * pe + wpen * bg + wepe * epe_loss;
     const double loss = data + (o.enable_cept ? o.cept_weight * cept : 0.0);
@@ -2791,7 +2821,9 @@ int litho_fullchip_lsm_step(litho_ctx* ctx, const litho_partition* p, const floa
   int st = ctx->ensure_scratch(2 * (size_t)G * tt * sizeof(float));
   if (st) return st;
   st = ctx->ensure_red(RED_PART + dt_slots(n));
+  if (!st) st = ctx->ensure_host(HOST_MORE + (size_t)n);
   if (st) return st;
+  ctx->red_clean = false;
   float* vw = static_cast<float*>(ctx->scratch.base);  // windowed speed of the chunk
   float* phi1 = vw + (size_t)G * tt;                   // RK2 stage 1, then the reinit distance
   cudaStream_t s = ctx->stream;
@@ -2846,12 +2878,10 @@ int litho_fullchip_lsm_step(litho_ctx* ctx, const litho_partition* p, const floa
                       "render_levelset_mask");
   ctx->launches += 1;
   if (st) return st;
-  std::vector<float> h(2 * (size_t)n);
-  LITHO_CUDA_TRY(ctx, cudaMemcpyAsync(h.data(), vd, h.size() * sizeof(float),
-                                      cudaMemcpyDeviceToHost, s));
-  st = fetch(ctx, 0);
+  st = fetch(ctx, ctx->d_red + RED_PART, n);
   if (st) return st;
   if (flag_set(ctx)) return ctx->fail(LITHO_ERR_NONFINITE, "normal speed must be finite");
+  const float* h = reinterpret_cast<const float*>(ctx->h_red + HOST_MORE);
   float lo = h[1], hi = h[1];
   for (int t = 1; t < n; ++t) {
     lo = std::min(lo, h[2 * (size_t)t + 1]);
@@ -2888,7 +2918,8 @@ int litho_evaluate_sparse_epe(litho_ctx* ctx, int rows, int cols, const float* d
   double* d_w = d_eps + 2 * n;
   double* d_se = d_w + n;
   cudaStream_t s = ctx->stream;
-  LITHO_CUDA_TRY(ctx, cudaMemsetAsync(ctx->d_red, 0, RED_PART * sizeof(double), s));
+  st = begin_red(ctx);
+  if (st) return st;
   if (n > 0) {
     LITHO_CUDA_TRY(ctx, cudaMemcpyAsync(d_eps, eps, 2 * n * sizeof(double), cudaMemcpyHostToDevice, s));
     LITHO_CUDA_TRY(ctx, cudaMemcpyAsync(d_w, weights, n * sizeof(double), cudaMemcpyHostToDevice, s));
@@ -2907,7 +2938,7 @@ int litho_evaluate_sparse_epe(litho_ctx* ctx, int rows, int cols, const float* d
   if (signed_epe && n > 0)
     LITHO_CUDA_TRY(ctx, cudaMemcpyAsync(signed_epe, d_se, n * sizeof(double),
                                         cudaMemcpyDeviceToHost, s));
-  st = fetch(ctx, 3);
+  st = fetch(ctx);
   if (st) return st;
   if (totals) std::memcpy(totals, ctx->h_red + RED_SUM, 3 * sizeof(double));
   return LITHO_OK;
@@ -2926,7 +2957,7 @@ int litho_epe_gradient(litho_ctx* ctx, const litho_field* field, const float* d_
   const int N = c.g.N;
   if (N < 3) return ctx->fail(LITHO_ERR_SHAPE, "epe_gradient: the image needs at least 3 x 3 pixels");
   Layout L;
-  int st = prepare(ctx, c, &L);
+  int st = reserve(ctx, c, &L);
   if (st) return st;
   const int n = n_eps;
   const size_t ep_off = align_up(L.total, 256);
@@ -2937,7 +2968,8 @@ int litho_epe_gradient(litho_ctx* ctx, const litho_field* field, const float* d_
   const int nb = n == 0 ? 1 : (n + 255) / 256;
   st = ctx->ensure_red(RED_PART + 3 * (size_t)nb + 8);
   if (st) return st;
-  LITHO_CUDA_TRY(ctx, cudaMemsetAsync(ctx->d_red, 0, RED_PART * sizeof(double), ctx->stream));
+  st = begin_red(ctx);
+  if (st) return st;
   double* d_eps = at<double>(ctx, ep_off);
   double* d_w = d_eps + 2 * n;
   cudaStream_t s = ctx->stream;
@@ -2959,7 +2991,7 @@ int litho_epe_gradient(litho_ctx* ctx, const litho_field* field, const float* d_
   ep.grad_mask = d_grad;
   int nb2 = 0;
   st = run_adjoint(ctx, c, *field, L, dldi, 2.0, ep, &nb2);
-  if (!st) st = fetch(ctx, 0);
+  if (!st) st = fetch(ctx);
   if (st) return st;
   if (flag_set(ctx)) return ctx->fail(LITHO_ERR_NONFINITE, "epe_gradient: dL/dI must be finite");
   return LITHO_OK;

@@ -96,11 +96,11 @@ struct Scratch {
 // Identity of one CTM evaluation's launch chain: every device pointer it
 // touches, the band geometry and the scalars baked into its kernels.
 struct EvalKey {
-  const void* ptr[16] = {};
+  const void* ptr[17] = {};
   int geom[6] = {};
   double thr = 0.0, alpha = 0.0;
   bool operator==(const EvalKey& o) const {
-    for (int i = 0; i < 16; ++i)
+    for (int i = 0; i < 17; ++i)
       if (ptr[i] != o.ptr[i]) return false;
     for (int i = 0; i < 6; ++i)
       if (geom[i] != o.geom[i]) return false;
@@ -141,7 +141,13 @@ struct Context {
   int* d_deferred = nullptr;
   int ensure_deferred();
   size_t red_cap = 0;
-  double* h_red = nullptr;       // pinned host mirror for results
+  // The header of d_red is zero: the last call handed it over and cleared it.
+  bool red_clean = false;
+  // Pinned host memory that the last kernel of a call writes its results to: the header of
+  // d_red, then (from HOST_MORE) per-image results.
+  double* h_red = nullptr;
+  size_t h_cap = 0;
+  int ensure_host(size_t n);
   std::string last_error;
   long long launches = 0;        // kernel launches issued by the library
   // Optional per-stage CUDA-event timing (litho_ctx_enable_stage_timing).
@@ -299,11 +305,19 @@ cudaError_t launch_synth_grad(cudaStream_t s, const float* AYt, const float* Bt,
 cudaError_t launch_sum_partials(cudaStream_t s, const double* part, int n, int stride,
                                 double* out);
 cudaError_t launch_sum_partials2(cudaStream_t s, const double* a, int na, int sa, double* out_a,
-                                 const double* b, int nb, int sb, double* out_b);
+                                 const double* b, int nb, int sb, double* out_b,
+                                 double* status = nullptr, double* host_status = nullptr);
 // Batched sums: per image b, sa components over na blocks of a (stride na sa per
-// image) then sb over nb blocks of b, into out[b][sa + sb].
+// image) then sb over nb blocks of b, into out[b ldo + 0..sa + sb). With `status` (both sums):
+// the last launch of a call, status and outputs in pinned host memory.
 cudaError_t launch_sum_partials_batch(cudaStream_t s, const double* a, int na, int sa,
-                                      const double* b, int nb, int sb, double* out, int batch);
+                                      const double* b, int nb, int sb, double* out, int ldo,
+                                      int batch, double* status = nullptr,
+                                      double* host_status = nullptr);
+// Copies nhead doubles (at most 256) of the reduction header and nmore others to pinned host
+// memory and clears the header.
+cudaError_t launch_publish(cudaStream_t s, double* head, int nhead, double* host,
+                           const double* more, int nmore, double* host_more);
 cudaError_t launch_export_field(cudaStream_t s, const Cache& c, const Field& f, int k,
                                 float2* tmp_rows, float2* out);
 cudaError_t launch_pe_loss(cudaStream_t s, const float* w, const float* t, const float* pe_win,
