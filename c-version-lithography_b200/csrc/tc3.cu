@@ -53,10 +53,27 @@ __device__ __forceinline__ uint8_t* align1024(uint8_t* p) {
 // then records `code` in *err (first failure wins) and returns false.
 __device__ __forceinline__ bool pwait(uint32_t bar, uint32_t parity, volatile int* fail, int* err,
                                       int code) {
+  if (tc::mbar_try_wait(bar, parity)) return true;
   const long long t0 = clock64();
   while (!tc::mbar_try_wait(bar, parity)) {
     if (*fail) return false;
     if (clock64() - t0 > (1LL << 31)) {
+      *fail = 1;
+      atomicCAS(err, 0, code);
+      return false;
+    }
+  }
+  return true;
+}
+// The same for a whole warp, which stays converged (the MMA warps).
+__device__ __forceinline__ bool pwait_warp(uint32_t bar, uint32_t parity, volatile int* fail,
+                                           int* err, int code) {
+  constexpr unsigned ALL = 0xffffffffu;
+  if (__all_sync(ALL, tc::mbar_try_wait(bar, parity))) return true;
+  const long long t0 = clock64();
+  while (!__all_sync(ALL, tc::mbar_try_wait(bar, parity))) {
+    if (__any_sync(ALL, *fail)) return false;
+    if (__any_sync(ALL, clock64() - t0 > (1LL << 31))) {
       *fail = 1;
       atomicCAS(err, 0, code);
       return false;
@@ -109,12 +126,12 @@ template <int NV>
 struct EpiSums {
   double v[EPI_SLOTS][16][NV];
 };
-template <int NV>
+template <int NP, int NV>
 __device__ __forceinline__ void epi_put(EpiSums<NV>& sh, uint32_t red_bar, int b,
-                                        const double (&v)[NV]) {
-  double t[NV];
+                                        const double (&v)[NP]) {
+  double t[NV] = {};   // values past NP are zero
 #pragma unroll
-  for (int k = 0; k < NV; ++k) {
+  for (int k = 0; k < NP; ++k) {
     t[k] = v[k];
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) t[k] += __shfl_xor_sync(0xffffffffu, t[k], o);
@@ -137,6 +154,21 @@ __device__ __forceinline__ bool epi_take(const EpiSums<NV>& sh, uint32_t red_bar
     for (int w = 0; w < nw; ++w) out[k] += sh.v[b][w][k];
   }
   return true;
+}
+
+// s2_mma_swapped of two 128-row tiles for the kp that the pipelines take.
+__device__ __forceinline__ void s2_mma_swapped_kp(uint32_t acc, uint32_t sa, uint32_t sb, int kp,
+                                                  uint32_t idesc, uint32_t lead) {
+  switch (kp) {
+    case 16: return s2_mma_swapped<16>(acc, sa, 128, sb, 128, idesc, lead);
+    case 32: return s2_mma_swapped<32>(acc, sa, 128, sb, 128, idesc, lead);
+    case 48: return s2_mma_swapped<48>(acc, sa, 128, sb, 128, idesc, lead);
+    case 64: return s2_mma_swapped<64>(acc, sa, 128, sb, 128, idesc, lead);
+    case 80: return s2_mma_swapped<80>(acc, sa, 128, sb, 128, idesc, lead);
+    case 96: return s2_mma_swapped<96>(acc, sa, 128, sb, 128, idesc, lead);
+    case 112: return s2_mma_swapped<112>(acc, sa, 128, sb, 128, idesc, lead);
+    default: return s2_mma_swapped<128>(acc, sa, 128, sb, 128, idesc, lead);
+  }
 }
 
 // i modulo n for any i (the periodic layout).
@@ -170,39 +202,39 @@ __device__ __forceinline__ bool collect2(const EpiSums<2>& sh, uint64_t* red_bar
 }
 
 // R (tensor memory: lanes y = lane_base + lane, columns f) -> sR, the K-major
-// [hi | lo] operand of stage 2 (rows f, K = y), for the 16-column groups q0, q0 + dq,
-// .. of BN. The words (f, y & ~1) hold the pair of lanes y & ~1 and y | 1: for each
-// pair of columns (f, f + 1) the even lane splits and stores column f (hi and lo
-// word), the odd lane column f + 1, after one exchange of values between the two.
+// [hi | lo] operand of stage 2 (rb rows f, K = y), for the 8-column groups u0, u0 + du,
+// .. below nu (rows f from 8 nu on are left as they are: the columns of the product that
+// they belong to are not used). The words (f, y & ~1) hold the pair of lanes y & ~1 and
+// y | 1: for each pair of columns (f, f + 1) the even lane splits and stores column f (hi
+// and lo word), the odd lane column f + 1, after one exchange of values between the two.
 // acc: the accumulator's address with this warp's lane base.
-template <int BN>
-__device__ __forceinline__ void r_to_operand(uint32_t acc, uint8_t* sR, int lane_base, int q0,
-                                             int dq) {
+__device__ __forceinline__ void r_to_operand(uint32_t acc, uint8_t* sR, int rb, int lane_base,
+                                             int u0, int du, int nu) {
   const uint32_t lane = threadIdx.x & 31u;
   const uint32_t ye = ((uint32_t)lane_base + lane) & ~1u;
   const uint32_t odd = lane & 1u;
-  // sw128_offset(BN, f, k) for f = 16 q + i + odd, k = ye (hi) or 128 + ye (lo): the
-  // part that depends on (f % 8), and the 1024-byte groups of 8 rows f / 8
+  // sw128_offset(rb, f, k) for f = 8 u + i + odd, k = ye (hi) or 128 + ye (lo): the
+  // part that depends on f % 8, and the 1024-byte group u
   uint32_t off[4];
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     const uint32_t f8 = 2u * i + odd;
-    off[i] = (ye >> 6) * (uint32_t)BN * 128u + f8 * 128u + ((((ye & 63u) >> 3) ^ f8) << 4) +
+    off[i] = (ye >> 6) * (uint32_t)rb * 128u + f8 * 128u + ((((ye & 63u) >> 3) ^ f8) << 4) +
              (ye & 7u) * 2u;
   }
-  constexpr uint32_t LO = 2u * (uint32_t)BN * 128u;   // k + 128: two atoms further
+  const uint32_t LO = 2u * (uint32_t)rb * 128u;   // k + 128: two atoms further
 #pragma unroll 1
-  for (int q = q0; q < BN / 16; q += dq) {
-    float rv[16];
-    tmem_ld16x(acc + (uint32_t)(16 * q), rv);
-    uint8_t* sq = sR + (uint32_t)q * 2048u;
+  for (int u = u0; u < nu; u += du) {
+    float rv[8];
+    tmem_ld8x(acc + (uint32_t)(8 * u), rv);
+    uint8_t* sq = sR + (uint32_t)u * 1024u;
 #pragma unroll
-    for (int i = 0; i < 16; i += 2) {
+    for (int i = 0; i < 8; i += 2) {
       // the even lane receives its partner's column i, the odd lane column i + 1
       const float got = __shfl_xor_sync(0xffffffffu, odd ? rv[i] : rv[i + 1], 1);
       uint32_t h2, l2;
       split_pair(odd ? got : rv[i], odd ? rv[i + 1] : got, h2, l2);
-      uint8_t* w = sq + (uint32_t)(i >> 3) * 1024u + off[(i & 7) >> 1];
+      uint8_t* w = sq + off[i >> 1];
       *reinterpret_cast<uint32_t*>(w) = h2;
       *reinterpret_cast<uint32_t*>(w + LO) = l2;
     }
@@ -212,16 +244,16 @@ __device__ __forceinline__ void r_to_operand(uint32_t acc, uint8_t* sR, int lane
 // Q (tensor memory: lanes n = 2 r + s, columns f = 2 c + t) -> the tile's partials
 // P[r][c] of the band (see analysis_stages in tc2.cu): Re = Q[2r][2c] - Q[2r+1][2c+1],
 // Im = Q[2r][2c+1] + Q[2r+1][2c]; with sym also the conjugate rows -r (from the odd
-// lane of the pair). The tile's block is stored column-major, P[c][row] at
-// out + c nrows_out + row, so that a warp's store of one column touches two runs of
-// consecutive rows instead of 32 rows ncols apart (reduce_tiles_kernel with trows =
-// nrows_out reads this layout).
-template <int BN>
+// lane of the pair), for the 8-column groups u0, u0 + du, .. below nu. The tile's block
+// is stored column-major, P[c][row] at out + c nrows_out + row, so that a warp's store of
+// one column touches two runs of consecutive rows instead of 32 rows ncols apart
+// (reduce_tiles_kernel with trows = nrows_out reads this layout).
 __device__ __forceinline__ void q_to_partials(uint32_t acc, float2* out, const Tc2Analysis& a,
-                                              int lane_base, int q0, int dq) {
+                                              int lane_base, int u0, int du, int nu) {
   const int lane = threadIdx.x & 31;
   const int nn = lane_base + lane;
   const int r = nn >> 1, s = nn & 1;
+  if (lane_base >= 2 * a.nr) return;   // none of this warp's lanes holds a row
   // the output row of this lane, or none
   float2* row = nullptr;
   if (r < a.nr) {
@@ -233,16 +265,16 @@ __device__ __forceinline__ void q_to_partials(uint32_t acc, float2* out, const T
       row = out + (a.nr - 1 - r);
   }
 #pragma unroll 1
-  for (int q = q0; q < BN / 16; q += dq) {
-    float qv[16], pv[16];
-    tmem_ld16x(acc + (uint32_t)(16 * q), qv);
+  for (int u = u0; u < nu; u += du) {
+    float qv[8], pv[8];
+    tmem_ld8x(acc + (uint32_t)(8 * u), qv);
 #pragma unroll
-    for (int i = 0; i < 16; ++i) pv[i] = __shfl_xor_sync(0xffffffffu, qv[i], 1);
+    for (int i = 0; i < 8; ++i) pv[i] = __shfl_xor_sync(0xffffffffu, qv[i], 1);
     if (row == nullptr) continue;
-    float2* rq = row + (size_t)(8 * q) * a.nrows_out;
-    const int nc = a.ncols - 8 * q;
+    float2* rq = row + (size_t)(4 * u) * a.nrows_out;
+    const int nc = a.ncols - 4 * u;
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
+    for (int i = 0; i < 4; ++i) {
       if (i >= nc) break;
       const float o0 = qv[2 * i], o1 = qv[2 * i + 1], p0 = pv[2 * i], p1 = pv[2 * i + 1];
       rq[(size_t)i * a.nrows_out] = s == 0 ? make_float2(o0 - p1, o1 + p0)
@@ -301,7 +333,7 @@ analysis_tc3_kernel(Tc2Analysis a, int T, int B, const uint8_t* __restrict__ txI
   uint8_t* sR = smem + 2 * A2_A_BYTES + TXB;
   const uint32_t uTY = tc::smem_u32(smem), uA = tc::smem_u32(sA);
   const uint32_t uTX = uA + A2_A_BYTES, uR = tc::smem_u32(sR);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   auto bar = [&](int i) { return tc::smem_u32(&bars[i]); };
   int lo, hi;
   my_items(T * T * B, lo, hi);
@@ -446,7 +478,8 @@ analysis_tc3_kernel(Tc2Analysis a, int T, int B, const uint8_t* __restrict__ txI
     pdl_wait();
     const int lane_base = (warp & 3) * 32;
     constexpr int DQ = A3_TMW / 4;
-    const int q0 = (warp - A3_LOADW) / 4;   // first 16-column group of this warp
+    const int u0 = (warp - A3_LOADW) / 4;   // first 8-column group of this warp
+    const int nu = (2 * a.ncols + 7) / 8;
     const int count = a.nrows_out * a.ncols;
     Item prv = item_at(lo, T, B), cur = prv;   // items j - 1 and j
     for (int j = 0; j <= n; ++j) {
@@ -459,8 +492,8 @@ analysis_tc3_kernel(Tc2Analysis a, int T, int B, const uint8_t* __restrict__ txI
       if (j > 0 && !pwait(bar(4 + ((j - 1) & 1)), ((j - 1) >> 1) & 1, vfail, err, 13)) break;
       tc::fence_after();
       if (j < n) {
-        r_to_operand<BN>(tmem + (uint32_t)((j & 1) * 128) + ((uint32_t)lane_base << 16), sR,
-                         lane_base, q0, DQ);
+        r_to_operand(tmem + (uint32_t)((j & 1) * 128) + ((uint32_t)lane_base << 16), sR, BN,
+                     lane_base, u0, DQ, nu);
         fence_async_smem();
         tc::fence_before();
         __syncwarp();
@@ -470,15 +503,16 @@ analysis_tc3_kernel(Tc2Analysis a, int T, int B, const uint8_t* __restrict__ txI
         // Q of the previous item -> its partials P[r][c] (see analysis_stages in tc2.cu)
         const int jp = j - 1;
         float2* out = a.part + (((size_t)prv.z * T + prv.yt) * T + prv.xt) * count;
-        q_to_partials<BN>(tmem + 256u + (uint32_t)((jp & 1) * 128) + ((uint32_t)lane_base << 16),
-                          out, a, lane_base, q0, DQ);
+        q_to_partials(tmem + 256u + (uint32_t)((jp & 1) * 128) + ((uint32_t)lane_base << 16), out,
+                      a, lane_base, u0, DQ, nu);
         tc::fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(bar(6 + (jp & 1)));
       }
     }
-  } else if (lane == 0) {
-    // ------------------------------------------------------------ MMA thread
+  } else {
+    // ------------------------------------------------------------ MMA warp
+    const uint32_t lead = tc::elect_one();
     int pxt = -1, pyt = -1;
     uint32_t ntx = 0, nty = 0;
     int m1 = 0, m2 = 0;
@@ -492,16 +526,16 @@ analysis_tc3_kernel(Tc2Analysis a, int T, int B, const uint8_t* __restrict__ txI
         const bool newx = it.xt != pxt;
         if (newx) {
           // the TX tile in use is read by stage 1 of the previous item
-          if (j > 0 && !pwait(bar(1 + ((j - 1) & 1)), ((j - 1) >> 1) & 1, vfail, err, 14)) break;
-          bulk_tile(uTX, txImg + (size_t)it.xt * TXB, TXB, bar(8));
+          if (j > 0 && !pwait_warp(bar(1 + ((j - 1) & 1)), ((j - 1) >> 1) & 1, vfail, err, 14)) break;
+          bulk_tile(uTX, txImg + (size_t)it.xt * TXB, TXB, bar(8), lead);
           ++ntx;
           pxt = it.xt;
         }
-        if (!pwait(bar(0), j & 1, vfail, err, 15)) break;
-        if (newx && !pwait(bar(8), (ntx - 1) & 1, vfail, err, 16)) break;
+        if (!pwait_warp(bar(0), j & 1, vfail, err, 15)) break;
+        if (newx && !pwait_warp(bar(8), (ntx - 1) & 1, vfail, err, 16)) break;
         tc::fence_after();
-        s2_mma(tmem + (uint32_t)((j & 1) * 128), uA, 128, uTX, BN, 128, idesc);
-        tc::mma_commit(bar(1 + (j & 1)));
+        s2_mma(tmem + (uint32_t)((j & 1) * 128), uA, 128, uTX, BN, 128, idesc, lead);
+        tc::mma_commit(bar(1 + (j & 1)), lead);
         ++m1;
       }
       if (j > 0) {
@@ -509,17 +543,17 @@ analysis_tc3_kernel(Tc2Analysis a, int T, int B, const uint8_t* __restrict__ txI
         const int jj = j - 1;
         const bool newy = prv.yt != pyt;
         if (newy) {
-          if (jj > 0 && !pwait(bar(4 + ((jj - 1) & 1)), ((jj - 1) >> 1) & 1, vfail, err, 17)) break;
-          bulk_tile(uTY, tyImg + (size_t)prv.yt * A2_A_BYTES, A2_A_BYTES, bar(9));
+          if (jj > 0 && !pwait_warp(bar(4 + ((jj - 1) & 1)), ((jj - 1) >> 1) & 1, vfail, err, 17)) break;
+          bulk_tile(uTY, tyImg + (size_t)prv.yt * A2_A_BYTES, A2_A_BYTES, bar(9), lead);
           ++nty;
           pyt = prv.yt;
         }
-        if (!pwait(bar(3), jj & 1, vfail, err, 18)) break;
-        if (newy && !pwait(bar(9), (nty - 1) & 1, vfail, err, 19)) break;
-        if (jj >= 2 && !pwait(bar(6 + (jj & 1)), ((jj - 2) >> 1) & 1, vfail, err, 20)) break;
+        if (!pwait_warp(bar(3), jj & 1, vfail, err, 18)) break;
+        if (newy && !pwait_warp(bar(9), (nty - 1) & 1, vfail, err, 19)) break;
+        if (jj >= 2 && !pwait_warp(bar(6 + (jj & 1)), ((jj - 2) >> 1) & 1, vfail, err, 20)) break;
         tc::fence_after();
-        s2_mma(tmem + 256u + (uint32_t)((jj & 1) * 128), uTY, 128, uR, BN, 128, idesc);
-        tc::mma_commit(bar(4 + (jj & 1)));
+        s2_mma(tmem + 256u + (uint32_t)((jj & 1) * 128), uTY, 128, uR, BN, 128, idesc, lead);
+        tc::mma_commit(bar(4 + (jj & 1)), lead);
         ++m2;
         prv = item_next(prv, T, B);
       }
@@ -650,7 +684,7 @@ synth_tc3_kernel(const uint8_t* __restrict__ Aimg, const uint8_t* __restrict__ B
   const uint32_t tb = s2_tile_bytes(128, kp);
   uint8_t* smem = align1024(smem_raw);
   const uint32_t uAY = tc::smem_u32(smem);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   auto bar = [&](int i) { return tc::smem_u32(&bars[i]); };
   int lo, hi;
   my_items(T * T * B, lo, hi);
@@ -792,7 +826,8 @@ synth_tc3_kernel(const uint8_t* __restrict__ Aimg, const uint8_t* __restrict__ B
       rows(16);
       if (sums) {
         const double v[2] = {(double)s0, (double)s1};
-        epi_put<2>(red, tc::smem_u32(&red_bar[j & 3]), j & 3, v);
+        if (KIND == 0) epi_put<1>(red, tc::smem_u32(&red_bar[j & 3]), j & 3, {v[0]});
+        else epi_put<2>(red, tc::smem_u32(&red_bar[j & 3]), j & 3, v);
         // the sums of item j - 1, by one warp in turn
         if (j > 0 && lane == 0 && warp == (j - 1) % S3_EPIW &&
             !collect2(red, red_bar, j - 1, S3_EPIW, vfail, err, 27, sums_out(ip), KIND == 0 ? 1 : 2))
@@ -803,8 +838,9 @@ synth_tc3_kernel(const uint8_t* __restrict__ Aimg, const uint8_t* __restrict__ B
     // the sums of the last item
     if (sums && n > 0 && done == n && lane == 0 && warp == (n - 1) % S3_EPIW)
       collect2(red, red_bar, n - 1, S3_EPIW, vfail, err, 28, sums_out(ip), KIND == 0 ? 1 : 2);
-  } else if (warp == S3_MMAW && lane == 0) {
-    // ------------------------------------------------------------ MMA thread
+  } else if (warp == S3_MMAW) {
+    // ------------------------------------------------------------ MMA warp
+    const uint32_t lead = tc::elect_one();
     // the band operand image is written by the previous kernel of the stream
     pdl_wait();
     constexpr uint32_t idesc = tc::idesc_bf16(128, 128);
@@ -814,31 +850,31 @@ synth_tc3_kernel(const uint8_t* __restrict__ Aimg, const uint8_t* __restrict__ B
     int nb = 0, nm = 0;
     Item it = item_at(lo, T, B);
     if (n > 0) {
-      bulk_tile(uAY + tb, bt_src(it), tb, bar(0));
+      bulk_tile(uAY + tb, bt_src(it), tb, bar(0), lead);
       nb = 1;
     }
     for (int j = 0; j < n; ++j, it = item_next(it, T, B)) {
       const bool newy = it.yt != pyt;
       if (newy) {
         // the AY tile in use is read by the previous item's MMA
-        if (j > 0 && !pwait(bar(3 + ((j - 1) & 1)), ((j - 1) >> 1) & 1, vfail, err, 22)) break;
-        bulk_tile(uAY, Aimg + (size_t)it.yt * tb, tb, bar(2));
+        if (j > 0 && !pwait_warp(bar(3 + ((j - 1) & 1)), ((j - 1) >> 1) & 1, vfail, err, 22)) break;
+        bulk_tile(uAY, Aimg + (size_t)it.yt * tb, tb, bar(2), lead);
         ++nay;
         pyt = it.yt;
       }
-      if (!pwait(bar(j & 1), (j >> 1) & 1, vfail, err, 23)) break;
-      if (newy && !pwait(bar(2), (nay - 1) & 1, vfail, err, 24)) break;
-      if (j >= 2 && !pwait(bar(5 + (j & 1)), ((j - 2) >> 1) & 1, vfail, err, 25)) break;
+      if (!pwait_warp(bar(j & 1), (j >> 1) & 1, vfail, err, 23)) break;
+      if (newy && !pwait_warp(bar(2), (nay - 1) & 1, vfail, err, 24)) break;
+      if (j >= 2 && !pwait_warp(bar(5 + (j & 1)), ((j - 2) >> 1) & 1, vfail, err, 25)) break;
       tc::fence_after();
-      s2_mma_swapped(tmem + (uint32_t)((j & 1) * 128), uAY, 128, uAY + (uint32_t)(1 + (j & 1)) * tb,
-                     128, kp, idesc);
-      tc::mma_commit(bar(3 + (j & 1)));
+      s2_mma_swapped_kp(tmem + (uint32_t)((j & 1) * 128), uAY, uAY + (uint32_t)(1 + (j & 1)) * tb, kp,
+                        idesc, lead);
+      tc::mma_commit(bar(3 + (j & 1)), lead);
       ++nm;
       if (j + 1 < n) {
         // Bt[(j + 1) & 1] is read by the MMA of item j - 1
-        if (j >= 1 && !pwait(bar(3 + ((j - 1) & 1)), ((j - 1) >> 1) & 1, vfail, err, 26)) break;
+        if (j >= 1 && !pwait_warp(bar(3 + ((j - 1) & 1)), ((j - 1) >> 1) & 1, vfail, err, 26)) break;
         bulk_tile(uAY + (uint32_t)(1 + ((j + 1) & 1)) * tb, bt_src(item_next(it, T, B)), tb,
-                  bar((j + 1) & 1));
+                  bar((j + 1) & 1), lead);
         ++nb;
       }
     }
@@ -892,23 +928,34 @@ cudaError_t launch_synth_resist_tc3(cudaStream_t s, const void* Aimg, const void
 // persistent pipeline. Per item j:
 //   SMMA(j)   I^T = Ut . AYD^T into accI[j & 1] (transposed: lanes x);
 //   epi(j)    warps 0-15: resist, loss terms, dL/dI, written as the split operand sA
-//             (M = y, K = x) in region X, while TXD(j) lands behind it. sA is MN-major
-//             (mn_chunk_offset): a thread holds the 32 rows y of its column x and
-//             writes them as 16-byte chunks, with no exchange between lanes;
-//   MMA1(j)   R = sA . TXD^T into accR; once done, X takes the synthesis operands of
-//             item j + 1 (Ut, AYD) and SMMA(j + 1) is issued;
-//   R(j)      warps 0-15: R -> sR;  MMA2(j)  Q = TYD . R^T into accQ;
-//   Q(j)      warps 0-15 (after epi(j + 1)): Q -> the item's adjoint partials.
-// Shared memory: X = max(sA + TXD, Ut + AYD) | TYD 64 KiB (per yt) | sR.
+//             (M = y, K = x) over Ut. sA is MN-major (mn_chunk_offset): a thread holds
+//             rows y of its column x and writes them as 16-byte chunks, with no exchange
+//             between lanes;
+//   MMA1(j)   R = sA . TXD^T into accR; once done, Ut of item j + 1 takes sA's place and
+//             SMMA(j + 1) is issued;
+//   R(j)      warps 16-23: R -> sR;  MMA2(j)  Q = TYD . R^T into accQ;
+//   Q(j)      warps 16-23, after R(j + 1): Q -> the item's adjoint partials.
+// One set of 16 warps that did epi, R and Q in turn left half of the issue slots idle, and
+// the MMA thread spent 3400 cycles on the 15 instructions of a synthesis (see elect_one); now
+// R and Q run beside the next item's epilogue. 16 tiles of 2048^2: 216 us before, 199 us so; 12 of
+// 1266^2 127 and 102, 16 micro tiles of 1280^2 with windows 146 and 119.
+// Shared memory: sA / Ut | TXD (per xt) | TYD (per yt) | sR | AYD (per yt). TXD and sR hold the
+// rf = 2 ncols rows f rounded to 8, TYD the rn = 2 nr rows n: the products read on to BN and
+// 128 rows, into the tiles that follow, and their columns and lanes past rf and rn are not
+// used. Where this does not fit (2 ncols or 2 nr above 80), AYD and TXD share one place: AYD is
+// copied with every Ut, TXD once SMMA is done.
 // Tensor memory: accI[b] at 128 b, accR at 256, accQ at 384.
-constexpr int F3_MW = 16, F3_MMAW = 16;
-constexpr int F3_NT = (F3_MW + 1) * 32;
+constexpr int F3_EPIW = 16, F3_TMW = 8, F3_MMAW = F3_EPIW + F3_TMW;
+constexpr int F3_NT = (F3_MMAW + 1) * 32;
 
-template <int BN>
-__host__ __device__ constexpr uint32_t f3_x_bytes(uint32_t tb) {
-  return (A2_A_BYTES + s2_tile_bytes(BN, 128)) > 2 * tb ? (A2_A_BYTES + s2_tile_bytes(BN, 128))
-                                                          : 2 * tb;
+__host__ __device__ constexpr uint32_t f3_rows(int ncols) { return (uint32_t)(2 * ncols + 7) / 8 * 8; }
+// Dynamic shared memory of rf rows f, rn rows n and synthesis tiles of tb bytes: 1 KiB to align
+// and, behind the last tile, 1 KiB for rows read past rf.
+__host__ __device__ constexpr uint32_t f3_smem(uint32_t rf, uint32_t rn, uint32_t tb, bool res) {
+  const uint32_t f = rf * 512u, x = A2_A_BYTES > tb ? A2_A_BYTES : tb;
+  return x + (res ? f + tb : (f > tb ? f : tb)) + rn * 512u + f + 2048;
 }
+constexpr uint32_t F3_SMEM_MAX = 232448 - 2048;   // beside the static barriers and sums
 
 // MODE 0: no window, no penalty, no image output (the CTM evaluation); 1: windows and
 // penalty; 2: aerial / wafer outputs too. 16 micro tiles of 1280^2 with windows: 435 us when
@@ -917,41 +964,39 @@ __host__ __device__ constexpr uint32_t f3_x_bytes(uint32_t tb) {
 template <int BN, int MODE>
 __global__ void __launch_bounds__(F3_NT, 1)
 fused_tc3_kernel(const uint8_t* __restrict__ Aimg, const uint8_t* __restrict__ Bimg, int N,
-                 int kp, int T, int B, S3Resist r, Tc2Analysis a,
+                 int kp, int T, int B, S3Resist r, Tc2Analysis a, int res,
                  const uint8_t* __restrict__ txImg, const uint8_t* __restrict__ tyImg,
                  int* __restrict__ err) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
-  // 0 synthesis operands landed, 1-2 SMMA done [b], 3 sA full (math warps), 4 TXD landed,
-  // 5 MMA1 done, 6 sR full (math warps), 7 TYD landed, 8 MMA2 done, 9 accQ free
-  // (math warps), 10-11 accI[b] free (math warps)
-  __shared__ __align__(8) uint64_t bars[12];
+  // Ut, AYD, TXD, TYD landed; SMMA done [j & 1]; sA full (epilogue warps); MMA1 done; accR free
+  // (TMEM warps); sR full (TMEM warps); MMA2 done; accQ free (TMEM warps). A phase of one item
+  // completes only after every waiter has seen that of the item before.
+  enum { UT, AY, TX, TY, SM, SM1, AFULL, M1, RFREE, SFULL, M2, QFREE, NBARS };
+  __shared__ __align__(8) uint64_t bars[NBARS];
   __shared__ uint32_t tmem_slot;
   __shared__ int fail;
   __shared__ __align__(8) uint64_t red_bar[EPI_SLOTS];
   __shared__ EpiSums<2> red;
-  constexpr uint32_t TXB = s2_tile_bytes(BN, 128);
+  const uint32_t rf = f3_rows(a.ncols), rn = f3_rows(a.nr);
   const uint32_t tb = s2_tile_bytes(128, kp);
-  const uint32_t XB = f3_x_bytes<BN>(tb);
-  uint8_t* smem = align1024(smem_raw);
-  uint8_t* sA = smem;
-  uint8_t* sR = smem + XB + A2_A_BYTES;
-  const uint32_t uX = tc::smem_u32(smem);
-  const uint32_t uUt = uX, uAYD = uX + tb, uTXD = uX + A2_A_BYTES, uTYD = uX + XB;
-  const uint32_t uR = tc::smem_u32(sR);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  uint8_t* sA = align1024(smem_raw);
+  const uint32_t uA = tc::smem_u32(sA), uUt = uA;
+  const uint32_t uTXD = uA + (A2_A_BYTES > tb ? A2_A_BYTES : tb);
+  const uint32_t uTYD = uTXD + (res || rf * 512u > tb ? rf * 512u : tb), uR = uTYD + rn * 512u;
+  const uint32_t uAYD = res ? uR + rf * 512u : uTXD;
+  uint8_t* sR = sA + (uR - uA);
+  const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   auto bar = [&](int i) { return tc::smem_u32(&bars[i]); };
   int lo, hi;
   my_items(T * T * B, lo, hi);
   const int n = hi - lo;
   pdl_trigger();
   if (threadIdx.x == 0) {
-    for (int i = 0; i < 12; ++i) tc::mbar_init(bar(i), 1);
-    tc::mbar_init(bar(3), F3_MW);
-    tc::mbar_init(bar(6), F3_MW);
-    tc::mbar_init(bar(9), F3_MW);
-    tc::mbar_init(bar(10), F3_MW);
-    tc::mbar_init(bar(11), F3_MW);
-    for (int i = 0; i < EPI_SLOTS; ++i) tc::mbar_init(tc::smem_u32(&red_bar[i]), F3_MW);
+    for (int i = 0; i < NBARS; ++i)
+      tc::mbar_init(bar(i), i == AFULL ? F3_EPIW
+                            : i == RFREE || i == SFULL || i == QFREE ? F3_TMW
+                                                                     : 1);
+    for (int i = 0; i < EPI_SLOTS; ++i) tc::mbar_init(tc::smem_u32(&red_bar[i]), F3_EPIW);
     fail = 0;
     tc::fence_mbar_init();
   }
@@ -960,27 +1005,25 @@ fused_tc3_kernel(const uint8_t* __restrict__ Aimg, const uint8_t* __restrict__ B
   __syncthreads();
   tc::fence_after();
   const uint32_t tmem = tmem_slot;
+  const uint32_t tR = tmem + 256u, tQ = tmem + 384u;
   volatile int* vfail = &fail;
 
-  if (warp < F3_MW) {
-    // ------------------------------------------------------------ math warps
+  if (warp < F3_EPIW) {
+    // ------------------------------------------------------------ epilogue warps
     pdl_wait();
     const int q = warp & 3, h = warp >> 2;
     const int lane_base = 32 * q;
     const uint32_t lane_addr = (uint32_t)lane_base << 16;
     const int xl = lane_base + lane;
-    const int count = a.nrows_out * a.ncols;
-    // this thread's four 16-byte chunks of sA (rows y = 32 h + 8 c .. + 7 of column xl)
-    uint32_t aoff[4];
-#pragma unroll
-    for (int c = 0; c < 4; ++c) aoff[c] = mn_chunk_offset((uint32_t)(32 * h + 8 * c), (uint32_t)xl);
     float pre[32];
+    // the layout comes with a loss region only (MODE 1)
+    const bool lay = MODE == 1 && r.p.layout != nullptr;
     auto prefetch = [&](const Item& it) {
       const int x = it.xt * 128 + xl, yb = it.yt * 128 + 32 * h;
       const float* tp;
       size_t step = N;
       int wrap = 32;   // row of the segment from which the layout starts again
-      if (r.p.layout) {
+      if (lay) {
         const int H = r.p.layout_h, W = r.p.layout_w;
         const int gy = wrapped(__ldg(r.p.origins + 2 * it.z) + yb, H);
         tp = r.p.layout + (size_t)gy * W + wrapped(__ldg(r.p.origins + 2 * it.z + 1) + x, W);
@@ -992,7 +1035,7 @@ fused_tc3_kernel(const uint8_t* __restrict__ Aimg, const uint8_t* __restrict__ B
       if (x < N && yb + 31 < N && wrap >= 32) {
 #pragma unroll
         for (int e = 0; e < 32; ++e) pre[e] = __ldg(tp + e * step);
-      } else if (r.p.layout) {
+      } else if (lay) {
         const int H = r.p.layout_h;
 #pragma unroll
         for (int e = 0; e < 32; ++e)
@@ -1004,28 +1047,30 @@ fused_tc3_kernel(const uint8_t* __restrict__ Aimg, const uint8_t* __restrict__ B
         for (int e = 0; e < 32; ++e) pre[e] = (x < N && yb + e < N) ? __ldg(tp + e * step) : 0.f;
       }
     };
-    // the target rows of item i + 2 are fetched into L2 during item i
-    const bool pf = !r.p.layout && N % 4 == 0 && reinterpret_cast<uintptr_t>(r.p.target) % 16 == 0;
-    Item it = item_at(lo, T, B), ip = it;   // items j and j - 1
+    Item it = item_at(lo, T, B);
     if (n > 0) prefetch(it);
-    for (int j = 0; j < n; ++j, ip = it, it = item_next(it, T, B)) {
-      if (j + 2 < n) {
-        const Item i2 = item_next(item_next(it, T, B), T, B);
-        prefetch_rows(r.p.target + (size_t)i2.z * N * N, N, i2.yt * 128 + 32 * h,
-                      i2.xt * 128 + lane_base, pf);
-      }
+    for (int j = 0; j < n; ++j, it = item_next(it, T, B)) {
       const int x = it.xt * 128 + xl, yb = it.yt * 128 + 32 * h;
       const bool xin = x < N;
       const size_t base = (size_t)it.z * N * N;
-      if (!pwait(bar(1 + (j & 1)), (j >> 1) & 1, vfail, err, 31)) break;
+      const uint32_t acc = tmem + (uint32_t)((j & 1) * 128) + lane_addr + (uint32_t)(32 * h);
+      // rows 32 h + e0 .. + 15 of column xl: two 16-byte chunks of hi, two of lo
+      auto store_a = [&](const float (&d)[16], int e0) {
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+          uint4 h4, l4;
+          split_pair(d[8 * c + 0], d[8 * c + 1], h4.x, l4.x);
+          split_pair(d[8 * c + 2], d[8 * c + 3], h4.y, l4.y);
+          split_pair(d[8 * c + 4], d[8 * c + 5], h4.z, l4.z);
+          split_pair(d[8 * c + 6], d[8 * c + 7], h4.w, l4.w);
+          uint8_t* w = sA + mn_chunk_offset((uint32_t)(32 * h + e0 + 8 * c), (uint32_t)xl);
+          *reinterpret_cast<uint4*>(w) = h4;
+          *reinterpret_cast<uint4*>(w + MN_LO) = l4;
+        }
+      };
+      if (!pwait(bar(SM + (j & 1)), (j >> 1) & 1, vfail, err, 31)) break;
       tc::fence_after();
-      float d[32];
-      tc::tmem_ld32(tmem + (uint32_t)((j & 1) * 128) + lane_addr + (uint32_t)(32 * h), d);
-      tc::fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(bar(10 + (j & 1)));
-      // sA is free: the MMA thread issues SMMA(j) only after MMA1(j - 1) completed.
-      // d[e] becomes dL/dI at (yb + e, x), 0 outside the image.
+      // d[e] becomes dL/dI at (yb + e0 + e, x), 0 outside the image.
       float s0 = 0.f, s1 = 0.f;
       bool bad;
       const int ny = xin ? N - yb : 0;   // rows e < ny lie in the image
@@ -1044,28 +1089,35 @@ fused_tc3_kernel(const uint8_t* __restrict__ Aimg, const uint8_t* __restrict__ B
         const float2 one = make_float2(1.f, 1.f), pw = make_float2(r.p.pe_weight, r.p.pe_weight);
         auto pixels = [&](auto edge) {
 #pragma unroll
-          for (int e = 0; e < 32; e += 2) {
-            const float2 z = __fmul2_rn(na, __fadd2_rn(make_float2(d[e], d[e + 1]), nt));
-            const float2 den = __fadd2_rn(one, make_float2(__expf(z.x), __expf(z.y)));
-            float2 W = make_float2(__fdividef(1.f, den.x), __fdividef(1.f, den.y));
-            float2 rr = __fadd2_rn(W, make_float2(-pre[e], -pre[e + 1]));
-            if (decltype(edge)::value) {
-              // the accumulator there may hold anything
-              if (e >= ny) rr.x = W.x = 0.f;
-              if (e + 1 >= ny) rr.y = W.y = 0.f;
+          for (int e0 = 0; e0 < 32; e0 += 16) {
+            float d[16];
+            tmem_ld16x(acc + (uint32_t)e0, d);
+#pragma unroll
+            for (int e = 0; e < 16; e += 2) {
+              const float2 z = __fmul2_rn(na, __fadd2_rn(make_float2(d[e], d[e + 1]), nt));
+              const float2 den = __fadd2_rn(one, make_float2(__expf(z.x), __expf(z.y)));
+              float2 W = make_float2(__fdividef(1.f, den.x), __fdividef(1.f, den.y));
+              float2 rr = __fadd2_rn(W, make_float2(-pre[e0 + e], -pre[e0 + e + 1]));
+              if (decltype(edge)::value) {
+                // the accumulator there may hold anything
+                if (e0 + e >= ny) rr.x = W.x = 0.f;
+                if (e0 + e + 1 >= ny) rr.y = W.y = 0.f;
+              }
+              if (decltype(edge)::value && ny < 32)
+                se.x = __fadd_rn(__fadd_rn(se.x, __fmul_rn(rr.x, rr.x)), __fmul_rn(rr.y, rr.y));
+              else
+                se = __ffma2_rn(rr, rr, se);
+              const float2 g = __fmul2_rn(__fmul2_rn(__fmul2_rn(pw, rr), W),
+                                          __fadd2_rn(one, make_float2(-W.x, -W.y)));
+              chk = __ffma2_rn(g, make_float2(0.f, 0.f), chk);
+              d[e] = g.x;
+              d[e + 1] = g.y;
             }
-            if (decltype(edge)::value)
-              se.x = __fadd_rn(__fadd_rn(se.x, __fmul_rn(rr.x, rr.x)), __fmul_rn(rr.y, rr.y));
-            else
-              se = __ffma2_rn(rr, rr, se);
-            const float2 g = __fmul2_rn(__fmul2_rn(__fmul2_rn(pw, rr), W),
-                                        __fadd2_rn(one, make_float2(-W.x, -W.y)));
-            chk = __ffma2_rn(g, make_float2(0.f, 0.f), chk);
-            d[e] = g.x;
-            d[e + 1] = g.y;
+            store_a(d, e0);
           }
         };
-        if (ny >= 32) pixels(std::false_type{});
+        // one branch for the warp: the tensor-memory accesses take all its lanes
+        if (__all_sync(0xffffffffu, ny >= 32)) pixels(std::false_type{});
         else pixels(std::true_type{});
         s0 = se.x + se.y;
         bad = chk.x + chk.y != 0.f;
@@ -1084,8 +1136,13 @@ fused_tc3_kernel(const uint8_t* __restrict__ Aimg, const uint8_t* __restrict__ B
         const size_t i0 = base + (size_t)yb * N + x;
         const float* pwp = r.p.pe_window ? r.p.pe_window + i0 : nullptr;
         const float* qwp = r.p.pen_window ? r.p.pen_window + i0 : nullptr;
+        float d[16];
 #pragma unroll
         for (int e0 = 0; e0 < 32; e0 += 8) {
+          if (e0 % 16 == 0) {
+            __syncwarp();
+            tmem_ld16x(acc + (uint32_t)e0, d);
+          }
           float pw[8], qw[8];
 #pragma unroll
           for (int e = 0; e < 8; ++e) {
@@ -1100,7 +1157,7 @@ fused_tc3_kernel(const uint8_t* __restrict__ Aimg, const uint8_t* __restrict__ B
           }
 #pragma unroll
           for (int e = 0; e < 8; ++e) {
-            const float I = d[e0 + e], T = pre[e0 + e];
+            const float I = d[e0 % 16 + e], T = pre[e0 + e];
             const float W = r.sigmoid(I);
             const float rr = W - T;
             const bool in = e0 + e < ny;   // the accumulator past the edge may hold anything
@@ -1117,141 +1174,150 @@ fused_tc3_kernel(const uint8_t* __restrict__ Aimg, const uint8_t* __restrict__ B
               if (r.p.wafer) r.p.wafer[i0 + (size_t)(e0 + e) * N] = W;
             }
             chk = __fmaf_rn(g, 0.f, chk);
-            d[e0 + e] = g;
+            d[e0 % 16 + e] = g;
           }
+          if (e0 % 16) store_a(d, e0 - 8);
         }
         bad = chk != 0.f;
       }
-      // rows 8 c .. 8 c + 7 of column xl: one 16-byte chunk of hi, one of lo
-#pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        uint4 h4, l4;
-        split_pair(d[8 * c + 0], d[8 * c + 1], h4.x, l4.x);
-        split_pair(d[8 * c + 2], d[8 * c + 3], h4.y, l4.y);
-        split_pair(d[8 * c + 4], d[8 * c + 5], h4.z, l4.z);
-        split_pair(d[8 * c + 6], d[8 * c + 7], h4.w, l4.w);
-        *reinterpret_cast<uint4*>(sA + aoff[c]) = h4;
-        *reinterpret_cast<uint4*>(sA + aoff[c] + MN_LO) = l4;
-      }
-      if (bad) atomicOr(a.flag, 1);
+      tc::fence_before();
       fence_async_smem();
       __syncwarp();
-      if (lane == 0) mbar_arrive(bar(3));
+      if (lane == 0) mbar_arrive(bar(AFULL));
+      if (bad) atomicOr(a.flag, 1);
       {
         const double v[2] = {(double)s0, (double)s1};
         const uint32_t rb = tc::smem_u32(&red_bar[j & 3]);
-        epi_put<2>(red, rb, j & 3, v);
-        double t[2];
-        if (threadIdx.x == 0 &&
-            epi_take<2>(red, rb, j & 3, (j >> 2) & 1, F3_MW, vfail, err, 46, t)) {
-          const size_t bid = ((size_t)it.z * T + it.yt) * T + it.xt;
-          r.p.loss_partial[2 * bid] = t[0];
-          r.p.loss_partial[2 * bid + 1] = t[1];
-        }
+        if (MODE == 0) epi_put<1>(red, rb, j & 3, {v[0]});   // no penalty term
+        else epi_put<2>(red, rb, j & 3, v);
       }
       if (j + 1 < n) prefetch(item_next(it, T, B));
-      if (j > 0) {
-        // MMA2 of the previous item: its Q is ready and sR is free
-        if (!pwait(bar(8), (j - 1) & 1, vfail, err, 32)) break;
-        tc::fence_after();
-        q_to_partials<BN>(tmem + 384u + lane_addr,
-                          a.part + (((size_t)ip.z * T + ip.yt) * T + ip.xt) * count, a,
-                          lane_base, h, 4);
-        tc::fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(bar(9));
-      }
-      if (!pwait(bar(5), j & 1, vfail, err, 33)) break;
+    }
+  } else if (warp < F3_MMAW) {
+    // ------------------------------------------------------------ TMEM warps
+    // Two warps per lane quarter, alternate 8-column groups. Iteration j: R(j), Q(j - 1).
+    pdl_wait();
+    const int lane_base = (warp & 3) * 32;
+    const uint32_t lane_addr = (uint32_t)lane_base << 16;
+    const int u0 = (warp - F3_EPIW) / 4;
+    const int count = a.nrows_out * a.ncols;
+    const int nu = (int)rf / 8;   // 8-column groups of the rows f
+    Item it = item_at(lo, T, B), ip = it;
+    for (int j = 0; j <= n; ++j, ip = it, it = item_next(it, T, B)) {
+      if (j < n && !pwait(bar(M1), j & 1, vfail, err, 33)) break;
+      // MMA2(j - 1) has read sR and written Q(j - 1)
+      if (j > 0 && !pwait(bar(M2), (j - 1) & 1, vfail, err, 32)) break;
       tc::fence_after();
-      r_to_operand<BN>(tmem + 256u + lane_addr, sR, lane_base, h, 4);
-      fence_async_smem();
-      tc::fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(bar(6));
-      if (j + 1 == n) {
-        if (!pwait(bar(8), j & 1, vfail, err, 34)) break;
-        tc::fence_after();
-        q_to_partials<BN>(tmem + 384u + lane_addr,
-                          a.part + (((size_t)it.z * T + it.yt) * T + it.xt) * count, a,
-                          lane_base, h, 4);
+      if (j < n) {
+        r_to_operand(tR + lane_addr, sR, (int)rf, lane_base, u0, F3_TMW / 4, nu);
+        fence_async_smem();
         tc::fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(bar(9));
+        // The loss sums of item j, by a warp without a share of Q, before it frees accR: their
+        // slot is written again in item j + 4, and SMMA(j + 2) already follows MMA1(j + 1).
+        if (warp == F3_MMAW - 1 && lane == 0) {
+          double t[2];
+          if (epi_take<2>(red, tc::smem_u32(&red_bar[j & 3]), j & 3, (j >> 2) & 1, F3_EPIW, vfail,
+                          err, 46, t)) {
+            const size_t bid = ((size_t)it.z * T + it.yt) * T + it.xt;
+            r.p.loss_partial[2 * bid] = t[0];
+            r.p.loss_partial[2 * bid + 1] = t[1];
+          }
+        }
+        if (lane == 0) {
+          mbar_arrive(bar(RFREE));
+          mbar_arrive(bar(SFULL));
+        }
+        __syncwarp();
+      }
+      if (j > 0) {
+        q_to_partials(tQ + lane_addr,
+                      a.part + (((size_t)ip.z * T + ip.yt) * T + ip.xt) * count, a, lane_base, u0,
+                      F3_TMW / 4, nu);
+        tc::fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bar(QFREE));
       }
     }
-  } else if (warp == F3_MMAW && lane == 0) {
-    // ------------------------------------------------------------ MMA thread
+  } else if (warp == F3_MMAW) {
+    // ------------------------------------------------------------ MMA warp
+    const uint32_t lead = tc::elect_one();
     // the band operand image is written by the previous kernel of the stream
     pdl_wait();
     constexpr uint32_t idI = tc::idesc_bf16(128, 128), idA = tc::idesc_bf16(128, BN);
-    auto load_ops = [&](const Item& it) {
-      tc::mbar_expect_tx(bar(0), 2 * tb);
-      bulk_chunks(uUt, Bimg + ((size_t)it.z * T + it.xt) * tb, tb, bar(0));
-      bulk_chunks(uAYD, Aimg + (size_t)it.yt * tb, tb, bar(0));
-    };
-    int pyt = -1;
-    uint32_t nty = 0;
-    int nops = 0, ntx = 0;
-    uint32_t last_bar = 0, last_par = 0;
-    bool any = false;
-    auto commit = [&](int b, uint32_t par) {
-      tc::mma_commit(bar(b));
+    constexpr uint32_t TXB = s2_tile_bytes(BN, 128);
+    // copies of each operand so far, the tiles they hold and the last commit
+    uint32_t nut = 0, nay = 0, ntx = 0, nty = 0, last_bar = 0, last_par = 0;
+    int yay = -1, xtx = -1, yty = -1;
+    auto commit = [&](int b, int par) {
+      tc::mma_commit(bar(b), lead);
       last_bar = bar(b);
-      last_par = par;
-      any = true;
+      last_par = (uint32_t)par & 1u;
     };
-    Item it = item_at(lo, T, B);
-    if (n > 0) {
-      load_ops(it);
-      nops = 1;
-    }
-    for (int j = 0; j < n; ++j, it = item_next(it, T, B)) {
-      if (j == 0) {
-        if (!pwait(bar(0), 0, vfail, err, 35)) break;
+    // the operands of an item's synthesis, whose places the caller knows to be free
+    auto load_ops = [&](const Item& it) {
+      bulk_tile(uUt, Bimg + ((size_t)it.z * T + it.xt) * tb, tb, bar(UT), lead);
+      ++nut;
+      if (!res || it.yt != yay) {
+        bulk_tile(uAYD, Aimg + (size_t)it.yt * tb, tb, bar(AY), lead);
+        ++nay;
+        yay = it.yt;
+      }
+    };
+    Item it = item_at(lo, T, B), ip = it;   // items j and j - 1
+    if (n > 0) load_ops(it);
+    // Step j: SMMA(j), MMA2(j - 1), MMA1(j), then the copies for SMMA(j + 1).
+    for (int j = 0; j <= n; ++j, ip = it, it = item_next(it, T, B)) {
+      if (j < n) {
+        if (!pwait_warp(bar(UT), j & 1, vfail, err, 35)) break;
+        if (!pwait_warp(bar(AY), (nay - 1) & 1, vfail, err, 36)) break;
         tc::fence_after();
-        s2_mma_swapped(tmem, uAYD, 128, uUt, 128, kp, idI);
-        commit(1, 0);
+        // accI[j & 1] was read by epi(j - 2), before MMA1(j - 1) could start
+        s2_mma_swapped_kp(tmem + (uint32_t)((j & 1) * 128), uAYD, uUt, kp, idI, lead);
+        commit(SM + (j & 1), j >> 1);
+        if (!res || it.xt != xtx) {
+          // MMA1(j - 1) has read the TXD tile in use; shared, AYD must have been read too
+          if (!res && !pwait_warp(bar(SM + (j & 1)), (j >> 1) & 1, vfail, err, 37)) break;
+          bulk_tile_rows(uTXD, txImg + (size_t)it.xt * TXB, BN, (int)rf, bar(TX), lead);
+          ++ntx;
+          xtx = it.xt;
+        }
       }
-      // synthesis of item j done: X's operands are dead, TXD(j) goes behind sA
-      if (!pwait(bar(1 + (j & 1)), (j >> 1) & 1, vfail, err, 36)) break;
-      bulk_tile(uTXD, txImg + (size_t)it.xt * TXB, TXB, bar(4));
-      ++ntx;
-      const bool newy = it.yt != pyt;
-      if (newy) {
-        if (j > 0 && !pwait(bar(8), (j - 1) & 1, vfail, err, 37)) break;
-        bulk_tile(uTYD, tyImg + (size_t)it.yt * A2_A_BYTES, A2_A_BYTES, bar(7));
-        ++nty;
-        pyt = it.yt;
-      }
-      if (!pwait(bar(3), j & 1, vfail, err, 38)) break;
-      if (!pwait(bar(4), j & 1, vfail, err, 39)) break;
-      tc::fence_after();
-      s2_mma_amn(tmem + 256u, uX, uTXD, BN, 128, idA | IDESC_A_MN);
-      commit(5, j & 1);
-      if (!pwait(bar(5), j & 1, vfail, err, 40)) break;
-      if (j + 1 < n) {
-        // X is free: the next item's synthesis operands, then its SMMA (accI[(j+1)&1]
-        // was read by the epilogue of item j - 1)
-        load_ops(item_next(it, T, B));
-        ++nops;
-        if (!pwait(bar(0), (j + 1) & 1, vfail, err, 41)) break;
-        if (j >= 1 && !pwait(bar(10 + ((j + 1) & 1)), ((j - 1) >> 1) & 1, vfail, err, 42)) break;
+      if (j > 0) {
+        const int i = j - 1;   // MMA2(i)
+        if (ip.yt != yty) {
+          if (i > 0 && !pwait_warp(bar(M2), (i - 1) & 1, vfail, err, 38)) break;
+          bulk_tile_rows(uTYD, tyImg + (size_t)ip.yt * A2_A_BYTES, 128, (int)rn, bar(TY), lead);
+          ++nty;
+          yty = ip.yt;
+        }
+        if (!pwait_warp(bar(TY), (nty - 1) & 1, vfail, err, 39)) break;
+        if (!pwait_warp(bar(SFULL), i & 1, vfail, err, 40)) break;
+        if (i > 0 && !pwait_warp(bar(QFREE), (i - 1) & 1, vfail, err, 41)) break;
         tc::fence_after();
-        s2_mma_swapped(tmem + (uint32_t)(((j + 1) & 1) * 128), uAYD, 128, uUt, 128, kp, idI);
-        commit(1 + ((j + 1) & 1), ((j + 1) >> 1) & 1);
+        s2_mma(tQ, uTYD, (int)rn, uR, (int)rf, 128, idA, lead);
+        commit(M2, i);
       }
-      if (!pwait(bar(6), j & 1, vfail, err, 43)) break;
-      if (newy && !pwait(bar(7), (nty - 1) & 1, vfail, err, 44)) break;
-      if (j >= 1 && !pwait(bar(9), (j - 1) & 1, vfail, err, 45)) break;
-      tc::fence_after();
-      s2_mma(tmem + 384u, uTYD, 128, uR, BN, 128, idA);
-      commit(8, j & 1);
+      if (j < n) {
+        if (!pwait_warp(bar(TX), (ntx - 1) & 1, vfail, err, 42)) break;
+        if (!pwait_warp(bar(AFULL), j & 1, vfail, err, 43)) break;
+        if (j > 0 && !pwait_warp(bar(RFREE), (j - 1) & 1, vfail, err, 44)) break;
+        tc::fence_after();
+        s2_mma_amn(tR, uA, uTXD, (int)rf, idA | IDESC_A_MN, lead);
+        commit(M1, j);
+        if (j + 1 < n) {
+          if (!pwait_warp(bar(M1), j & 1, vfail, err, 45)) break;
+          load_ops(item_next(it, T, B));
+        }
+      }
     }
     if (*vfail) {
-      if (nops) tc::mbar_wait(bar(0), (nops - 1) & 1);
-      if (ntx) tc::mbar_wait(bar(4), (ntx - 1) & 1);
-      if (nty) tc::mbar_wait(bar(7), (nty - 1) & 1);
-      if (any) tc::mbar_wait(last_bar, last_par);
+      // nothing of this CTA may still be in flight when it exits
+      if (nut) tc::mbar_wait(bar(UT), (nut - 1) & 1);
+      if (nay) tc::mbar_wait(bar(AY), (nay - 1) & 1);
+      if (ntx) tc::mbar_wait(bar(TX), (ntx - 1) & 1);
+      if (nty) tc::mbar_wait(bar(TY), (nty - 1) & 1);
+      if (last_bar) tc::mbar_wait(last_bar, last_par);
     }
   }
   tc::fence_before();
@@ -1263,9 +1329,10 @@ template <int BN, int MODE>
 static cudaError_t fused_tc3_m(cudaStream_t s, const void* Aimg, const void* Bimg, int N, int kp,
                                const ResistEpilogue& e, const Tc2Analysis& a, const void* tx,
                                const void* ty, int* err, int* nblocks, int batch) {
-  const uint32_t tb = s2_tile_bytes(128, kp);
-  const size_t smem = (size_t)f3_x_bytes<BN>(tb) + A2_A_BYTES + s2_tile_bytes(BN, 128) + 1024;
-  if (smem > 232448 - 512) return cudaErrorInvalidValue;
+  const uint32_t tb = s2_tile_bytes(128, kp), rf = f3_rows(a.ncols), rn = f3_rows(a.nr);
+  const bool res = f3_smem(rf, rn, tb, true) <= F3_SMEM_MAX;
+  const size_t smem = f3_smem(rf, rn, tb, res);
+  if (smem > F3_SMEM_MAX) return cudaErrorInvalidValue;
   cudaError_t r = cudaFuncSetAttribute(fused_tc3_kernel<BN, MODE>,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (r != cudaSuccess) return r;
@@ -1275,7 +1342,7 @@ static cudaError_t fused_tc3_m(cudaStream_t s, const void* Aimg, const void* Bim
   *nblocks = T * T;
   return launch_pdl(fused_tc3_kernel<BN, MODE>, dim3(grid), dim3(F3_NT), smem, s,
                     static_cast<const uint8_t*>(Aimg), static_cast<const uint8_t*>(Bimg), N, kp, T,
-                    batch, S3Resist{e}, a, static_cast<const uint8_t*>(tx),
+                    batch, S3Resist{e}, a, (int)res, static_cast<const uint8_t*>(tx),
                     static_cast<const uint8_t*>(ty), err);
 }
 template <int BN>
@@ -1284,6 +1351,7 @@ static cudaError_t fused_tc3_t(cudaStream_t s, const void* Aimg, const void* Bim
                                const void* ty, int* err, int* nblocks, int batch) {
   const bool out = e.aerial || e.wafer;
   const bool plain = S3Resist{e}.plain() && !e.region;
+  if (e.layout && (out || plain)) return cudaErrorInvalidValue;
   return out ? fused_tc3_m<BN, 2>(s, Aimg, Bimg, N, kp, e, a, tx, ty, err, nblocks, batch)
          : plain ? fused_tc3_m<BN, 0>(s, Aimg, Bimg, N, kp, e, a, tx, ty, err, nblocks, batch)
                  : fused_tc3_m<BN, 1>(s, Aimg, Bimg, N, kp, e, a, tx, ty, err, nblocks, batch);
@@ -1291,11 +1359,7 @@ static cudaError_t fused_tc3_t(cudaStream_t s, const void* Aimg, const void* Bim
 
 bool tc3_fused_supported(int kp, int ncols, int nr) {
   if (!tc3_analysis_supported(ncols, nr) || !tc3_synth_supported(kp)) return false;
-  const uint32_t tb = s2_tile_bytes(128, kp);
-  const uint32_t bn = (uint32_t)tc2_analysis_rows(ncols);
-  const uint32_t txb = s2_tile_bytes((int)bn, 128);
-  const uint32_t xb = A2_A_BYTES + txb > 2 * tb ? A2_A_BYTES + txb : 2 * tb;
-  return (size_t)xb + A2_A_BYTES + txb + 1024 <= 232448 - 512;
+  return f3_smem(f3_rows(ncols), f3_rows(nr), s2_tile_bytes(128, kp), false) <= F3_SMEM_MAX;
 }
 
 cudaError_t launch_synth_resist_analysis_tc3(cudaStream_t s, const void* Aimg, const void* Bimg,

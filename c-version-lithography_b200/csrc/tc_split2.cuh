@@ -28,15 +28,14 @@ __device__ __forceinline__ uint64_t s2_desc(uint32_t base, int RB, int k) {
 // The three split-BF16 sections of D[M][N] = A[M][K] . B[N][K]^T (K % 16 == 0):
 // 3 K / 16 tcgen05.mma instructions, issued by one thread.
 __device__ __forceinline__ void s2_mma(uint32_t tmem, uint32_t sa, int ra, uint32_t sb, int rb,
-                                       int K, uint32_t idesc) {
+                                       int K, uint32_t idesc, uint32_t lead = 1) {
   const int aoff[3] = {0, 0, K}, boff[3] = {0, K, 0};
-  bool first = true;
+#pragma unroll
   for (int s = 0; s < 3; ++s)
-    for (int k = 0; k < K; k += 16) {
+#pragma unroll
+    for (int k = 0; k < K; k += 16)
       tc::mma_bf16(tmem, s2_desc(sa, ra, aoff[s] + k), s2_desc(sb, rb, boff[s] + k), idesc,
-                   first ? 0u : 1u);
-      first = false;
-    }
+                   s + k > 0, lead);
 }
 
 __device__ __forceinline__ void split_bf16(float v, __nv_bfloat16& hi, __nv_bfloat16& lo) {
@@ -57,16 +56,16 @@ __device__ __forceinline__ void split_pair(float a, float b, uint32_t& hi2, uint
 // tiles of D^T = A . B^T, D[M][N] = Bt[M][K] . At[N][K]^T with M from the tile sb and N
 // from sa. Every element sums the same products in the same order as s2_mma on
 // (sa, sb): a_hi b_hi, then a_hi b_lo, then a_lo b_hi.
+template <int K>
 __device__ __forceinline__ void s2_mma_swapped(uint32_t tmem, uint32_t sa, int ra, uint32_t sb,
-                                               int rb, int K, uint32_t idesc) {
-  const int aoff[3] = {0, 0, K}, boff[3] = {0, K, 0};
-  bool first = true;
+                                               int rb, uint32_t idesc, uint32_t lead) {
+  constexpr int aoff[3] = {0, 0, K}, boff[3] = {0, K, 0};
+#pragma unroll
   for (int s = 0; s < 3; ++s)
-    for (int k = 0; k < K; k += 16) {
+#pragma unroll
+    for (int k = 0; k < K; k += 16)
       tc::mma_bf16(tmem, s2_desc(sb, rb, boff[s] + k), s2_desc(sa, ra, aoff[s] + k), idesc,
-                   first ? 0u : 1u);
-      first = false;
-    }
+                   s + k > 0, lead);
 }
 
 // MN-major split tile of a 128 (M) x 128 (K) block, 128-byte swizzle: for each k the
@@ -98,20 +97,30 @@ constexpr uint32_t IDESC_A_MN = 1u << 15;
 // s2_mma with A (M = 128 rows, K = 128) in the MN-major split layout at sa (hi) and
 // sa + MN_LO (lo): the same three sections and K steps in the same order. idesc must
 // carry IDESC_A_MN.
-__device__ __forceinline__ void s2_mma_amn(uint32_t tmem, uint32_t sa, uint32_t sb, int rb, int K,
-                                           uint32_t idesc) {
-  const uint32_t aoff[3] = {0u, 0u, MN_LO};
-  const int boff[3] = {0, K, 0};
-  bool first = true;
+__device__ __forceinline__ void s2_mma_amn(uint32_t tmem, uint32_t sa, uint32_t sb, int rb,
+                                           uint32_t idesc, uint32_t lead) {
+  constexpr uint32_t aoff[3] = {0u, 0u, MN_LO};
+  constexpr int boff[3] = {0, 128, 0};
+#pragma unroll
   for (int s = 0; s < 3; ++s)
-    for (int k = 0; k < K; k += 16) {
+#pragma unroll
+    for (int k = 0; k < 128; k += 16)
       tc::mma_bf16(tmem, desc_mn_sw128(sa + aoff[s] + (uint32_t)k * 256u),
-                   s2_desc(sb, rb, boff[s] + k), idesc, first ? 0u : 1u);
-      first = false;
-    }
+                   s2_desc(sb, rb, boff[s] + k), idesc, s + k > 0, lead);
 }
 
-// 16 consecutive FP32 columns of this thread's TMEM lane.
+// 8 and 16 consecutive FP32 columns of this thread's TMEM lane.
+__device__ __forceinline__ void tmem_ld8x(uint32_t taddr, float (&v)[8]) {
+  uint32_t r[8];
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
+        "=r"(r[7])
+      : "r"(taddr));
+  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+  for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(r[i]);
+}
 __device__ __forceinline__ void tmem_ld16x(uint32_t taddr, float (&v)[16]) {
   uint32_t r[16];
   asm volatile(
@@ -129,19 +138,28 @@ __device__ __forceinline__ void tmem_ld16x(uint32_t taddr, float (&v)[16]) {
 // Bulk copy of `bytes` (a multiple of 16) in pieces of at most 16 KiB onto mbarrier
 // `bar`, without announcing the bytes (bulk_tile announces them).
 __device__ __forceinline__ void bulk_chunks(uint32_t dst, const uint8_t* src, uint32_t bytes,
-                                            uint32_t bar) {
+                                            uint32_t bar, uint32_t lead = 1) {
   for (uint32_t q = 0; q < bytes; q += 16384) {
     const uint32_t n = bytes - q < 16384u ? bytes - q : 16384u;
-    tc::bulk_g2s(dst + q, src + q, n, bar);
+    tc::bulk_g2s(dst + q, src + q, n, bar, lead);
   }
 }
 __device__ __forceinline__ void bulk_tile(uint32_t dst, const uint8_t* src, uint32_t bytes,
-                                          uint32_t bar) {
-  tc::mbar_expect_tx(bar, bytes);
-  bulk_chunks(dst, src, bytes, bar);
+                                          uint32_t bar, uint32_t lead = 1) {
+  tc::mbar_expect_tx(bar, bytes, lead);
+  bulk_chunks(dst, src, bytes, bar, lead);
 }
 
 constexpr uint32_t A2_A_BYTES = s2_tile_bytes(128, 128);   // 64 KiB: a 128 x 128 image tile
+
+// The first rb rows of a split tile of rows rows and K = 128 as a tile of rb rows.
+__device__ __forceinline__ void bulk_tile_rows(uint32_t dst, const uint8_t* src, int rows, int rb,
+                                               uint32_t bar, uint32_t lead) {
+  const uint32_t atom = (uint32_t)rb * 128u;
+  tc::mbar_expect_tx(bar, s2_atoms(128) * atom, lead);
+  for (uint32_t q = 0; q < s2_atoms(128); ++q)
+    tc::bulk_g2s(dst + q * atom, src + q * (uint32_t)rows * 128u, atom, bar, lead);
+}
 
 // Arguments of a tile analysis (tc2.cu, tc3.cu): for every 128 x 128 tile of the image
 // in (mode 1: theta, analysed as (1 + cos theta) / 2 and optionally stored to mask_out),
@@ -158,6 +176,6 @@ struct Tc2Analysis {
 };
 
 // Rows of the tile-analysis operand TX for ncols complex columns (2 ncols rounded to 16).
-int tc2_analysis_rows(int ncols);
+int tc2_analysis_rows(int ncols);   // and of TY for ncols band rows
 
 }  // namespace litho_b200
