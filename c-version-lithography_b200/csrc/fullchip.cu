@@ -244,21 +244,20 @@ __device__ __forceinline__ float linear_strength(int dir, int y, int x, int rows
   }
 }
 
-// Relation slot j of every tile (tile blockIdx.y; its j-th neighbour in the
-// reference's order), spread over gridDim.x CTAs per tile. grad holds a copy of raw
-// before slot 0 and leaves the last slot as raw (fused on guards) + cept_weight *
-// cept_grad. A relation's guard strip (outside the Core) and, two-sided, its
-// overlap strip (inside the Core) are disjoint, so one launch covers both; the
-// overlap strips of different relations share Core corners, so the slots run as
-// separate launches in the reference's order. part[(tile * max_rel + j) * gridDim.x +
-// block] = this block's sum of (A guard mask - B core mask)^2.
+// Guard strip of relation slot blockIdx.z of tile blockIdx.y (its j-th neighbour in the
+// reference's order), spread over gridDim.x CTAs. grad holds a copy of raw before and leaves as
+// raw (fused on guards) + cept_weight * cept_grad. A guard strip lies in that neighbour's
+// Core, so the strips of a tile's relations are disjoint and one launch takes them all: 16
+// tiles of 1280^2 take 18 us, a launch per slot took 44 us in all, each bound by the latency of a
+// few loads. part[(tile * max_rel + j) * gridDim.x + block] = this block's sum of (A guard
+// mask - B core mask)^2.
 __global__ void __launch_bounds__(EX_NT)
-exchange_rel_kernel(const float* __restrict__ masks, const float* __restrict__ raw, int ts,
-                    const int* __restrict__ nrel, const int* __restrict__ rel, int max_rel, int j,
-                    litho_exchange_options o, float* __restrict__ grad,
-                    double* __restrict__ part) {
+exchange_guard_kernel(const float* __restrict__ masks, const float* __restrict__ raw, int ts,
+                      const int* __restrict__ nrel, const int* __restrict__ rel, int max_rel,
+                      litho_exchange_options o, float* __restrict__ grad,
+                      double* __restrict__ part) {
   __shared__ double sh[EX_NT / 32];
-  const int t = blockIdx.y, nch = gridDim.x;
+  const int t = blockIdx.y, nch = gridDim.x, j = blockIdx.z;
   double* out = part + ((size_t)t * max_rel + j) * nch + blockIdx.x;
   if (j >= nrel[t]) {
     if (threadIdx.x == 0) *out = 0.0;
@@ -295,30 +294,44 @@ exchange_rel_kernel(const float* __restrict__ masks, const float* __restrict__ r
     }
     gA[ia] = g;
   }
-  if (o.enable_cept && !o.cept_guard_only) {
-    // The neighbour's guard over this tile's Core edge drives the Core side too.
-    const int oy0 = R[10], oy1 = R[11], ox0 = R[12], ox1 = R[13];   // my overlap (local A)
-    const int ny0 = R[14], nx0 = R[16];                              // neighbour guard (local B)
-    const int orows = oy1 - oy0, ocols = ox1 - ox0;
-    for (int i = blockIdx.x * EX_NT + threadIdx.x; i < orows * ocols; i += nch * EX_NT) {
-      const int y = i / ocols, x = i % ocols;
-      const size_t ia = (size_t)(oy0 + y) * ts + ox0 + x;
-      const size_t ib = (size_t)(ny0 + y) * ts + nx0 + x;
-      gA[ia] += (float)o.cept_weight * 2.f * (mA[ia] - mB[ib]);
-    }
-  }
   const double total = block_sum<EX_NT>(acc, sh);
   if (threadIdx.x == 0) *out = total;
 }
 
-// cept_loss[t] = the tile's partial sums in a fixed order.
-__global__ void exchange_sum_kernel(const double* __restrict__ part, int per_tile, int ntiles,
+// Two-sided CEPT: the neighbour's guard over this tile's Core edge drives the Core side too.
+// The overlap strips of different relations share Core corners, so the slots j run as separate
+// launches in the reference's order.
+__global__ void __launch_bounds__(EX_NT)
+exchange_overlap_kernel(const float* __restrict__ masks, int ts, const int* __restrict__ nrel,
+                        const int* __restrict__ rel, int max_rel, int j, float cept_weight,
+                        float* __restrict__ grad) {
+  const int t = blockIdx.y;
+  if (j >= nrel[t]) return;
+  const size_t tt = (size_t)ts * ts;
+  const int* R = rel + ((size_t)t * max_rel + j) * REL_INTS;
+  const float* mA = masks + t * tt;
+  const float* mB = masks + (size_t)R[0] * tt;
+  float* gA = grad + t * tt;
+  const int oy0 = R[10], oy1 = R[11], ox0 = R[12], ox1 = R[13];   // my overlap (local A)
+  const int ny0 = R[14], nx0 = R[16];                              // neighbour guard (local B)
+  const int rows = oy1 - oy0, cols = ox1 - ox0;
+  for (int i = blockIdx.x * EX_NT + threadIdx.x; i < rows * cols; i += gridDim.x * EX_NT) {
+    const int y = i / cols, x = i % cols;
+    const size_t ia = (size_t)(oy0 + y) * ts + ox0 + x;
+    const size_t ib = (size_t)(ny0 + y) * ts + nx0 + x;
+    gA[ia] += cept_weight * 2.f * (mA[ia] - mB[ib]);
+  }
+}
+
+// cept_loss[t] = the tile's partial sums, a warp per tile in a fixed order.
+__global__ void exchange_sum_kernel(const double* __restrict__ part, int per_tile,
                                     double* __restrict__ cept_loss) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= ntiles) return;
+  const int t = blockIdx.x;
   double s = 0.0;
-  for (int k = 0; k < per_tile; ++k) s += part[(size_t)t * per_tile + k];
-  cept_loss[t] = s;
+  for (int k = threadIdx.x; k < per_tile; k += 32) s += part[(size_t)t * per_tile + k];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  if (threadIdx.x == 0) cept_loss[t] = s;
 }
 
 int exchange_chunks(int ntiles) {
@@ -332,13 +345,16 @@ cudaError_t launch_exchange(cudaStream_t s, const float* masks, const float* raw
                             double* part) {
   if (ntiles < 1 || ntiles > 65535) return cudaErrorInvalidValue;
   const int nch = exchange_chunks(ntiles);
-  for (int j = 0; j < max_rel; ++j) {
-    exchange_rel_kernel<<<dim3(nch, ntiles), EX_NT, 0, s>>>(masks, raw, ts, nrel, rel, max_rel, j,
-                                                           o, grad, part);
-    const cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
+  exchange_guard_kernel<<<dim3(nch, ntiles, max_rel), EX_NT, 0, s>>>(masks, raw, ts, nrel, rel,
+                                                                     max_rel, o, grad, part);
+  cudaError_t e = cudaGetLastError();
+  for (int j = 0; j < max_rel && o.enable_cept && !o.cept_guard_only && e == cudaSuccess; ++j) {
+    exchange_overlap_kernel<<<dim3(nch, ntiles), EX_NT, 0, s>>>(masks, ts, nrel, rel, max_rel, j,
+                                                                (float)o.cept_weight, grad);
+    e = cudaGetLastError();
   }
-  exchange_sum_kernel<<<(ntiles + 127) / 128, 128, 0, s>>>(part, max_rel * nch, ntiles, cept_loss);
+  if (e != cudaSuccess) return e;
+  exchange_sum_kernel<<<ntiles, 32, 0, s>>>(part, max_rel * nch, cept_loss);
   return cudaGetLastError();
 }
 
