@@ -1133,50 +1133,95 @@ fused_tc3_kernel(const uint8_t* __restrict__ Aimg, const uint8_t* __restrict__ B
           ry1 = x >= x0 && x < x1 ? __ldg(R + 1) - yb : ry0;
         }
         const bool pen_on = r.p.penalty != 0.f || r.p.loss_penalty_term;
-        const size_t i0 = base + (size_t)yb * N + x;
-        const float* pwp = r.p.pe_window ? r.p.pe_window + i0 : nullptr;
-        const float* qwp = r.p.pen_window ? r.p.pen_window + i0 : nullptr;
-        float d[16];
+        if (MODE == 1 && r.p.region && __all_sync(0xffffffffu, ny >= 32)) {
+          // The same arithmetic on pixel pairs where the windows come from the loss region and
+          // no row is past the image: a window is 0 or 1, and 0 adds nothing to a sum. 16 micro
+          // tiles of 1280^2: 120 us with the scalar form for them all, 100 us so.
+          const int lo = max(ry0, 0), hi = min(ry1, 32);
+          const uint32_t rm = hi > lo ? (0xffffffffu >> (32 - (hi - lo))) << lo : 0u;
+          const float2 na = make_float2(-r.p.alpha, -r.p.alpha), nt = make_float2(-r.p.thr, -r.p.thr);
+          const float2 one = make_float2(1.f, 1.f), pwt = make_float2(r.p.pe_weight, r.p.pe_weight);
+          const float2 pen = make_float2(r.p.penalty, r.p.penalty);
+          const float2 npt = make_float2(-r.p.pen_thr, -r.p.pen_thr);
+          float2 ck = make_float2(0.f, 0.f);
 #pragma unroll
-        for (int e0 = 0; e0 < 32; e0 += 8) {
-          if (e0 % 16 == 0) {
+          for (int e0 = 0; e0 < 32; e0 += 16) {
+            float d[16];
             __syncwarp();
             tmem_ld16x(acc + (uint32_t)e0, d);
-          }
-          float pw[8], qw[8];
 #pragma unroll
-          for (int e = 0; e < 8; ++e) {
-            if (r.p.region) {
-              const bool in = e0 + e >= ry0 && e0 + e < ry1;
-              pw[e] = in && (!r.p.region_main || pre[e0 + e] > 0.5f) ? 1.f : 0.f;
-              qw[e] = in ? 1.f : 0.f;   // used where T < 0.5
-            } else {
-              pw[e] = pwp && e0 + e < ny ? __ldg(pwp + (e0 + e) * N) : 1.f;
-              qw[e] = qwp && e0 + e < ny ? __ldg(qwp + (e0 + e) * N) : pw[e];
+            for (int e = 0; e < 16; e += 2) {
+              const float2 z = __fmul2_rn(na, __fadd2_rn(make_float2(d[e], d[e + 1]), nt));
+              const float2 den = __fadd2_rn(one, make_float2(__expf(z.x), __expf(z.y)));
+              const float2 W = make_float2(__fdividef(1.f, den.x), __fdividef(1.f, den.y));
+              const float2 Tv = make_float2(pre[e0 + e], pre[e0 + e + 1]);
+              const float2 rr = __fadd2_rn(W, make_float2(-Tv.x, -Tv.y));
+              const bool inx = rm >> (e0 + e) & 1u, iny = rm >> (e0 + e + 1) & 1u;
+              const float2 pw = make_float2(inx && (!r.p.region_main || Tv.x > 0.5f) ? 1.f : 0.f,
+                                            iny && (!r.p.region_main || Tv.y > 0.5f) ? 1.f : 0.f);
+              const float2 qw = make_float2(inx && pen_on && Tv.x < 0.5f ? 1.f : 0.f,
+                                            iny && pen_on && Tv.y < 0.5f ? 1.f : 0.f);
+              const float2 ep = __fadd2_rn(W, npt);
+              const float2 ex = make_float2(fmaxf(ep.x, 0.f), fmaxf(ep.y, 0.f));
+              const float2 r2 = __fmul2_rn(rr, rr), x2 = __fmul2_rn(ex, ex);
+              s0 = __fmaf_rn(r2.y, pw.y, __fmaf_rn(r2.x, pw.x, s0));
+              s1 = __fmaf_rn(x2.y, qw.y, __fmaf_rn(x2.x, qw.x, s1));
+              const float2 sum =
+                  __ffma2_rn(__fmul2_rn(pen, ex), qw, __fmul2_rn(__fmul2_rn(pwt, rr), pw));
+              const float2 g = __fmul2_rn(__fmul2_rn(sum, W), __fadd2_rn(one, make_float2(-W.x, -W.y)));
+              ck = __ffma2_rn(g, make_float2(0.f, 0.f), ck);
+              d[e] = g.x;
+              d[e + 1] = g.y;
             }
+            store_a(d, e0);
           }
+          chk = ck.x + ck.y;
+        } else {
+          const size_t i0 = base + (size_t)yb * N + x;
+          const float* pwp = r.p.pe_window ? r.p.pe_window + i0 : nullptr;
+          const float* qwp = r.p.pen_window ? r.p.pen_window + i0 : nullptr;
+          float d[16];
 #pragma unroll
-          for (int e = 0; e < 8; ++e) {
-            const float I = d[e0 % 16 + e], T = pre[e0 + e];
-            const float W = r.sigmoid(I);
-            const float rr = W - T;
-            const bool in = e0 + e < ny;   // the accumulator past the edge may hold anything
-            float sum = r.p.pe_weight * rr * pw[e];
-            if (in) s0 += rr * rr * pw[e];
-            if (pen_on && T < 0.5f) {
-              const float ex = fmaxf(W - r.p.pen_thr, 0.f);
-              if (in) s1 += ex * ex * qw[e];
-              sum += r.p.penalty * ex * qw[e];
+          for (int e0 = 0; e0 < 32; e0 += 8) {
+            if (e0 % 16 == 0) {
+              __syncwarp();
+              tmem_ld16x(acc + (uint32_t)e0, d);
             }
-            const float g = in ? sum * W * (1.f - W) : 0.f;
-            if (OUT && in) {
-              if (r.p.aerial) r.p.aerial[i0 + (size_t)(e0 + e) * N] = I;
-              if (r.p.wafer) r.p.wafer[i0 + (size_t)(e0 + e) * N] = W;
+            float pw[8], qw[8];
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+              if (r.p.region) {
+                const bool in = e0 + e >= ry0 && e0 + e < ry1;
+                pw[e] = in && (!r.p.region_main || pre[e0 + e] > 0.5f) ? 1.f : 0.f;
+                qw[e] = in ? 1.f : 0.f;   // used where T < 0.5
+              } else {
+                pw[e] = pwp && e0 + e < ny ? __ldg(pwp + (e0 + e) * N) : 1.f;
+                qw[e] = qwp && e0 + e < ny ? __ldg(qwp + (e0 + e) * N) : pw[e];
+              }
             }
-            chk = __fmaf_rn(g, 0.f, chk);
-            d[e0 % 16 + e] = g;
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+              const float I = d[e0 % 16 + e], T = pre[e0 + e];
+              const float W = r.sigmoid(I);
+              const float rr = W - T;
+              const bool in = e0 + e < ny;   // the accumulator past the edge may hold anything
+              float sum = r.p.pe_weight * rr * pw[e];
+              if (in) s0 += rr * rr * pw[e];
+              if (pen_on && T < 0.5f) {
+                const float ex = fmaxf(W - r.p.pen_thr, 0.f);
+                if (in) s1 += ex * ex * qw[e];
+                sum += r.p.penalty * ex * qw[e];
+              }
+              const float g = in ? sum * W * (1.f - W) : 0.f;
+              if (OUT && in) {
+                if (r.p.aerial) r.p.aerial[i0 + (size_t)(e0 + e) * N] = I;
+                if (r.p.wafer) r.p.wafer[i0 + (size_t)(e0 + e) * N] = W;
+              }
+              chk = __fmaf_rn(g, 0.f, chk);
+              d[e0 % 16 + e] = g;
+            }
+            if (e0 % 16) store_a(d, e0 - 8);
           }
-          if (e0 % 16) store_a(d, e0 - 8);
         }
         bad = chk != 0.f;
       }
