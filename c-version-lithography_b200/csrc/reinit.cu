@@ -422,9 +422,10 @@ cudaError_t launch_reinit_sdf(cudaStream_t s, int rows, int cols, const float* p
                                   : columns(reinit_columns_kernel<false>);
   if (e != cudaSuccess) return e;
   if (threads <= 0) {
-    // One CTA per SM (wide images): as many threads as fit (4096^2: 342 us, 377 us with
+    // One CTA per SM (wide images): as many threads as fit (4096^2: 195 us, 212 us with
     // 512). Few row blocks: larger CTAs, whose rows are then the parallelism there is
-    // (2048^2: 110 us with 512 threads, 121 with 256; 24 x 1266^2: 596 and 555).
+    // (4 x 1266^2: 84 us with 512 threads, 86 with 256 and 90 with 1024; 24 x 1266^2: 385, 365
+    // and 442).
     const long long ctas = (long long)((rows + RI_RB - 1) / RI_RB) * nimg;
     threads = ri_rows_smem<4>(cols) > RI_SMEM / 2 ? 1024 : ctas <= 592 ? 512 : 256;
   }

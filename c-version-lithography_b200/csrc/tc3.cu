@@ -9,14 +9,14 @@
 // neighbouring items overlapped:
 //   * loader / epilogue warps move image data between global memory and shared or
 //     tensor memory;
-//   * one thread issues the bulk copies of the constant operand images and every
-//     tcgen05.mma, and commits each MMA group to an mbarrier;
+//   * one converged warp issues, by one elected lane, the bulk copies of the constant
+//     operand images and every tcgen05.mma, and commits each MMA group to an mbarrier;
 //   * the accumulators are double-buffered in tensor memory, so the epilogue of
 //     item j runs while the MMAs of item j + 1 do.
 // The roles hand buffers to each other through mbarriers (full / free per buffer,
 // phase parity per use). Every wait is bounded: on expiry, or when another role has
 // given up, a role records a code in *err (first failure only) and leaves its loop;
-// the MMA thread then waits (bounded) for its own copies and MMAs in flight, the
+// the MMA warp then waits (bounded) for its own copies and MMAs in flight, the
 // tensor memory is released and the kernel returns.
 //
 // The syntheses compute the transposed accumulator D[x][y] (tensor-memory lane =
@@ -115,12 +115,12 @@ __device__ __forceinline__ Item item_next(Item it, int T, int B) {
 // leaves its loop on a failed wait must not strand the others): every warp adds its
 // lanes' values in a fixed shuffle order and its lane 0 stores them in slot b = j & 3
 // and arrives on red_bar[b] (count = epilogue warps); a collecting thread waits for
-// the slot (bounded), adds the warps in order and writes the partials: thread 0 right
-// after its own part (fused kernel), or, in the syntheses, one warp in turn during its
-// item j + 1 (collect2). Either reads slot b before it reads the accumulator of item
-// j + 2, and no warp reaches item j + 4, which writes slot b again, before every warp
-// has read the accumulator of item j + 2 (the accumulators are double-buffered), so a
-// slot is read before it is written again.
+// the slot (bounded), adds the warps in order and writes the partials: in the fused kernel
+// a TMEM warp before it frees the accumulator that item j + 1 needs; in the syntheses one
+// warp in turn during its item j + 1 (collect2), which reads slot b before it reads the
+// accumulator of item j + 2, and no warp reaches item j + 4, which writes slot b again,
+// before every warp has read the accumulator of item j + 2 (the accumulators are
+// double-buffered). Either way a slot is read before it is written again.
 constexpr int EPI_SLOTS = 4;
 template <int NV>
 struct EpiSums {
@@ -303,7 +303,7 @@ int sm_count() {
 // part[image][yt][xt][row][c]) from a persistent pipeline:
 //   warps 0-15  load the image tile (theta -> mask for mode 1), split it into the
 //               [hi | lo] operand sA;
-//   warp 24     (one thread) copies the TX tile (per xt) and the TY tile (per yt),
+//   warp 24     (one elected lane) copies the TX tile (per xt) and the TY tile (per yt),
 //               issues stage 1 R = sA . TX^T into accR[j & 1] and stage 2
 //               Q = TY . R^T into accQ[j & 1];
 //   warps 16-23 turn R into the stage-2 operand sR, and Q into the item's partials
@@ -660,7 +660,7 @@ struct S3Resist {
 // resist (KIND 1, ResistEpilogue) or the plain (KIND 2, GradEpilogue without theta: dPE/dM
 // stored once or twice) epilogue, as launch_synth_grad_tc2 /
 // launch_synth_resist_tc2, from a persistent pipeline:
-//   warp 16      (one thread) copies the AY tile (per yt), double-buffers the band
+//   warp 16      (one elected lane) copies the AY tile (per yt), double-buffers the band
 //                operand tile Bt (per image and xt) and issues D[x][y] into acc[j & 1];
 //   warps 0-15   run the epilogue of item j while the MMA of item j + 1 runs: warp w
 //                takes lanes x = 32 (w % 4) + lane and rows y = 32 (w / 4) .. + 31.
