@@ -41,6 +41,9 @@ __device__ __forceinline__ void cp_async_wait() {
   asm volatile("cp.async.wait_group %0;" ::"n"(LEFT) : "memory");
 }
 
+// Shared memory of a CTA (227 KiB) less the static sums of the epilogues.
+constexpr size_t SMEM_CTA = 227 * 1024 - 256;
+
 // ---------------------------------------------------------------- tile analysis
 // For every 128 x 128 tile: R[y][f] = sum_x A[y][x] tw[f][x] (phase 1, f the real columns
 // Re, Im of the column twiddles), then P[r][c] = sum_y T(r, y) R[y][c] (phase 2), each sum
@@ -52,7 +55,9 @@ __device__ __forceinline__ void cp_async_wait() {
 // registers while the current ones are multiplied (two shared buffers, one barrier per
 // block), the row twiddles of phase 2 are copied asynchronously during phase 1 and kept for
 // all rows, and phase 2 gives every thread RPT rows (with their conjugates when sym) x 2
-// columns: 62 and 72 us (forward, adjoint) -> 45 and 45 at 2048^2.
+// columns: 62 and 72 us (forward, adjoint) -> 45 and 45 at 2048^2. Bands whose row twiddles
+// (1 KiB a row) do not fit beside the rest of a CTA's shared memory, from about 160 rows on,
+// take them in equal pieces of `rows` rows (PIECES): only the first one is copied during phase 1.
 constexpr int AT_NT = 256, AT_TM = 8, AT_BK = 32;
 constexpr int AT_TILE = 128;             // rows, and columns of x per tile
 constexpr int AT_AS = AT_TILE + 4;       // row stride of an image block [BK][128]
@@ -67,6 +72,7 @@ struct AnalysisArgs {
   int ncols;
   const float2* TY;    // [nr][N] row twiddles
   int nrows_out, nr, sym;
+  int rows;            // PIECES: rows whose twiddles are staged at a time (a multiple of RPT)
   float2* part;        // [tiles][nrows_out][ncols]
 };
 
@@ -74,7 +80,7 @@ struct AnalysisArgs {
 // 32 consecutive y then fall into different banks).
 __host__ __device__ constexpr int at_ts(int nr, int rpt) { return (nr + rpt - 1) / rpt * rpt | 1; }
 
-template <int TN, int RPT>
+template <int TN, int RPT, bool PIECES>
 __global__ void __launch_bounds__(AT_NT, 2)
 analysis_tile_kernel(AnalysisArgs a) {
   extern __shared__ __align__(16) float smem[];
@@ -85,7 +91,8 @@ analysis_tile_kernel(AnalysisArgs a) {
   float* R = smem;                                     // [128][RS] (after phase 1)
   constexpr int P1 = 2 * AT_BK * (AT_AS + BS), P2 = AT_TILE * RS;
   float2* TYs = reinterpret_cast<float2*>(smem + ((P1 > P2 ? P1 : P2) + 3) / 4 * 4);   // [128][ts]
-  const int ts = at_ts(a.nr, RPT);
+  const int rows = PIECES ? a.rows : a.nr;
+  const int ts = at_ts(rows, RPT);
   const int tid = threadIdx.x, tx = tid % 16, ty = tid / 16;
   const int x0 = blockIdx.x * AT_TILE, y0 = blockIdx.y * AT_TILE;
   const int f0 = blockIdx.z * BN;
@@ -93,12 +100,15 @@ analysis_tile_kernel(AnalysisArgs a) {
   const int nkt = (min(N - x0, AT_TILE) + AT_BK - 1) / AT_BK;
   pdl_trigger();
   // the row twiddles (constant tables), ready long before phase 2
-  for (int e = tid; e < AT_TILE * ts; e += AT_NT) {
-    const int yy = e % AT_TILE, r = e / AT_TILE;
-    const bool ok = r < a.nr && y0 + yy < N;
-    cp_async<8>(TYs + yy * ts + r, a.TY + (ok ? (size_t)r * N + y0 + yy : 0), ok);
-  }
-  cp_async_commit();
+  auto copy_rows = [&](int first) {
+    for (int e = tid; e < AT_TILE * ts; e += AT_NT) {
+      const int yy = e % AT_TILE, r = e / AT_TILE;
+      const bool ok = first + r < a.nr && y0 + yy < N;
+      cp_async<8>(TYs + yy * ts + r, a.TY + (ok ? (size_t)(first + r) * N + y0 + yy : 0), ok);
+    }
+    cp_async_commit();
+  };
+  copy_rows(0);
   float va[16], vb[2 * TN];
   // image block kt: rows (tid >> 3) + 32 q, columns 4 (tid & 7) ..; twiddle block kt: column
   // tid % 32 of the rows f tid / 32 + 8 q
@@ -193,70 +203,84 @@ analysis_tile_kernel(AnalysisArgs a) {
   __syncthreads();
   // Phase 2: item (row group, column pair).
   const int c0 = f0 / 2, npairs = (min(BN / 2, a.ncols - c0) + 1) / 2;
-  const int items = (a.nr + RPT - 1) / RPT * npairs;
   float2* out = a.part + (size_t)(blockIdx.y * gridDim.x + blockIdx.x) * a.nrows_out * a.ncols;
-  for (int it = tid; it < items; it += AT_NT) {
-    const int r0 = it / npairs * RPT, cp = it % npairs, c = c0 + 2 * cp;
-    float2 p[RPT][2], m[RPT][2];   // rows r, and (sym) their conjugates' rows -r
+  for (int first = 0;; first += rows) {
+    const int items = (min(rows, a.nr - first) + RPT - 1) / RPT * npairs;
+    for (int it = tid; it < items; it += AT_NT) {
+      const int r0 = it / npairs * RPT, cp = it % npairs, c = c0 + 2 * cp;
+      float2 p[RPT][2], m[RPT][2];   // rows r, and (sym) their conjugates' rows -r
 #pragma unroll
-    for (int i = 0; i < RPT; ++i) p[i][0] = p[i][1] = m[i][0] = m[i][1] = make_float2(0.f, 0.f);
-    const float2* t0 = TYs + r0;
-    const float* rr = R + 4 * cp;
-    if (!a.sym) {
+      for (int i = 0; i < RPT; ++i) p[i][0] = p[i][1] = m[i][0] = m[i][1] = make_float2(0.f, 0.f);
+      const float2* t0 = TYs + r0;
+      const float* rr = R + 4 * cp;
+      if (!a.sym) {
 #pragma unroll 4
-      for (int yy = 0; yy < AT_TILE; ++yy) {
-        const float4 rv = *reinterpret_cast<const float4*>(rr + yy * RS);
-        const float2 ra = make_float2(rv.x, rv.y), rb = make_float2(rv.z, rv.w);
+        for (int yy = 0; yy < AT_TILE; ++yy) {
+          const float4 rv = *reinterpret_cast<const float4*>(rr + yy * RS);
+          const float2 ra = make_float2(rv.x, rv.y), rb = make_float2(rv.z, rv.w);
 #pragma unroll
-        for (int i = 0; i < RPT; ++i) {
-          const float2 t = t0[yy * ts + i];
-          cfma(p[i][0], t, ra);
-          cfma(p[i][1], t, rb);
+          for (int i = 0; i < RPT; ++i) {
+            const float2 t = t0[yy * ts + i];
+            cfma(p[i][0], t, ra);
+            cfma(p[i][1], t, rb);
+          }
         }
-      }
-    } else {
+      } else {
 #pragma unroll 2
-      for (int yy = 0; yy < AT_TILE; ++yy) {
-        const float4 rv = *reinterpret_cast<const float4*>(rr + yy * RS);
-        const float2 ra = make_float2(rv.x, rv.y), rb = make_float2(rv.z, rv.w);
+        for (int yy = 0; yy < AT_TILE; ++yy) {
+          const float4 rv = *reinterpret_cast<const float4*>(rr + yy * RS);
+          const float2 ra = make_float2(rv.x, rv.y), rb = make_float2(rv.z, rv.w);
 #pragma unroll
-        for (int i = 0; i < RPT; ++i) {
-          const float2 t = t0[yy * ts + i], tc = conjf2(t);
-          cfma(p[i][0], t, ra);
-          cfma(p[i][1], t, rb);
-          cfma(m[i][0], tc, ra);
-          cfma(m[i][1], tc, rb);
+          for (int i = 0; i < RPT; ++i) {
+            const float2 t = t0[yy * ts + i], tc = conjf2(t);
+            cfma(p[i][0], t, ra);
+            cfma(p[i][1], t, rb);
+            cfma(m[i][0], tc, ra);
+            cfma(m[i][1], tc, rb);
+          }
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < RPT; ++i) {
+        const int r = first + r0 + i;
+        if (r >= a.nr) break;
+        float2* o = out + (size_t)(a.sym ? a.nr - 1 + r : r) * a.ncols + c;
+        o[0] = p[i][0];
+        if (c + 1 < a.ncols) o[1] = p[i][1];
+        if (a.sym && r > 0) {
+          o = out + (size_t)(a.nr - 1 - r) * a.ncols + c;
+          o[0] = m[i][0];
+          if (c + 1 < a.ncols) o[1] = m[i][1];
         }
       }
     }
-#pragma unroll
-    for (int i = 0; i < RPT; ++i) {
-      const int r = r0 + i;
-      if (r >= a.nr) break;
-      float2* o = out + (size_t)(a.sym ? a.nr - 1 + r : r) * a.ncols + c;
-      o[0] = p[i][0];
-      if (c + 1 < a.ncols) o[1] = p[i][1];
-      if (a.sym && r > 0) {
-        o = out + (size_t)(a.nr - 1 - r) * a.ncols + c;
-        o[0] = m[i][0];
-        if (c + 1 < a.ncols) o[1] = m[i][1];
-      }
-    }
+    if (!PIECES || first + rows >= a.nr) break;
+    __syncthreads();   // the rows in use have been read
+    copy_rows(first + rows);
+    cp_async_wait<0>();
+    __syncthreads();
   }
 }
 
-template <int TN, int RPT>
-static cudaError_t analysis_tile_t(cudaStream_t s, const AnalysisArgs& a) {
+template <int TN, int RPT, bool PIECES = false>
+static cudaError_t analysis_tile_t(cudaStream_t s, AnalysisArgs a) {
   constexpr int BN = 16 * TN;
   constexpr size_t p1 = 2 * AT_BK * (AT_AS + BN + 1), p2 = AT_TILE * (BN + 4);
-  const size_t smem = ((p1 > p2 ? p1 : p2) + 3) / 4 * 4 * sizeof(float) +
-                      (size_t)AT_TILE * at_ts(a.nr, RPT) * sizeof(float2);
-  cudaError_t e = cudaFuncSetAttribute(analysis_tile_kernel<TN, RPT>,
+  constexpr size_t base = ((p1 > p2 ? p1 : p2) + 3) / 4 * 4 * sizeof(float);
+  auto rows_smem = [](int rows) { return (size_t)AT_TILE * at_ts(rows, RPT) * sizeof(float2); };
+  a.rows = a.nr;
+  for (int pieces = 2; base + rows_smem(a.rows) > SMEM_CTA; ++pieces) {
+    // no rule of its own for a tall band: pieces of the 32-column variant
+    if constexpr (!PIECES) return analysis_tile_t<2, 2, true>(s, a);
+    a.rows = ((a.nr + pieces - 1) / pieces + RPT - 1) / RPT * RPT;
+  }
+  const size_t smem = base + rows_smem(a.rows);
+  cudaError_t e = cudaFuncSetAttribute(analysis_tile_kernel<TN, RPT, PIECES>,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   const int t = (a.N + AT_TILE - 1) / AT_TILE;
   dim3 grid(t, t, (2 * a.ncols + BN - 1) / BN);
-  return launch_pdl(analysis_tile_kernel<TN, RPT>, grid, dim3(AT_NT), smem, s, a);
+  return launch_pdl(analysis_tile_kernel<TN, RPT, PIECES>, grid, dim3(AT_NT), smem, s, a);
 }
 
 int analysis_tiles(int N) {
@@ -276,7 +300,7 @@ cudaError_t launch_analysis(cudaStream_t s, int mode, const float* in, float* ma
                             int* flag, const float* tw, int N, int ncols, const float2* TY,
                             int nrows_out, int nr, int sym, float2* part) {
   const int vec4 = (N % 4 == 0) && (reinterpret_cast<uintptr_t>(in) % 16 == 0);
-  const AnalysisArgs a{in, mask_out, flag, N, mode, vec4, tw, ncols, TY, nrows_out, nr, sym, part};
+  const AnalysisArgs a{in, mask_out, flag, N, mode, vec4, tw, ncols, TY, nrows_out, nr, sym, nr, part};
   const int n2 = 2 * ncols, tiles = analysis_tiles(N);
   if (tiles < AT_SMALL) return analysis_tile_t<1, 1>(s, a);
   if (tiles < AT_MID) return analysis_tile_t<2, 2>(s, a);
@@ -344,19 +368,21 @@ cudaError_t launch_reduce_tiles(cudaStream_t s, const float2* part, int tiles, i
 // warps of small thread tiles count for more than the FMAs per operand byte of large ones
 // (8 x 8 pixels per thread: a 2048^2 CTM evaluation 215 us against 206). With 128 x 128 tiles
 // and two barriers per 16 inner columns the two syntheses of 2048^2 took 48 and 47 us (FMA
-// pipe 25 % busy), now 33 and 29; of 256^2 23 us, now 7.
+// pipe 25 % busy), now 33 and 29; of 256^2 23 us, now 7. An inner dimension whose operands do
+// not fit in shared memory (512 bytes per f: bands from 227 rows on) is taken in slices of ns
+// (SLICES).
 constexpr int SF_T = 64, SF_NT = 256, SF_SS = SF_T + 4;
 
-template <class Epi>
+template <class Epi, bool SLICES>
 __global__ void __launch_bounds__(SF_NT)
 synth_kernel(const float* __restrict__ AYt, const float* __restrict__ Bt, int N, int ld, int nf,
-             Epi epi) {
+             int slice, Epi epi) {
   extern __shared__ __align__(16) float sf[];
-  float* As = sf;                   // [nf][64]
-  float* Bs = sf + nf * SF_T;       // [nf][64]
+  const int ns = SLICES ? slice : nf;
+  float* As = sf;                   // [ns][64]
+  float* Bs = sf + ns * SF_T;       // [ns][64]
   const int tid = threadIdx.x, tx = tid % 16, ty = tid / 16;
   const int m0 = blockIdx.y * SF_T, n0 = blockIdx.x * SF_T;
-  const int half = (nf + 1) / 2;
   // rows f0 .. f1 - 1 of an operand, 64 floats from `first`: zeros past the row stride
   auto copy = [&](float* dst, const float* src, int f0, int f1, int first) {
     const int c = 4 * (tid % 16);
@@ -365,12 +391,13 @@ synth_kernel(const float* __restrict__ AYt, const float* __restrict__ Bt, int N,
       cp_async<16>(dst + f * SF_T + c, ok ? src + (size_t)f * ld + first + c : src, ok);
   };
   pdl_trigger();
+  int half = (ns + 1) / 2;
   copy(As, AYt, 0, half, m0);
   pdl_wait();   // the band operand comes from the previous kernel
   copy(Bs, Bt, 0, half, n0);
   cp_async_commit();
-  copy(As, AYt, half, nf, m0);
-  copy(Bs, Bt, half, nf, n0);
+  copy(As, AYt, half, ns, m0);
+  copy(Bs, Bt, half, ns, n0);
   cp_async_commit();
   // the epilogue's input lines into L2
   if (const float* img = epi.input()) {
@@ -400,8 +427,27 @@ synth_kernel(const float* __restrict__ AYt, const float* __restrict__ Bt, int N,
   multiply(0, half);
   cp_async_wait<0>();
   __syncthreads();
-  multiply(half, nf);
+  multiply(half, ns);
   __syncthreads();
+  for (int f0 = ns; SLICES && f0 < nf; f0 += ns) {   // the slices after the first
+    const int n = min(ns, nf - f0);
+    half = (n + 1) / 2;
+    const float* At = AYt + (size_t)f0 * ld;
+    const float* Bf = Bt + (size_t)f0 * ld;
+    copy(As, At, 0, half, m0);
+    copy(Bs, Bf, 0, half, n0);
+    cp_async_commit();
+    copy(As, At, half, n, m0);
+    copy(Bs, Bf, half, n, n0);
+    cp_async_commit();
+    cp_async_wait<1>();
+    __syncthreads();
+    multiply(0, half);
+    cp_async_wait<0>();
+    __syncthreads();
+    multiply(half, n);
+    __syncthreads();
+  }
   float* stage = sf;   // [64][SS], over the operands
 #pragma unroll
   for (int i = 0; i < 4; ++i)
@@ -423,14 +469,19 @@ int synth_blocks(int N) { return ((N + SF_T - 1) / SF_T) * ((N + SF_T - 1) / SF_
 template <class Epi>
 static cudaError_t launch_synth(cudaStream_t s, const float* AYt, const float* Bt, int N, int nf,
                                 const Epi& e, int* nblocks) {
-  const size_t smem = std::max((size_t)2 * nf * SF_T, (size_t)SF_T * SF_SS) * sizeof(float);
-  cudaError_t err = cudaFuncSetAttribute(synth_kernel<Epi>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (err != cudaSuccess) return err;
+  int ns = nf;   // equal slices
+  for (int slices = 2; (size_t)2 * ns * SF_T * sizeof(float) > SMEM_CTA; ++slices)
+    ns = (nf + slices - 1) / slices;
+  const size_t smem = std::max((size_t)2 * ns * SF_T, (size_t)SF_T * SF_SS) * sizeof(float);
   const int t = (N + SF_T - 1) / SF_T;
   *nblocks = t * t;
-  return launch_pdl(synth_kernel<Epi>, dim3(t, t, 1), dim3(SF_NT), smem, s, AYt, Bt, N, synth_ld(N),
-                    nf, e);
+  auto launch = [&](auto kernel) -> cudaError_t {
+    const cudaError_t err =
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (err != cudaSuccess) return err;
+    return launch_pdl(kernel, dim3(t, t, 1), dim3(SF_NT), smem, s, AYt, Bt, N, synth_ld(N), nf, ns, e);
+  };
+  return ns < nf ? launch(synth_kernel<Epi, true>) : launch(synth_kernel<Epi, false>);
 }
 
 cudaError_t launch_synth_resist(cudaStream_t s, const float* AYt, const float* Bt, int N, int nf,
