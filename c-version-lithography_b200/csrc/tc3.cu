@@ -14,10 +14,10 @@
 //   * the accumulators are double-buffered in tensor memory, so the epilogue of
 //     item j runs while the MMAs of item j + 1 do.
 // The roles hand buffers to each other through mbarriers (full / free per buffer,
-// phase parity per use). Every wait is bounded: on expiry, or when another role has
-// given up, a role records a code in *err (first failure only) and leaves its loop;
-// the MMA warp then waits (bounded) for its own copies and MMAs in flight, the
-// tensor memory is released and the kernel returns.
+// phase parity per use). Every wait is bounded and a whole warp's (pwait_warp): on
+// expiry, or when another role has given up, the warp records a code in *err (first
+// failure only) and leaves its loop; the MMA warp then waits (bounded) for its own
+// copies and MMAs in flight, the tensor memory is released and the kernel returns.
 //
 // The syntheses compute the transposed accumulator D[x][y] (tensor-memory lane =
 // image column x) so that the 32 lanes of a warp touch 32 consecutive pixels of an
@@ -48,24 +48,11 @@ __device__ __forceinline__ uint8_t* align1024(uint8_t* p) {
                                     ~static_cast<uintptr_t>(1023));
 }
 
-// Bounded wait for the completion of the phase of `bar` with parity `parity`. Gives
-// up when another role has failed (*fail) or after about 2^31 SM cycles (one second),
-// then records `code` in *err (first failure wins) and returns false.
-__device__ __forceinline__ bool pwait(uint32_t bar, uint32_t parity, volatile int* fail, int* err,
-                                      int code) {
-  if (tc::mbar_try_wait(bar, parity)) return true;
-  const long long t0 = clock64();
-  while (!tc::mbar_try_wait(bar, parity)) {
-    if (*fail) return false;
-    if (clock64() - t0 > (1LL << 31)) {
-      *fail = 1;
-      atomicCAS(err, 0, code);
-      return false;
-    }
-  }
-  return true;
-}
-// The same for a whole warp, which stays converged (the MMA warps).
+// Bounded wait of a whole warp for the completion of the phase of `bar` with parity `parity`.
+// Gives up when another role has failed (*fail) or after about 2^31 SM cycles (one second),
+// then records `code` in *err (first failure wins) and returns false. Every lane gets the same
+// answer: a lane that gave up alone would leave the others at the warp-wide instructions that
+// follow (tcgen05.ld, shuffles, __syncwarp), which wait for it without a limit.
 __device__ __forceinline__ bool pwait_warp(uint32_t bar, uint32_t parity, volatile int* fail,
                                            int* err, int code) {
   constexpr unsigned ALL = 0xffffffffu;
@@ -142,12 +129,13 @@ __device__ __forceinline__ void epi_put(EpiSums<NV>& sh, uint32_t red_bar, int b
     mbar_arrive(red_bar);
   }
 }
-// The slot's sums over nw warps, added in warp order (false when the wait gave up).
+// The slot's sums over nw warps, added in warp order (false when the wait gave up); a whole
+// warp calls it, and every lane gets them.
 template <int NV>
 __device__ __forceinline__ bool epi_take(const EpiSums<NV>& sh, uint32_t red_bar, int b,
                                          uint32_t parity, int nw, volatile int* fail, int* err,
                                          int code, double (&out)[NV]) {
-  if (!pwait(red_bar, parity, fail, err, code)) return false;
+  if (!pwait_warp(red_bar, parity, fail, err, code)) return false;
 #pragma unroll
   for (int k = 0; k < NV; ++k) {
     out[k] = 0.0;
@@ -185,8 +173,8 @@ __device__ __forceinline__ void prefetch_rows(const float* img, int N, int yb, i
   if (pf && y < N && x0 + 32 <= N) tc::prefetch_l2_line(img + (size_t)y * N + x0);
 }
 
-// The sums of item j (slot j & 3) over nw warps into out[0 .. nv - 1], by lane 0 of the
-// warp that collects item j (false when the wait gave up). Item j is collected by warp
+// The sums of item j (slot j & 3) over nw warps into out[0 .. nv - 1], by the whole warp that
+// collects item j (false when the wait gave up). Item j is collected by warp
 // j % nw one item later, when every warp has normally stored its part, so that no warp
 // waits for the others in the common case.
 __device__ __forceinline__ bool collect2(const EpiSums<2>& sh, uint64_t* red_bar, int j, int nw,
@@ -196,8 +184,10 @@ __device__ __forceinline__ bool collect2(const EpiSums<2>& sh, uint64_t* red_bar
   if (!epi_take<2>(sh, tc::smem_u32(&red_bar[j & 3]), j & 3, (j >> 2) & 1, nw, fail, err, code,
                    t))
     return false;
-  out[0] = t[0];
-  if (nv > 1) out[1] = t[1];
+  if ((threadIdx.x & 31) == 0) {
+    out[0] = t[0];
+    if (nv > 1) out[1] = t[1];
+  }
   return true;
 }
 
@@ -463,7 +453,7 @@ analysis_tc3_kernel(Tc2Analysis a, int T, int B, const uint8_t* __restrict__ txI
       bool bad = false;
       conv_half(cur, 0, bad);
       // sA is free once stage 1 of the previous item has completed
-      if (j > 0 && !pwait(bar(1 + ((j - 1) & 1)), ((j - 1) >> 1) & 1, vfail, err, 11)) break;
+      if (j > 0 && !pwait_warp(bar(1 + ((j - 1) & 1)), ((j - 1) >> 1) & 1, vfail, err, 11)) break;
       store_half(0);
       if (j + 1 < n) load_half(item_next(cur, T, B), 0);
       conv_half(cur, HALF, bad);
@@ -487,9 +477,9 @@ analysis_tc3_kernel(Tc2Analysis a, int T, int B, const uint8_t* __restrict__ txI
         prv = cur;
         cur = item_next(cur, T, B);
       }
-      if (j < n && !pwait(bar(1 + (j & 1)), (j >> 1) & 1, vfail, err, 12)) break;
+      if (j < n && !pwait_warp(bar(1 + (j & 1)), (j >> 1) & 1, vfail, err, 12)) break;
       // stage 2 of the previous item done: sR is free and its Q is ready
-      if (j > 0 && !pwait(bar(4 + ((j - 1) & 1)), ((j - 1) >> 1) & 1, vfail, err, 13)) break;
+      if (j > 0 && !pwait_warp(bar(4 + ((j - 1) & 1)), ((j - 1) >> 1) & 1, vfail, err, 13)) break;
       tc::fence_after();
       if (j < n) {
         r_to_operand(tmem + (uint32_t)((j & 1) * 128) + ((uint32_t)lane_base << 16), sR, BN,
@@ -754,7 +744,7 @@ synth_tc3_kernel(const uint8_t* __restrict__ Aimg, const uint8_t* __restrict__ B
       const bool xin = x < N;
       const bool full = xin && yb + 31 < N;
       const size_t base = (size_t)it.z * N * N;
-      if (!pwait(bar(3 + (j & 1)), (j >> 1) & 1, vfail, err, 21)) break;
+      if (!pwait_warp(bar(3 + (j & 1)), (j >> 1) & 1, vfail, err, 21)) break;
       tc::fence_after();
       float d[32];
       tc::tmem_ld32(tmem + (uint32_t)((j & 1) * 128) + lane_addr + (uint32_t)(32 * h), d);
@@ -829,14 +819,14 @@ synth_tc3_kernel(const uint8_t* __restrict__ Aimg, const uint8_t* __restrict__ B
         if (KIND == 0) epi_put<1>(red, tc::smem_u32(&red_bar[j & 3]), j & 3, {v[0]});
         else epi_put<2>(red, tc::smem_u32(&red_bar[j & 3]), j & 3, v);
         // the sums of item j - 1, by one warp in turn
-        if (j > 0 && lane == 0 && warp == (j - 1) % S3_EPIW &&
+        if (j > 0 && warp == (j - 1) % S3_EPIW &&
             !collect2(red, red_bar, j - 1, S3_EPIW, vfail, err, 27, sums_out(ip), KIND == 0 ? 1 : 2))
           break;
       }
       done = j + 1;
     }
     // the sums of the last item
-    if (sums && n > 0 && done == n && lane == 0 && warp == (n - 1) % S3_EPIW)
+    if (sums && n > 0 && done == n && warp == (n - 1) % S3_EPIW)
       collect2(red, red_bar, n - 1, S3_EPIW, vfail, err, 28, sums_out(ip), KIND == 0 ? 1 : 2);
   } else if (warp == S3_MMAW) {
     // ------------------------------------------------------------ MMA warp
@@ -1068,7 +1058,7 @@ fused_tc3_kernel(const uint8_t* __restrict__ Aimg, const uint8_t* __restrict__ B
           *reinterpret_cast<uint4*>(w + MN_LO) = l4;
         }
       };
-      if (!pwait(bar(SM + (j & 1)), (j >> 1) & 1, vfail, err, 31)) break;
+      if (!pwait_warp(bar(SM + (j & 1)), (j >> 1) & 1, vfail, err, 31)) break;
       tc::fence_after();
       // d[e] becomes dL/dI at (yb + e0 + e, x), 0 outside the image.
       float s0 = 0.f, s1 = 0.f;
@@ -1249,9 +1239,9 @@ fused_tc3_kernel(const uint8_t* __restrict__ Aimg, const uint8_t* __restrict__ B
     const int nu = (int)rf / 8;   // 8-column groups of the rows f
     Item it = item_at(lo, T, B), ip = it;
     for (int j = 0; j <= n; ++j, ip = it, it = item_next(it, T, B)) {
-      if (j < n && !pwait(bar(M1), j & 1, vfail, err, 33)) break;
+      if (j < n && !pwait_warp(bar(M1), j & 1, vfail, err, 33)) break;
       // MMA2(j - 1) has read sR and written Q(j - 1)
-      if (j > 0 && !pwait(bar(M2), (j - 1) & 1, vfail, err, 32)) break;
+      if (j > 0 && !pwait_warp(bar(M2), (j - 1) & 1, vfail, err, 32)) break;
       tc::fence_after();
       if (j < n) {
         r_to_operand(tR + lane_addr, sR, (int)rf, lane_base, u0, F3_TMW / 4, nu);
@@ -1260,10 +1250,10 @@ fused_tc3_kernel(const uint8_t* __restrict__ Aimg, const uint8_t* __restrict__ B
         __syncwarp();
         // The loss sums of item j, by a warp without a share of Q, before it frees accR: their
         // slot is written again in item j + 4, and SMMA(j + 2) already follows MMA1(j + 1).
-        if (warp == F3_MMAW - 1 && lane == 0) {
+        if (warp == F3_MMAW - 1) {
           double t[2];
           if (epi_take<2>(red, tc::smem_u32(&red_bar[j & 3]), j & 3, (j >> 2) & 1, F3_EPIW, vfail,
-                          err, 46, t)) {
+                          err, 46, t) && lane == 0) {
             const size_t bid = ((size_t)it.z * T + it.yt) * T + it.xt;
             r.p.loss_partial[2 * bid] = t[0];
             r.p.loss_partial[2 * bid + 1] = t[1];
