@@ -1701,6 +1701,8 @@ int litho_ctx_reserve(litho_ctx* ctx, const litho_cache* cache, int batch) {
   st = ctx->ensure_scratch(std::max(L.total, n * batch * sizeof(float)));
   if (st) return st;
   st = ctx->ensure_red(RED_PART + std::max(dt_slots(batch), (size_t)batch + 8));
+  // The per-image results of the host-synchronous calls, three of the CTM evaluation at most.
+  if (!st) st = ctx->ensure_host(HOST_MORE + 3 * (size_t)batch);
   if (!st) st = ctx->ensure_deferred();
   if (st) return st;
   LITHO_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));

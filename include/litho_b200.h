@@ -308,9 +308,9 @@ int litho_evolution_term(litho_ctx* ctx, int rows, int cols, const float* d_phi,
  * value). d_mask (nullable) receives the printed mask sdf >= 0 as 1/0 floats. */
 int litho_reinit_sdf(litho_ctx* ctx, int rows, int cols, const float* d_phi, double dx,
                      double dy, float* d_sdf, float* d_mask);
-/* Grows the context's device scratch to what the batched calls on `batch` images of
- * this cache need (the CTM / PE-gradient chain and the batched RK2 update), so that a
- * serving loop never allocates between its steps. */
+/* Grows the context's device scratch, and its pinned host memory for results, to what the
+ * batched calls on `batch` images of this cache need (the CTM / PE-gradient chain and the
+ * batched RK2 update), so that a serving loop never allocates between its steps. */
 int litho_ctx_reserve(litho_ctx* ctx, const litho_cache* cache, int batch);
 /* Autotuner: times the candidate schedules on this device and keeps the fastest in
  * the context for the calls that follow. With a cache: the schedule of the

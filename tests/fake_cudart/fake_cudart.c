@@ -1,0 +1,38 @@
+/* A CUDA runtime for tests of the library's host side without a GPU: loaded before libcudart
+ * (LD_PRELOAD), it serves "device" and pinned memory from the heap, accepts every launch
+ * without running it, and counts the allocations. */
+#include <stdlib.h>
+#include <string.h>
+
+int fake_allocs = 0;              /* cudaMalloc and cudaMallocHost calls so far */
+size_t fake_sizes[4096];          /* their sizes in bytes */
+
+static int take(void **p, size_t n) {
+  if (fake_allocs < 4096) fake_sizes[fake_allocs] = n;
+  ++fake_allocs;
+  *p = calloc(1, n ? n : 1);
+  return *p ? 0 : 2;
+}
+int cudaMalloc(void **p, size_t n) { return take(p, n); }
+int cudaMallocHost(void **p, size_t n) { return take(p, n); }
+int cudaFree(void *p) { free(p); return 0; }
+int cudaFreeHost(void *p) { free(p); return 0; }
+int cudaMemcpy(void *d, const void *s, size_t n, int k) { (void)k; memcpy(d, s, n); return 0; }
+int cudaMemcpyAsync(void *d, const void *s, size_t n, int k, void *st) {
+  (void)k; (void)st; memcpy(d, s, n); return 0;
+}
+int cudaMemsetAsync(void *d, int v, size_t n, void *st) { (void)st; memset(d, v, n); return 0; }
+int cudaSetDevice(int d) { (void)d; return 0; }
+int cudaGetDevice(int *d) { *d = 0; return 0; }
+int cudaGetDeviceCount(int *n) { *n = 1; return 0; }
+int cudaDeviceSynchronize(void) { return 0; }
+int cudaDeviceGetAttribute(int *v, int a, int d) { (void)a; (void)d; *v = 148; return 0; }
+int cudaGetLastError(void) { return 0; }
+int cudaPeekAtLastError(void) { return 0; }
+int cudaStreamSynchronize(void *s) { (void)s; return 0; }
+int cudaFuncSetAttribute(const void *f, int a, int v) { (void)f; (void)a; (void)v; return 0; }
+int cudaLaunchKernelExC(const void *c, const void *f, void **a) { (void)c; (void)f; (void)a; return 0; }
+struct fake_dim3 { unsigned x, y, z; };
+int cudaLaunchKernel(const void *f, struct fake_dim3 g, struct fake_dim3 b, void **a, size_t m, void *s) {
+  (void)f; (void)g; (void)b; (void)a; (void)m; (void)s; return 0;
+}
