@@ -61,7 +61,9 @@ __device__ __forceinline__ float sqrt_normal(float x) {
 // before the weights, which are invariant under that; the scaled values stay inside FP32
 // range. alpha_i = gamma_i / S_i^2 and sum(alpha_i d_i) / sum(alpha_i) are both multiplied
 // by 10 S1^2 S2^2 S3^2: one division, of values in [1e-24, 1e8]. A window of differences
-// below 1e-18 counts as 1e-18: its weights only mix values of that size.
+// below 1.1e-19, whose squares FP32 does not hold as normal numbers, counts as 1.1e-19: its
+// weights only mix values of that size.
+constexpr float WENO_TINY = 1.1e-19f;
 template <int N>
 __device__ __forceinline__ void weno5_chain(const float2 (&D)[N + 5], float2 (&m)[N], float2 (&p)[N]) {
   float2 e[N + 4], t[N + 3], t2[N + 3];
@@ -83,8 +85,8 @@ __device__ __forceinline__ void weno5_chain(const float2 (&D)[N + 5], float2 (&m
     cB[i + 1] = cand(D[i + 2], -1.f / 3.f, e[i + 1], -1.f / 6.f, e[i + 2]);
   }
   static_assert(N == 2, "three windows around D[2 .. 4]");
-  const float2 mid = make_float2(fmaxf(fmaxf(fabsf(D[2].x), fabsf(D[3].x)), fmaxf(fabsf(D[4].x), 1e-18f)),
-                                 fmaxf(fmaxf(fabsf(D[2].y), fabsf(D[3].y)), fmaxf(fabsf(D[4].y), 1e-18f)));
+  const float2 mid = make_float2(fmaxf(fmaxf(fabsf(D[2].x), fabsf(D[3].x)), fmaxf(fabsf(D[4].x), WENO_TINY)),
+                                 fmaxf(fmaxf(fabsf(D[2].y), fabsf(D[3].y)), fmaxf(fabsf(D[4].y), WENO_TINY)));
 #pragma unroll
   for (int i = 0; i <= N; ++i) {
     // the largest |D| of the window: its three middle ones and two of (left, right) ends
@@ -229,7 +231,15 @@ struct LsArgs {
 // Longer strips fed by cp.async one pass ahead removed the wait for the tile but cost as
 // many instructions as they hid (1.24 against 1.23 ms per update at that stage), and scalar
 // FFMA on blocks of 2 x 4 pixels ran out of registers and instruction cache (1.6 ms).
-template <int WHAT, int RPT, bool WIN>
+//
+// DIV: every difference is divided by the spacing before any product of differences, as the
+// reference does it. Products of undivided ones leave FP32's range when the spacing, and a
+// signed distance with it, is far from 1: the curvature's are its third power, at a spacing of
+// 1e-12 its error has doubled and at 1e-15 it is NaN. So DIV serves the spacings outside
+// LS_NEAR .. LS_FAR, inside which the products of slopes from 1e-8 to 1e9 stay in range and
+// the divisions would cost 3.6 % (16 images of 2048^2: 1136 us an update against 1096).
+constexpr float LS_NEAR = 1.f / 4096, LS_FAR = 4096.f;
+template <int WHAT, int RPT, bool WIN, bool DIV>
 __global__ void __launch_bounds__(LS_NT, RPT == 1 ? 6 : 7) levelset_kernel(LsArgs a) {
   constexpr int SH = LS_TY * RPT + 2 * LS_H;
   __shared__ __align__(16) float t[SH][LS_SW];
@@ -279,7 +289,8 @@ __global__ void __launch_bounds__(LS_NT, RPT == 1 ? 6 : 7) levelset_kernel(LsArg
   load_tile<SH>(t, phi, a.rows, a.cols, y0, x0, a.vec4 != 0);
   __syncthreads();
   const float idx = 1.f / a.dx, idy = 1.f / a.dy;
-  const float ix2 = 0.25f * idx * idx, iy2 = 0.25f * idy * idy, kb = a.b * ix2 * iy2;
+  const float ix2 = DIV ? 1.f : 0.25f * idx * idx, iy2 = DIV ? 1.f : 0.25f * idy * idy;
+  const float kb = a.b * ix2 * iy2;
   const float dt = (WHAT >= 3) ? a.dt[(size_t)blockIdx.z * a.dt_stride] : 0.f;
   if (x >= a.cols) return;
 #pragma unroll 1
@@ -326,16 +337,23 @@ __global__ void __launch_bounds__(LS_NT, RPT == 1 ? 6 : 7) levelset_kernel(LsArg
       if (x >= 2 && x + 1 < a.cols - 2 && y >= 2 && y + 1 < a.rows - 2) {
         // Every difference is central. d(y, x) = phi(y, x + 1) - phi(y, x - 1) of columns x
         // and x + 1 on the rows y - 1 .. y + 2; along x, d of x + 1 is also the step from x.
+        // DIV: first and second differences are divided by the two spacings they span, and
+        // kappa_value by 1.
+        const float2 hx = f2(0.5f * idx), hy = f2(0.5f * idy);
+        auto over = [](float2 d, float2 h) { return DIV ? __fmul2_rn(d, h) : d; };
         const float2 up = at2(-1, -2), un = at2(-1, 2), dp = at2(2, -2), dn = at2(2, 2);
-        const float2 dm = make_float2(col[2].y - up.y, un.x - col[2].x);   // row y - 1
-        const float2 da = make_float2(ra[5] - ra[3], ra[6] - ra[4]);       // row y
-        const float2 db = make_float2(rb[5] - rb[3], rb[6] - rb[4]);       // row y + 1
-        const float2 dd = make_float2(col[5].y - dp.y, dn.x - col[5].x);   // row y + 2
-        const float2 pyA = sub2(col[4], col[2]), pyB = sub2(col[5], col[3]);
-        const float2 pyyA = sub2(pyB, sub2(col[3], col[1])), pyyB = sub2(sub2(col[6], col[4]), pyA);
-        const float2 pxyA = sub2(db, dm), pxyB = sub2(dd, da);
-        const float2 pxxA = make_float2(da.y - (ra[4] - ra[2]), (ra[7] - ra[5]) - da.x);
-        const float2 pxxB = make_float2(db.y - (rb[4] - rb[2]), (rb[7] - rb[5]) - db.x);
+        const float2 dm = over(make_float2(col[2].y - up.y, un.x - col[2].x), hx);   // row y - 1
+        const float2 da = over(make_float2(ra[5] - ra[3], ra[6] - ra[4]), hx);       // row y
+        const float2 db = over(make_float2(rb[5] - rb[3], rb[6] - rb[4]), hx);       // row y + 1
+        const float2 dd = over(make_float2(col[5].y - dp.y, dn.x - col[5].x), hx);   // row y + 2
+        const float2 ea = over(make_float2(ra[4] - ra[2], ra[7] - ra[5]), hx);       // of x - 1, x + 2
+        const float2 eb = over(make_float2(rb[4] - rb[2], rb[7] - rb[5]), hx);
+        const float2 pyA = over(sub2(col[4], col[2]), hy), pyB = over(sub2(col[5], col[3]), hy);
+        const float2 pyyA = over(sub2(pyB, over(sub2(col[3], col[1]), hy)), hy);
+        const float2 pyyB = over(sub2(over(sub2(col[6], col[4]), hy), pyA), hy);
+        const float2 pxyA = over(sub2(db, dm), hy), pxyB = over(sub2(dd, da), hy);
+        const float2 pxxA = over(make_float2(da.y - ea.x, ea.y - da.x), hx);
+        const float2 pxxB = over(make_float2(db.y - eb.x, eb.y - db.x), hx);
         kap[0].x = kappa_value(da.x, pyA.x, pxxA.x, pxyA.x, pyyA.x, ix2, iy2, kb);
         kap[0].y = kappa_value(da.y, pyA.y, pxxA.y, pxyA.y, pyyA.y, ix2, iy2, kb);
         kap[1].x = kappa_value(db.x, pyB.x, pxxB.x, pxyB.x, pyyB.x, ix2, iy2, kb);
@@ -354,24 +372,31 @@ __global__ void __launch_bounds__(LS_NT, RPT == 1 ? 6 : 7) levelset_kernel(LsArg
     if (WHAT != 1) {
       const float2 sg0 = make_float2(sp[0].x < 0.f ? -1.f : 1.f, sp[0].y < 0.f ? -1.f : 1.f);
       const float2 sg1 = make_float2(sp[1].x < 0.f ? -1.f : 1.f, sp[1].y < 0.f ? -1.f : 1.f);
+      const float sx = DIV ? 1.f : idx, sy = DIV ? 1.f : idy;   // what the slopes still lack
       float2 g[2];
       {
         float2 D[7];
 #pragma unroll
-        for (int k = 0; k < 7; ++k) D[k] = make_float2(ra[k + 2] - ra[k + 1], rb[k + 2] - rb[k + 1]);
+        for (int k = 0; k < 7; ++k) {
+          D[k] = make_float2(ra[k + 2] - ra[k + 1], rb[k + 2] - rb[k + 1]);
+          if (DIV) D[k] = __fmul2_rn(D[k], f2(idx));
+        }
         float2 m[2], p[2];   // [column], lanes rows
         weno5_chain<2>(D, m, p);
-        g[0] = make_float2(godunov(sg0.x, m[0].x, p[0].x) * idx, godunov(sg0.y, m[1].x, p[1].x) * idx);
-        g[1] = make_float2(godunov(sg1.x, m[0].y, p[0].y) * idx, godunov(sg1.y, m[1].y, p[1].y) * idx);
+        g[0] = make_float2(godunov(sg0.x, m[0].x, p[0].x) * sx, godunov(sg0.y, m[1].x, p[1].x) * sx);
+        g[1] = make_float2(godunov(sg1.x, m[0].y, p[0].y) * sx, godunov(sg1.y, m[1].y, p[1].y) * sx);
       }
       {
         float2 D[7];
 #pragma unroll
-        for (int k = 0; k < 7; ++k) D[k] = sub2(col[k + 1], col[k]);
+        for (int k = 0; k < 7; ++k) {
+          D[k] = sub2(col[k + 1], col[k]);
+          if (DIV) D[k] = __fmul2_rn(D[k], f2(idy));
+        }
         float2 m[2], p[2];   // [row], lanes columns
         weno5_chain<2>(D, m, p);
         auto length = [&](float gx, float sgn, float mi, float pl) {
-          const float gy = godunov(sgn, mi, pl) * idy;
+          const float gy = godunov(sgn, mi, pl) * sy;
           return sqrt_normal(fmaf(gx, gx, gy * gy));
         };
         del[0] = make_float2(sp[0].x * length(g[0].x, sg0.x, m[0].x, p[0].x),
@@ -432,25 +457,32 @@ __global__ void __launch_bounds__(LS_ET) window_kernel(LsArgs a) {
   }
 }
 
-template <int WHAT, int RPT>
+template <int WHAT, int RPT, bool DIV>
 static void ls_launch_t(cudaStream_t s, const LsArgs& a, int nimg) {
   const dim3 g((a.cols + LS_TX - 1) / LS_TX, (a.rows + LS_TY * RPT - 1) / (LS_TY * RPT), nimg);
   if constexpr (WHAT >= 3) {
     if (a.wins) {
-      levelset_kernel<WHAT, RPT, true><<<g, LS_NT, 0, s>>>(a);
+      levelset_kernel<WHAT, RPT, true, DIV><<<g, LS_NT, 0, s>>>(a);
       return;
     }
   }
-  levelset_kernel<WHAT, RPT, false><<<g, LS_NT, 0, s>>>(a);
+  levelset_kernel<WHAT, RPT, false, DIV><<<g, LS_NT, 0, s>>>(a);
 }
 
-template <int WHAT>
+template <int WHAT, bool DIV>
 static void ls_launch(cudaStream_t s, const LsArgs& a, int nimg) {
   // Tall tiles (fewer halo rows per pixel) where they fill the GPU, else one pass per CTA.
   const long long tall = (long long)((a.cols + LS_TX - 1) / LS_TX) *
                          ((a.rows + 4 * LS_TY - 1) / (4 * LS_TY)) * nimg;
-  if (tall >= LS_TALL_CTAS) ls_launch_t<WHAT, 4>(s, a, nimg);
-  else ls_launch_t<WHAT, 1>(s, a, nimg);
+  if (tall >= LS_TALL_CTAS) ls_launch_t<WHAT, 4, DIV>(s, a, nimg);
+  else ls_launch_t<WHAT, 1, DIV>(s, a, nimg);
+}
+template <int WHAT>
+static void ls_launch(cudaStream_t s, const LsArgs& a, int nimg) {
+  if (std::min(a.dx, a.dy) < LS_NEAR || std::max(a.dx, a.dy) > LS_FAR)
+    ls_launch<WHAT, true>(s, a, nimg);
+  else
+    ls_launch<WHAT, false>(s, a, nimg);
 }
 
 cudaError_t launch_levelset(cudaStream_t s, int what, int rows, int cols, const float* phi,
