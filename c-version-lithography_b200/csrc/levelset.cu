@@ -117,9 +117,13 @@ __device__ __forceinline__ void weno5_chain(const float2 (&D)[N + 5], float2 (&m
 
 // Godunov's one-sided slope along an axis for the sign of the normal speed
 // (level_set_utils.cpp:180-213): of (minus, plus), max(m, 0) and -min(p, 0) where the
-// speed is positive, max(-m, 0) and -min(-p, 0) where it is negative; the larger counts.
+// speed is positive, max(-m, 0) and -min(-p, 0) where it is negative; the larger counts. Where
+// the speed is zero the slope does not count, whatever it is (speed_times).
 __device__ __forceinline__ float godunov(float sign, float m, float p) {
   return fmaxf(fmaxf(sign * m, -sign * p), 0.f);
+}
+__device__ __forceinline__ float speed_times(float speed, float length) {
+  return speed == 0.f ? 0.f : speed * length;
 }
 
 // Tile rows y0 - LS_H .. , columns x0 - LS_HX ..: every index clamped into the image.
@@ -370,8 +374,8 @@ __global__ void __launch_bounds__(LS_NT, RPT == 1 ? 6 : 7) levelset_kernel(LsArg
     }
     float2 del[2] = {f2(0.f), f2(0.f)};     // Vn |grad phi|
     if (WHAT != 1) {
-      const float2 sg0 = make_float2(sp[0].x < 0.f ? -1.f : 1.f, sp[0].y < 0.f ? -1.f : 1.f);
-      const float2 sg1 = make_float2(sp[1].x < 0.f ? -1.f : 1.f, sp[1].y < 0.f ? -1.f : 1.f);
+      const float2 sg0 = make_float2(copysignf(1.f, sp[0].x), copysignf(1.f, sp[0].y));
+      const float2 sg1 = make_float2(copysignf(1.f, sp[1].x), copysignf(1.f, sp[1].y));
       const float sx = DIV ? 1.f : idx, sy = DIV ? 1.f : idy;   // what the slopes still lack
       float2 g[2];
       {
@@ -399,10 +403,10 @@ __global__ void __launch_bounds__(LS_NT, RPT == 1 ? 6 : 7) levelset_kernel(LsArg
           const float gy = godunov(sgn, mi, pl) * sy;
           return sqrt_normal(fmaf(gx, gx, gy * gy));
         };
-        del[0] = make_float2(sp[0].x * length(g[0].x, sg0.x, m[0].x, p[0].x),
-                             sp[0].y * length(g[0].y, sg0.y, m[0].y, p[0].y));
-        del[1] = make_float2(sp[1].x * length(g[1].x, sg1.x, m[1].x, p[1].x),
-                             sp[1].y * length(g[1].y, sg1.y, m[1].y, p[1].y));
+        del[0] = make_float2(speed_times(sp[0].x, length(g[0].x, sg0.x, m[0].x, p[0].x)),
+                             speed_times(sp[0].y, length(g[0].y, sg0.y, m[0].y, p[0].y)));
+        del[1] = make_float2(speed_times(sp[1].x, length(g[1].x, sg1.x, m[1].x, p[1].x)),
+                             speed_times(sp[1].y, length(g[1].y, sg1.y, m[1].y, p[1].y)));
       }
     }
 #pragma unroll
