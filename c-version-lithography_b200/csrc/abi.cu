@@ -2367,14 +2367,14 @@ int litho_exchange_compute_epe(litho_ctx* ctx, const litho_partition* cp, const 
   const size_t ncand = (size_t)e.n_eps * (2 * periods + 1) * (2 * periods + 1);
   if (ncand > (size_t)1 << 28)   // the sorted scatter takes 4 entries per candidate
     return ctx->fail(LITHO_ERR_INVALID_ARGUMENT, "MicroGradientExchange: too many EPs");
-  if (!p->d_work) {
-    if (cudaMalloc(&p->d_work, 4 * n * tt * sizeof(float)) != cudaSuccess ||
-        cudaMalloc(&p->d_loss, (size_t)(S + 1) * n * sizeof(double)) != cudaSuccess ||
-        cudaMalloc(&p->d_xpart, (size_t)litho_partition::kMaxRel * n * 32 * sizeof(double)) !=
-            cudaSuccess) {
-      cudaGetLastError();
-      return ctx->fail(LITHO_ERR_OOM, "full-chip work allocation failed");
-    }
+  // Each on its own: after a failed call the next one takes up those that are missing.
+  auto hold = [](auto** q, size_t count) {
+    return *q != nullptr || cudaMalloc(q, count * sizeof(**q)) == cudaSuccess;
+  };
+  if (!hold(&p->d_work, 4 * n * tt) || !hold(&p->d_loss, (size_t)(S + 1) * n) ||
+      !hold(&p->d_xpart, (size_t)litho_partition::kMaxRel * n * 32)) {
+    cudaGetLastError();
+    return ctx->fail(LITHO_ERR_OOM, "full-chip work allocation failed");
   }
   // EP work: EPE window, main region, dilation scratch (n tiles each), then the
   // aerial and wafer images and the dL/dI of a group of tiles.

@@ -6,8 +6,10 @@
 
 int fake_allocs = 0;              /* cudaMalloc and cudaMallocHost calls so far */
 size_t fake_sizes[4096];          /* their sizes in bytes */
+int fake_fail = 0;                /* the fake_fail-th call from now on fails */
 
 static int take(void **p, size_t n) {
+  if (fake_fail && --fake_fail == 0) return 2;   /* cudaErrorMemoryAllocation */
   if (fake_allocs < 4096) fake_sizes[fake_allocs] = n;
   ++fake_allocs;
   *p = calloc(1, n ? n : 1);
@@ -36,3 +38,10 @@ struct fake_dim3 { unsigned x, y, z; };
 int cudaLaunchKernel(const void *f, struct fake_dim3 g, struct fake_dim3 b, void **a, size_t m, void *s) {
   (void)f; (void)g; (void)b; (void)a; (void)m; (void)s; return 0;
 }
+int cudaStreamCreateWithFlags(void **s, unsigned f) { (void)f; *s = malloc(1); return *s ? 0 : 2; }
+int cudaStreamDestroy(void *s) { free(s); return 0; }
+int cudaStreamWaitEvent(void *s, void *e, unsigned f) { (void)s; (void)e; (void)f; return 0; }
+int cudaEventCreateWithFlags(void **e, unsigned f) { (void)f; *e = malloc(1); return *e ? 0 : 2; }
+int cudaEventDestroy(void *e) { free(e); return 0; }
+int cudaEventRecord(void *e, void *s) { (void)e; (void)s; return 0; }
+int cudaEventSynchronize(void *e) { (void)e; return 0; }
