@@ -2075,9 +2075,11 @@ struct litho_partition {
   // each) | neighbour count (1/tile) | relations (kMaxRel * FC_REL_INTS per tile).
   int* d_meta = nullptr;
   size_t off_origin = 0, off_core_g = 0, off_core_l = 0, off_update = 0, off_nrel = 0, off_rel = 0;
-  // Exchange work, allocated on first use: targets | pe windows | penalty windows |
-  // raw gradients (ntiles * ts * ts floats each), the imaging field, loss sums.
+  // Exchange work, grown to what a call needs: targets | pe windows | penalty windows (not
+  // with the windows formed on chip) | raw gradients (where the caller gives no room for
+  // them), ntiles * ts * ts floats each; the imaging field; loss sums.
   float* d_work = nullptr;
+  size_t work_n = 0;
   float2* fe = nullptr;
   float2* fm = nullptr;
   size_t fe_n = 0, fm_n = 0;
@@ -2371,10 +2373,26 @@ int litho_exchange_compute_epe(litho_ctx* ctx, const litho_partition* cp, const 
   auto hold = [](auto** q, size_t count) {
     return *q != nullptr || cudaMalloc(q, count * sizeof(**q)) == cudaSuccess;
   };
-  if (!hold(&p->d_work, 4 * n * tt) || !hold(&p->d_loss, (size_t)(S + 1) * n) ||
+  if (!hold(&p->d_loss, (size_t)(S + 1) * n) ||
       !hold(&p->d_xpart, (size_t)litho_partition::kMaxRel * n * 32)) {
     cudaGetLastError();
     return ctx->fail(LITHO_ERR_OOM, "full-chip work allocation failed");
+  }
+  // The persistent fused kernel reads the layout itself and forms the windows from the loss
+  // region; EP work, Core metrics and the other schedules take them as images.
+  const bool on_chip = batched && !eval_epe && tc3_fused_supported(cache->g.kp_rows, cache->g.Nc, cache->g.Nr) &&
+                       ctx->tc_persistent(ts, group) &&
+                       (n % group == 0 || ctx->tc_persistent(ts, n % group));
+  const size_t work_n = ((on_chip ? 0 : 3) + (d_raw ? 0 : 1)) * (size_t)n * tt;
+  if (p->work_n < work_n) {
+    LITHO_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
+    if (p->d_work) cudaFree(p->d_work);
+    p->d_work = nullptr; p->work_n = 0;
+    if (cudaMalloc(&p->d_work, work_n * sizeof(float)) != cudaSuccess) {
+      cudaGetLastError();
+      return ctx->fail(LITHO_ERR_OOM, "full-chip work allocation failed");
+    }
+    p->work_n = work_n;
   }
   // EP work: EPE window, main region, dilation scratch (n tiles each), then the
   // aerial and wafer images and the dL/dI of a group of tiles.
@@ -2434,10 +2452,10 @@ int litho_exchange_compute_epe(litho_ctx* ctx, const litho_partition* cp, const 
   if (!st) st = ctx->ensure_host(HOST_MORE + (size_t)(S + 1) * n);
   if (!st) st = begin_red(ctx);
   if (st) return st;
-  float* targets = p->d_work;
-  float* pe_w = targets + n * tt;
-  float* pen_w = pe_w + n * tt;
-  float* raw = d_raw ? d_raw : pen_w + n * tt;
+  float* targets = on_chip ? nullptr : p->d_work;
+  float* pe_w = on_chip ? nullptr : targets + n * tt;
+  float* pen_w = on_chip ? nullptr : pe_w + n * tt;
+  float* raw = d_raw ? d_raw : on_chip ? p->d_work : pen_w + n * tt;
   float* epe_w = eval_epe ? p->d_epe_work : nullptr;
   float* main_dil = eval_epe ? epe_w + n * tt : nullptr;
   float* dil_tmp = eval_epe ? main_dil + n * tt : nullptr;
@@ -2459,11 +2477,6 @@ int litho_exchange_compute_epe(litho_ctx* ctx, const litho_partition* cp, const 
                                         (size_t)e.n_eps * sizeof(double), cudaMemcpyHostToDevice, s));
   }
   const bool pe_epe = o.loss_type == LITHO_MICRO_LOSS_PE_EPE;
-  // The persistent fused kernel reads the layout itself and forms the windows from the loss
-  // region; EP work, Core metrics and the other schedules take them as images.
-  const bool on_chip = batched && !eval_epe && tc3_fused_supported(cache->g.kp_rows, cache->g.Nc, cache->g.Nr) &&
-                       ctx->tc_persistent(ts, group) &&
-                       (n % group == 0 || ctx->tc_persistent(ts, n % group));
   const int* region_meta = p->d_meta + (guard_region ? p->off_update : p->off_core_l);
   if (!on_chip)
     st = check_launch(ctx, launch_tiles_extract(s, d_global_target, p->height, p->width, n,
