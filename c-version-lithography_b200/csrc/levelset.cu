@@ -14,17 +14,19 @@
 
 namespace litho_b200 {
 
-constexpr int LS_PX = 2;             // a thread computes blocks of LS_PX x 2 pixels
-constexpr int LS_TX = 32 * LS_PX;    // tile width (x, columns): one warp
-constexpr int LS_TY = 8;             // rows per pass of the CTA (4 warps x 2 rows)
+constexpr int LS_NT = 128;
 constexpr int LS_H = 3;              // halo rows
 constexpr int LS_HX = 4;             // halo columns on each side (3 used; keeps pairs aligned)
-constexpr int LS_SW = LS_TX + 2 * LS_HX;
-constexpr int LS_NT = 128;
+// A tile takes TXL threads along x, each of which computes blocks of 2 x 2 pixels: its width,
+// the rows per pass of the CTA, and the width with halo.
+constexpr int LS_WIDE = 32, LS_NARROW = 16;
+constexpr int ls_tx(int txl) { return 2 * txl; }
+constexpr int ls_ty(int txl) { return 2 * (LS_NT / txl); }
+constexpr int ls_sw(int txl) { return ls_tx(txl) + 2 * LS_HX; }
 constexpr int LS_ET = 256;           // threads of the elementwise and reduction kernels
 // CTAs of tall tiles from which they are used (at least four per SM).
 constexpr int LS_TALL_CTAS = 592;
-static_assert(LS_SW % 4 == 0, "tile rows are 16-byte aligned");
+static_assert(ls_sw(LS_WIDE) % 4 == 0 && ls_sw(LS_NARROW) % 4 == 0, "tile rows are 16-byte aligned");
 
 __device__ __forceinline__ float2 f2(float a) { return make_float2(a, a); }
 __device__ __forceinline__ float2 sub2(float2 a, float2 b) { return __ffma2_rn(b, f2(-1.f), a); }
@@ -127,11 +129,11 @@ __device__ __forceinline__ float speed_times(float speed, float length) {
 }
 
 // Tile rows y0 - LS_H .. , columns x0 - LS_HX ..: every index clamped into the image.
-template <int SH>
-__device__ __forceinline__ void load_tile(float (*t)[LS_SW], const float* __restrict__ phi,
+template <int SH, int SW>
+__device__ __forceinline__ void load_tile(float (*t)[SW], const float* __restrict__ phi,
                                           int rows, int cols, int y0, int x0, bool vec4) {
-  if (vec4 && x0 >= LS_HX && x0 - LS_HX + LS_SW <= cols) {
-    constexpr int Q = LS_SW / 4;
+  if (vec4 && x0 >= LS_HX && x0 - LS_HX + SW <= cols) {
+    constexpr int Q = SW / 4;
     const float* base = phi + x0 - LS_HX;
 #pragma unroll
     for (int i0 = 0; i0 < SH * Q; i0 += LS_NT) {
@@ -144,27 +146,30 @@ __device__ __forceinline__ void load_tile(float (*t)[LS_SW], const float* __rest
     }
     return;
   }
-  // warp w loads tile rows w, w + 4, ...; each lane columns lane, lane + 32, lane + 64
+  // warp w loads tile rows w, w + 4, ...; each lane columns lane, lane + 32, ...
+  constexpr int NC = (SW + 31) / 32;
   const int lane = threadIdx.x & 31;
-  int xc[3];
+  int xc[NC];
 #pragma unroll
-  for (int k = 0; k < 3; ++k) xc[k] = min(max(x0 - LS_HX + lane + 32 * k, 0), cols - 1);
+  for (int k = 0; k < NC; ++k) xc[k] = min(max(x0 - LS_HX + lane + 32 * k, 0), cols - 1);
   for (int ty = threadIdx.x >> 5; ty < SH; ty += LS_NT / 32) {
     const float* row = phi + (size_t)min(max(y0 - LS_H + ty, 0), rows - 1) * cols;
-    t[ty][lane] = __ldg(row + xc[0]);
-    t[ty][lane + 32] = __ldg(row + xc[1]);
-    if (lane + 64 < LS_SW) t[ty][lane + 64] = __ldg(row + xc[2]);
+#pragma unroll
+    for (int k = 0; k < NC; ++k)
+      if (lane + 32 * k < SW) t[ty][lane + 32 * k] = __ldg(row + xc[k]);
   }
 }
 
 // _gradient_1d along x (level_set_utils.cpp:228-255) at global column x of row ly.
-__device__ __forceinline__ float grad_x(const float (*t)[LS_SW], int ly, int lx, int x, int cols,
+template <int SW>
+__device__ __forceinline__ float grad_x(const float (*t)[SW], int ly, int lx, int x, int cols,
                                         float inv2d) {
   if (x == 0) return (-3.f * t[ly][lx] + 4.f * t[ly][lx + 1] - t[ly][lx + 2]) * inv2d;
   if (x == cols - 1) return (3.f * t[ly][lx] - 4.f * t[ly][lx - 1] + t[ly][lx - 2]) * inv2d;
   return (t[ly][lx + 1] - t[ly][lx - 1]) * inv2d;
 }
-__device__ __forceinline__ float grad_y(const float (*t)[LS_SW], int ly, int lx, int y, int rows,
+template <int SW>
+__device__ __forceinline__ float grad_y(const float (*t)[SW], int ly, int lx, int y, int rows,
                                         float inv2d) {
   if (y == 0) return (-3.f * t[ly][lx] + 4.f * t[ly + 1][lx] - t[ly + 2][lx]) * inv2d;
   if (y == rows - 1) return (3.f * t[ly][lx] - 4.f * t[ly - 1][lx] + t[ly - 2][lx]) * inv2d;
@@ -182,7 +187,8 @@ __device__ __forceinline__ float kappa_value(float px, float py, float pxx, floa
 }
 
 // The same at global (y, x) near the image border, where some differences are one-sided.
-__device__ __noinline__ float kappa_border(const float (*t)[LS_SW], int ly, int lx, int y, int x,
+template <int SW>
+__device__ __noinline__ float kappa_border(const float (*t)[SW], int ly, int lx, int y, int x,
                                            int rows, int cols, float dx, float dy, float b) {
   const float ix = 1.f / (2.f * dx), iy = 1.f / (2.f * dy);
   float pxy, pxx, pyy;
@@ -225,8 +231,7 @@ struct LsArgs {
   int vec4, vec2;     // 16-byte loads of phi rows; 8-byte accesses of pixel pairs elsewhere
 };
 
-// Stencil modes 0-4. A CTA computes LS_TX x (LS_TY RPT) pixels from a tile in shared
-// memory, each thread RPT blocks of 2 x 2 pixels: packed FP32x2 lanes are the two rows
+// Stencil modes 0-4. A CTA computes TX x (TY RPT) pixels from a tile in shared memory, each thread RPT blocks of 2 x 2 pixels: packed FP32x2 lanes are the two rows
 // along x and the two columns along y, and neighbouring pixels of a block share their
 // smoothness indicators and candidates (weno5_chain). The stencil is bound by FP32 issue
 // (a packed instruction takes the issue port and the FMA pipe twice): 176-197 thread
@@ -243,10 +248,10 @@ struct LsArgs {
 // LS_NEAR .. LS_FAR, inside which the products of slopes from 1e-8 to 1e9 stay in range and
 // the divisions would cost 3.6 % (16 images of 2048^2: 1136 us an update against 1096).
 constexpr float LS_NEAR = 1.f / 4096, LS_FAR = 4096.f;
-template <int WHAT, int RPT, bool WIN, bool DIV>
+template <int WHAT, int RPT, bool WIN, bool DIV, int TXL>
 __global__ void __launch_bounds__(LS_NT, RPT == 1 ? 6 : 7) levelset_kernel(LsArgs a) {
-  constexpr int SH = LS_TY * RPT + 2 * LS_H;
-  __shared__ __align__(16) float t[SH][LS_SW];
+  constexpr int TY = ls_ty(TXL), SH = TY * RPT + 2 * LS_H, SW = ls_sw(TXL);
+  __shared__ __align__(16) float t[SH][SW];
   const size_t img = (size_t)blockIdx.z * a.rows * a.cols;
   const float* phi = a.phi + img;
   float* out = a.out + img;
@@ -255,11 +260,11 @@ __global__ void __launch_bounds__(LS_NT, RPT == 1 ? 6 : 7) levelset_kernel(LsArg
     const int* w = a.wins + 4 * (size_t)blockIdx.z;
     wy0 = w[0]; wy1 = w[1]; wx0 = w[2]; wx1 = w[3];
   }
-  const int x0 = blockIdx.x * LS_TX, y0 = blockIdx.y * (LS_TY * RPT);
+  const int x0 = blockIdx.x * ls_tx(TXL), y0 = blockIdx.y * (TY * RPT);
   const float* phi0 = a.phi0 ? a.phi0 + img : nullptr;
   const float* vn = a.vn ? a.vn + img : nullptr;
   float* out2 = a.out2 ? a.out2 + img : nullptr;
-  const int lx = 2 * (threadIdx.x & 31), x = x0 + lx;
+  const int lx = 2 * (threadIdx.x % TXL), x = x0 + lx;
   const bool pair = x + 1 < a.cols;       // both columns of the block lie in the image
   const bool v2 = pair && a.vec2;
   auto load2 = [&](const float* p, size_t i) -> float2 {
@@ -277,7 +282,7 @@ __global__ void __launch_bounds__(LS_NT, RPT == 1 ? 6 : 7) levelset_kernel(LsArg
   // The normal speed of a block, [row](x, x + 1), loaded one pass ahead of its use.
   float2 sp_n[2] = {f2(0.f), f2(0.f)};
   auto fetch = [&](int r) {
-    const int y = y0 + 2 * (threadIdx.x >> 5) + r * LS_TY;
+    const int y = y0 + 2 * (threadIdx.x / TXL) + r * TY;
     const size_t i = (size_t)y * a.cols + x;
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
@@ -290,7 +295,7 @@ __global__ void __launch_bounds__(LS_NT, RPT == 1 ? 6 : 7) levelset_kernel(LsArg
     }
   };
   fetch(0);
-  load_tile<SH>(t, phi, a.rows, a.cols, y0, x0, a.vec4 != 0);
+  load_tile<SH, SW>(t, phi, a.rows, a.cols, y0, x0, a.vec4 != 0);
   __syncthreads();
   const float idx = 1.f / a.dx, idy = 1.f / a.dy;
   const float ix2 = DIV ? 1.f : 0.25f * idx * idx, iy2 = DIV ? 1.f : 0.25f * idy * idy;
@@ -299,7 +304,7 @@ __global__ void __launch_bounds__(LS_NT, RPT == 1 ? 6 : 7) levelset_kernel(LsArg
   if (x >= a.cols) return;
 #pragma unroll 1
   for (int r = 0; r < RPT; ++r) {
-    const int ly = 2 * (threadIdx.x >> 5) + r * LS_TY, y = y0 + ly;
+    const int ly = 2 * (threadIdx.x / TXL) + r * TY, y = y0 + ly;
     if (y >= a.rows) break;
     const bool two = y + 1 < a.rows;        // both rows lie in the image
     const size_t i0 = (size_t)y * a.cols + x, i1 = i0 + a.cols;
@@ -308,8 +313,8 @@ __global__ void __launch_bounds__(LS_NT, RPT == 1 ? 6 : 7) levelset_kernel(LsArg
       ph[0] = load2(phi0, i0);
       if (two) ph[1] = load2(phi0, i1);
     }
-    const float* c = &t[ly + LS_H][lx + LS_HX];   // pixel (y, x); row stride LS_SW
-    auto at2 = [&](int oy, int ox) { return *reinterpret_cast<const float2*>(c + oy * LS_SW + ox); };
+    const float* c = &t[ly + LS_H][lx + LS_HX];   // pixel (y, x)
+    auto at2 = [&](int oy, int ox) { return *reinterpret_cast<const float2*>(c + oy * SW + ox); };
     const float2 sp[2] = {sp_n[0], sp_n[1]};
     if (r + 1 < RPT) fetch(r + 1);
     if (WIN && (y + 1 < wy0 || y >= wy1 || x + 1 < wx0 || x >= wx1)) {
@@ -461,23 +466,26 @@ __global__ void __launch_bounds__(LS_ET) window_kernel(LsArgs a) {
   }
 }
 
-template <int WHAT, int RPT, bool DIV>
+template <int WHAT, int RPT, bool DIV, int TXL = LS_WIDE>
 static void ls_launch_t(cudaStream_t s, const LsArgs& a, int nimg) {
-  const dim3 g((a.cols + LS_TX - 1) / LS_TX, (a.rows + LS_TY * RPT - 1) / (LS_TY * RPT), nimg);
+  constexpr int TX = ls_tx(TXL), TY = ls_ty(TXL) * RPT;
+  const dim3 g((a.cols + TX - 1) / TX, (a.rows + TY - 1) / TY, nimg);
   if constexpr (WHAT >= 3) {
     if (a.wins) {
-      levelset_kernel<WHAT, RPT, true, DIV><<<g, LS_NT, 0, s>>>(a);
+      levelset_kernel<WHAT, RPT, true, DIV, TXL><<<g, LS_NT, 0, s>>>(a);
       return;
     }
   }
-  levelset_kernel<WHAT, RPT, false, DIV><<<g, LS_NT, 0, s>>>(a);
+  levelset_kernel<WHAT, RPT, false, DIV, TXL><<<g, LS_NT, 0, s>>>(a);
 }
 
 template <int WHAT, bool DIV>
 static void ls_launch(cudaStream_t s, const LsArgs& a, int nimg) {
+  // Images of one narrow tile, of whose wide one half the lanes would have no pixel.
+  if (a.cols <= ls_tx(LS_NARROW)) return ls_launch_t<WHAT, 1, DIV, LS_NARROW>(s, a, nimg);
   // Tall tiles (fewer halo rows per pixel) where they fill the GPU, else one pass per CTA.
-  const long long tall = (long long)((a.cols + LS_TX - 1) / LS_TX) *
-                         ((a.rows + 4 * LS_TY - 1) / (4 * LS_TY)) * nimg;
+  constexpr int TX = ls_tx(LS_WIDE), TY = 4 * ls_ty(LS_WIDE);
+  const long long tall = (long long)((a.cols + TX - 1) / TX) * ((a.rows + TY - 1) / TY) * nimg;
   if (tall >= LS_TALL_CTAS) ls_launch_t<WHAT, 4, DIV>(s, a, nimg);
   else ls_launch_t<WHAT, 1, DIV>(s, a, nimg);
 }
