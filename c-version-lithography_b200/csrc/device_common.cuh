@@ -217,7 +217,11 @@ struct GradEpiT {
     gt.z = -0.5f * G.z * sn(th.z);
     gt.w = -0.5f * G.w * sn(th.w);
     if (FAST) {
-      // lanes past the edge hold theta = 0 and G = 0, so they add nothing
+      // lanes past the edge add nothing: the band operand's rows there are not part of the
+      // image and may hold anything
+      if (nvalid < 2) gt.y = 0.f;
+      if (nvalid < 3) gt.z = 0.f;
+      if (nvalid < 4) gt.w = 0.f;
       nrm += (double)(gt.x * gt.x + gt.y * gt.y + gt.z * gt.z + gt.w * gt.w);
     } else {
       if (nvalid > 0) nrm += (double)gt.x * gt.x;
