@@ -164,7 +164,10 @@ struct Context {
   }
   void collect_stages();  // after a stream synchronize
 
+  // The runtime forgets an error that the call reports, which the caller's next check of the
+  // runtime would take for its own.
   int fail(int code, const std::string& m) {
+    if (code == LITHO_ERR_CUDA) cudaGetLastError();
     last_error = m;
     return code;
   }

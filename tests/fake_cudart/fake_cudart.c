@@ -29,14 +29,20 @@ int cudaGetDevice(int *d) { *d = 0; return 0; }
 int cudaGetDeviceCount(int *n) { *n = 1; return 0; }
 int cudaDeviceSynchronize(void) { return 0; }
 int cudaDeviceGetAttribute(int *v, int a, int d) { (void)a; (void)d; *v = 148; return 0; }
-int cudaGetLastError(void) { return 0; }
-int cudaPeekAtLastError(void) { return 0; }
 int cudaStreamSynchronize(void *s) { (void)s; return 0; }
 int cudaFuncSetAttribute(const void *f, int a, int v) { (void)f; (void)a; (void)v; return 0; }
-int cudaLaunchKernelExC(const void *c, const void *f, void **a) { (void)c; (void)f; (void)a; return 0; }
+int fake_launch_fail = 0;         /* the fake_launch_fail-th launch from now on fails */
+int fake_last = 0;                /* the error that cudaGetLastError reports and forgets */
+static int launch(void) {
+  if (fake_launch_fail && --fake_launch_fail == 0) return fake_last = 1;   /* cudaErrorInvalidValue */
+  return 0;
+}
+int cudaGetLastError(void) { const int e = fake_last; fake_last = 0; return e; }
+int cudaPeekAtLastError(void) { return fake_last; }
+int cudaLaunchKernelExC(const void *c, const void *f, void **a) { (void)c; (void)f; (void)a; return launch(); }
 struct fake_dim3 { unsigned x, y, z; };
 int cudaLaunchKernel(const void *f, struct fake_dim3 g, struct fake_dim3 b, void **a, size_t m, void *s) {
-  (void)f; (void)g; (void)b; (void)a; (void)m; (void)s; return 0;
+  (void)f; (void)g; (void)b; (void)a; (void)m; (void)s; return launch();
 }
 int cudaStreamCreateWithFlags(void **s, unsigned f) { (void)f; *s = malloc(1); return *s ? 0 : 2; }
 int cudaStreamDestroy(void *s) { free(s); return 0; }
