@@ -481,7 +481,7 @@ def levelset_run(L, torch, stream, N=2048, B=16, steps=10, warmup=3):
     byts = 36.0 * B * N * N
     hbm, src = peaks()
     gbs = byts / (ms * 1e-3) / 1e9
-    out = {"bound": "hbm", "kernel": "levelset_kernel RK2 stages + absmax/dt (one batched call)",
+    out = {"bound": "hbm", "kernel": "levelset_kernel RK2 stages + speed maximum and dt (one batched call)",
            "workload": f"{B} images of {N}^2 per call, CFL 0.5, curvature weight 0.01",
            "ms_per_call": ms, "ms_per_image_update": ms / B, "algorithmic_bytes": byts,
            "achieved": gbs, "peak": hbm, "peak_source": src, "unit": "GB/s", "frac": gbs / hbm,

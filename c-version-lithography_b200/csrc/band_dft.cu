@@ -291,10 +291,12 @@ int analysis_tiles(int N) {
 // Tile partials of sum_{y, x} T(a, y) A[y][x] tw(c, x) for every 128 x 128 tile:
 // part[tile][a][c], tiles in row-major order of the tile grid (each tile's partials
 // contiguous, so that the tensor-core epilogue writes them as one coalesced block).
-// Tiles below which the columns are split over more CTAs, 8 columns each (256^2: 4 tiles,
-// 76 us per imaging call, 86 with 16 columns each and 90 unsplit), or 16 (1001^2: 64 tiles,
-// forward and adjoint 197 us per gradient call, 211 and 198); 2048^2 has 256 tiles, and there
-// the split repeats the loads and cosines for nothing (276 us against 215 per evaluation).
+// Tiles below which the columns are split over more CTAs, 8 columns each or 16: the split fills
+// the SMs and repeats the loads and cosines of a tile. Evaluations with 35 x 35 frequencies, 8
+// columns each / 16 / unsplit: 4 tiles 107 / 118 / 125 us, 25 tiles 121 / 133 / 137, 36 tiles 127 /
+// 130 / 149, 49 tiles 129 / 135 / 156, 64 tiles 155 / 142 / 158; 81 tiles 161 / 145 / 163, 100
+// tiles 167 / 168 / 162, 121 tiles 194 / 187 / 166. With 52 x 52 the first line lies between 36 and
+// 49 tiles (160 / 164 and 188 / 171 us), with 21 x 21 at 49 (103 / 102).
 constexpr int AT_SMALL = 32, AT_MID = 96;
 cudaError_t launch_analysis(cudaStream_t s, int mode, const float* in, float* mask_out,
                             int* flag, const float* tw, int N, int ncols, const float2* TY,

@@ -234,9 +234,9 @@ struct LsArgs {
 // Stencil modes 0-4. A CTA computes TX x (TY RPT) pixels from a tile in shared memory, each thread RPT blocks of 2 x 2 pixels: packed FP32x2 lanes are the two rows
 // along x and the two columns along y, and neighbouring pixels of a block share their
 // smoothness indicators and candidates (weno5_chain). The stencil is bound by FP32 issue
-// (a packed instruction takes the issue port and the FMA pipe twice): 176-197 thread
-// instructions per pixel and stage, 82 of them packed, against 422-443 for one pixel per
-// thread. Stages of 16 images of 2048^2: 932 -> 486 us and 1005 -> 535 us (1.9 and 2.0 TB/s).
+// (a packed instruction takes the issue port and the FMA pipe twice): 187 and 206 thread
+// instructions per pixel in stages 1 and 2, 82 of them packed, against 422 and 443 for one pixel
+// per thread. Stages of 16 images of 2048^2: 932 -> 488 us and 1005 -> 538 us (1.9 and 2.0 TB/s).
 // Longer strips fed by cp.async one pass ahead removed the wait for the tile but cost as
 // many instructions as they hid (1.24 against 1.23 ms per update at that stage), and scalar
 // FFMA on blocks of 2 x 4 pixels ran out of registers and instruction cache (1.6 ms).

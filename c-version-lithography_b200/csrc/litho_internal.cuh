@@ -405,7 +405,8 @@ cudaError_t launch_render_mask(cudaStream_t s, const float* phi, int rows, int c
                                int gray, int scale, float* mask);
 // Chamfer signed distance of reinit_sdf over nimg rows x cols images back to back:
 // inside = phi > level (phi >= level when inclusive); sdf must not alias phi. mask
-// (nullable): sdf >= 0. threads: CTA size of the row search (128, 256, 512 or 1024; 0: 256).
+// (nullable): sdf >= 0. threads: CTA size of the row search (128, 256, 512 or 1024; 0: chosen
+// from the row length and the number of row blocks).
 cudaError_t launch_reinit_sdf(cudaStream_t s, int rows, int cols, const float* phi, float level,
                               int inclusive, float dx, float* sdf, float* mask, int nimg = 1,
                               int threads = 0);

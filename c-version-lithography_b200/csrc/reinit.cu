@@ -26,7 +26,7 @@
 // its CTA reads and then overwrites: the transform needs no memory besides its output.
 //
 // The search is bound by issue and the min / max pipe (218 instructions a pixel on patterns
-// of 18-57 pixels in 64-pixel cells: ncu 76 % issue active, the ALU pipe 65 %), where the
+// of 18-57 pixels in 64-pixel cells: ncu 73 % issue active, the ALU pipe 66 %), where the
 // row-sequential form it replaces was bound by the latency of 2 rows steps of three barriers.
 // Times with the printed mask, row-sequential -> now: 24 images of 1266^2 4.19 -> 0.365 ms
 // (rows 307 us, columns 54), one 2048^2 image 8.5 -> 0.060 ms, 64 of 257^2 0.70 -> 0.061 ms;

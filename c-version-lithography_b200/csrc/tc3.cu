@@ -927,8 +927,8 @@ cudaError_t launch_synth_resist_tc3(cudaStream_t s, const void* Aimg, const void
 //   Q(j)      warps 16-23, after R(j + 1): Q -> the item's adjoint partials.
 // One set of 16 warps that did epi, R and Q in turn left half of the issue slots idle, and
 // the MMA thread spent 3400 cycles on the 15 instructions of a synthesis (see elect_one); now
-// R and Q run beside the next item's epilogue. 16 tiles of 2048^2: 216 us before, 199 us so; 12 of
-// 1266^2 127 and 102, 16 micro tiles of 1280^2 with windows 146 and 119.
+// R and Q run beside the next item's epilogue. 16 tiles of 2048^2: 216 us before, 184 us now; 12 of
+// 1266^2 127 and 102, 16 micro tiles of 1280^2 with windows 146 and 101.
 // Shared memory: sA / Ut | TXD (per xt) | TYD (per yt) | sR | AYD (per yt). TXD and sR hold the
 // rf = 2 ncols rows f rounded to 8, TYD the rn = 2 nr rows n: the products read on to BN and
 // 128 rows, into the tiles that follow, and their columns and lanes past rf and rn are not
@@ -949,8 +949,9 @@ constexpr uint32_t F3_SMEM_MAX = 232448 - 2048;   // beside the static barriers 
 
 // MODE 0: no window, no penalty, no image output (the CTM evaluation); 1: windows and
 // penalty; 2: aerial / wafer outputs too. 16 micro tiles of 1280^2 with windows: 435 us when
-// one epilogue served all modes and loaded each pixel's windows in turn, 151 us so; 12 tiles
-// of 1266^2 (19 % of the tiles ragged) 137 -> 116 us with the edge in the packed arithmetic.
+// one epilogue served all modes and loaded each pixel's windows in turn, 101 us now (383 us with
+// windows as images and both outputs); 12 tiles of 1266^2 (19 % of the tiles ragged) 102 us, 137
+// when their edge left the packed arithmetic.
 template <int BN, int MODE>
 __global__ void __launch_bounds__(F3_NT, 1)
 fused_tc3_kernel(const uint8_t* __restrict__ Aimg, const uint8_t* __restrict__ Bimg, int N,
