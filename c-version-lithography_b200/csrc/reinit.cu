@@ -30,8 +30,14 @@
 // row-sequential form it replaces was bound by the latency of 2 rows steps of three barriers.
 // Times with the printed mask, row-sequential -> now: 24 images of 1266^2 4.19 -> 0.365 ms
 // (rows 307 us, columns 54), one 2048^2 image 8.5 -> 0.060 ms, 64 of 257^2 0.70 -> 0.061 ms;
-// a single inside pixel, the longest searches: 84 images of 1266^2 7.9 -> 5.0 ms, one 16384^2
-// 2020 -> 19.5 ms.
+// a single inside pixel, long searches: 84 images of 1266^2 7.9 -> 5.0 ms, one 16384^2 2020 ->
+// 19.5 ms. The longest ones, where every column on the way is nearer than the last, are those
+// around one diagonal line across an otherwise empty image: batches that fill the GPU are slower
+// with them than the row-sequential form was (84 images of 1266^2 8.0 -> 14.7 ms, 300 of 512^2
+// 2.7 -> 4.6), smaller ones faster (one 2048^2 image 8.8 -> 1.0). So are images of a single block
+// of rows (3 x 1000: 27 -> 32 us), of which one CTA does the search. Searching outwards from x
+// helps sparse points (300 of 512^2, one pixel in 10^4: 2.9 -> 2.0 ms) and not the diagonal, and
+// costs 4 to 12 % elsewhere in registers and steps.
 #include <cuda_runtime.h>
 
 #include <algorithm>
