@@ -867,12 +867,30 @@ __device__ __forceinline__ float2 sum4(const float2 (&a)[4]) {
 // row; one thread per pair of outputs keeps the four interleaved partial sums of
 // band_chat_kernel and adds them in its order, so the results are bit-identical.
 constexpr int BC_DR = 5;
-// Rows per CTA of the row-grouped small-grid kernels: few enough for BAND_CTAS CTAs, two per
-// SM. Staging is shared by the rows of a CTA, but a grid below that leaves SMs idle.
+// Rows per CTA (1 .. most) of the row-grouped small-grid kernels, whose CTAs take smem bytes. The
+// rows of a CTA share the staging of its tables, but a grid below two CTAs per SM leaves SMs idle:
+// few enough for BAND_CTAS CTAs. Where the tables leave room for one CTA per SM (bands from about
+// 48 x 48 on), the count with the least waves x (rows + 2), the staging taking about as long as
+// two rows. Evaluations of 300^2 images with 6 kernels, these rules / the first one for all bands /
+// as many rows as leave 148 CTAs: 9 images of 58 x 58 frequencies 266 / 291 / 266 us, 16 images
+// 317 / 318 / 346; 9 images of 40 x 64 231 / 252 / 231, 16 images of 52 x 52 288 / 288 / 303.
 constexpr int BAND_CTAS = 296;
-static int rows_per_cta(int rows, int batch, int most) {
-  const long long per = ((long long)rows * batch + BAND_CTAS - 1) / BAND_CTAS;
-  return (int)std::max<long long>(1, std::min<long long>(per, most));
+static int rows_per_cta(int rows, int batch, int most, size_t smem) {
+  if (2 * (smem + 1024) <= 228 * 1024) {
+    const long long per = ((long long)rows * batch + BAND_CTAS - 1) / BAND_CTAS;
+    return (int)std::max<long long>(1, std::min<long long>(per, most));
+  }
+  int best = 1;
+  long long cost = 0;
+  for (int per = 1; per <= most; ++per) {
+    const long long ctas = (long long)((rows + per - 1) / per) * batch;
+    const long long c = (ctas + BAND_CTAS / 2 - 1) / (BAND_CTAS / 2) * (per + 2);
+    if (per == 1 || c < cost) {
+      best = per;
+      cost = c;
+    }
+  }
+  return best;
 }
 __global__ void __launch_bounds__(256)
 band_chat_rows_kernel(const float* __restrict__ iP, int Nr, int Nc, int Pr, int Pc,
@@ -1302,7 +1320,7 @@ cudaError_t launch_band_forward(cudaStream_t s, const Cache& c, Field& f, float*
     err = cudaFuncSetAttribute(band_chat_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                (int)smc);
     if (err != cudaSuccess) return err;
-    const int per = rows_per_cta(g.Nr, batch, BC_DR);
+    const int per = rows_per_cta(g.Nr, batch, BC_DR, smc);
     err = launch_pdl(band_chat_rows_kernel, dim3((g.Nr + per - 1) / per, batch), dim3(256),
                      smc, s, static_cast<const float*>(iP), g.Nr, g.Nc, g.Pr, g.Pc, c.EDr_t, c.EDc,
                      1.f / ((float)g.Pr * (float)g.Pc), per, chat);
@@ -1706,7 +1724,7 @@ cudaError_t launch_band_adjoint(cudaStream_t s, const Cache& c, const Field& f, 
     e0 = cudaFuncSetAttribute(band_gamma_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                               (int)smg);
     if (e0 != cudaSuccess) return e0;
-    const int per = rows_per_cta(g.Pr, batch, BG_JR);
+    const int per = rows_per_cta(g.Pr, batch, BG_JR, smg);
     e0 = launch_pdl(band_gamma_rows_kernel, dim3((g.Pr + per - 1) / per, batch), dim3(256),
                     smg, s, gh, g.Nr, g.Nc, g.Pr, g.Pc, c.EDr_t, c.EDc_t, per, gam);
   } else {
